@@ -547,7 +547,7 @@ std::vector<unsigned char> make_table_bytes(const Plan& p, DevGeom* g) {
 // point lie in that unit's two rows.  Units are ordered by point count, largest first.
 // Leaves the fusion off (plan unchanged) when a point falls in a parity class without
 // a channel or CFFT_ZRECON=0.
-Status build_zrecon_units(Plan* p, std::string* err) {
+Status build_zrecon_units(Plan* p, const DevGeom& g, std::string* err) {
   if (const char* e = std::getenv("CFFT_ZRECON")) if (e[0] == '0') return Status::kOk;
   const PlanTables& T = p->T;
   const int H = p->fast_h, nch = T.n_ch;
@@ -603,16 +603,52 @@ Status build_zrecon_units(Plan* p, std::string* err) {
     pts.insert(pts.end(), u.pts.begin(), u.pts.end());
   }
   if (ut.empty()) return Status::kOk;
+  // Points with their packed h, and the weights of the Hermitian tap pairs (sg, 7 - sg): with
+  // u = w[sg], v = w[7 - sg] the phases e^{-2 pi i h.t / N} of the two sign images,
+  // Pw = (u + v) / 2 and Qw = ((v.y - u.y) / 2, (u.x - v.x) / 2).
+  std::vector<uint2> pt(pts.size());
+  std::vector<double> pq(pts.size() * 16), phase(2 * static_cast<size_t>(T.P));
+  for (int j = 0; j < T.P; ++j) {
+    phase[2 * j] = std::cos(2.0 * M_PI * j / T.P);
+    phase[2 * j + 1] = -std::sin(2.0 * M_PI * j / T.P);
+  }
+  for (size_t i = 0; i < pts.size(); ++i) {
+    const auto& h = T.spec[pts[i]].h;
+    pt[i] = make_uint2(pts[i], static_cast<uint32_t>(h[0]) | (static_cast<uint32_t>(h[1]) << 10) | (static_cast<uint32_t>(h[2]) << 20));
+    const double* w[8];
+    for (int sg = 0; sg < 8; ++sg) {
+      long j = 0;
+      for (int d = 0; d < 3; ++d) j += static_cast<long>(h[d]) * g.rep_tp[g.sign_op[sg]][d];
+      w[sg] = &phase[2 * floor_mod(j, T.P)];
+    }
+    for (int sg = 0; sg < 4; ++sg) {
+      const double* u = w[sg];
+      const double* v = w[7 - sg];
+      double* op = &pq[(static_cast<size_t>(2 * sg) * pts.size() + i) * 2];
+      double* oq = op + pts.size() * 2;
+      op[0] = 0.5 * (u[0] + v[0]);
+      op[1] = 0.5 * (u[1] + v[1]);
+      oq[0] = 0.5 * (v[1] - u[1]);
+      oq[1] = 0.5 * (u[0] - v[0]);
+    }
+  }
+  std::vector<float> pqf;
+  if (p->precision == 4) pqf.assign(pq.begin(), pq.end());
+  const void* pq_src = p->precision == 4 ? static_cast<const void*>(pqf.data()) : pq.data();
+  const size_t pq_bytes = pq.size() * p->precision;
   // Plan-owned device tables: counted in the plan's device bytes, allocation failures
   // reported as such (like the other plan buffers).
   for (auto [ptr, bytes, what] : {std::tuple<void**, size_t, const char*>{&p->d_zr_units, ut.size() * sizeof(uint4), "fused gather units"},
-                                  std::tuple<void**, size_t, const char*>{&p->d_zr_pts, pts.size() * 4, "fused gather points"}}) {
+                                  std::tuple<void**, size_t, const char*>{&p->d_zr_pts, pt.size() * sizeof(uint2), "fused gather points"},
+                                  std::tuple<void**, size_t, const char*>{&p->d_zr_pq, pq_bytes, "fused gather weights"}}) {
     const cudaError_t e = cudaMalloc(ptr, bytes);
     if (e != cudaSuccess) { *err = cuda_msg(e, what); return Status::kAlloc; }
     p->workspace_bytes += bytes;
   }
   CFFT_CUDA(cudaMemcpy(p->d_zr_units, ut.data(), ut.size() * sizeof(uint4), cudaMemcpyHostToDevice), "upload units");
-  CFFT_CUDA(cudaMemcpy(p->d_zr_pts, pts.data(), pts.size() * 4, cudaMemcpyHostToDevice), "upload unit points");
+  CFFT_CUDA(cudaMemcpy(p->d_zr_pts, pt.data(), pt.size() * sizeof(uint2), cudaMemcpyHostToDevice), "upload unit points");
+  CFFT_CUDA(cudaMemcpy(p->d_zr_pq, pq_src, pq_bytes, cudaMemcpyHostToDevice), "upload unit weights");
+  p->zr_npts = static_cast<int>(pts.size());
   p->zr_units = static_cast<int>(ut.size());
   p->zrecon = true;
   return Status::kOk;
@@ -634,17 +670,17 @@ Status launch_stage(Plan* p, int stage, const T* f0, typename Cx<T>::type* F, co
     if (p->cluster && (stage == 1 || stage == 4)) return Status::kOk;  // fused into stages 0 and 5
     FastArgs a;
     a.geom = p->d_geom; a.tables = p->d_tables; a.spec_h = p->d_spec_h; a.K = p->d_K;
-    a.inv_spec = p->d_inv_spec; a.inv_phase = p->d_inv_phase; a.inv_pk = p->d_inv_pk; a.expand = p->d_expand;
+    a.inv_spec = p->d_inv_spec; a.inv_phase = p->d_inv_phase; a.expand = p->d_expand;
+    a.fib_taps = p->d_fib_taps; a.fib_outs = p->d_fib_outs; a.n_fib = p->n_fib;
     a.W = W;
     a.G0R = p->d_g0r ? static_cast<char*>(p->d_g0r) + lane * p->g0r_lane_bytes : nullptr;
-    a.FT = p->d_ft ? static_cast<char*>(p->d_ft) + lane * p->ft_lane_bytes : nullptr;
     a.f0 = f0; a.F = F; a.Fin = Fin; a.f0_out = f0_out; a.E = E;
     a.stage = stage; a.nb = nb; a.H = p->fast_h; a.n_ch = T_.n_ch; a.centered = T_.centered ? 1 : 0;
     a.cent_type = p->cent_type; a.d = T_.d;
     a.n_spec = static_cast<int>(T_.spec.size()); a.n_orbits = static_cast<int>(T_.orbit_rep.size());
     a.use_K = use_K; a.rep_diag8 = p->rep_diag8; a.rep_perm = p->rep_perm; a.reps_quad = p->reps_quad;
     a.reps_wide = p->reps_wide && !p->cluster;
-    a.zr_units = p->d_zr_units; a.zr_pts = p->d_zr_pts; a.zr_n_units = p->zr_units;
+    a.zr_units = p->d_zr_units; a.zr_pts = p->d_zr_pts; a.zr_pq = p->d_zr_pq; a.n_spec_pts = p->zr_npts; a.zr_n_units = p->zr_units;
     a.cluster = p->cluster;
     a.cluster_ctas = p->cluster_ctas;
     a.status = p->d_status;
@@ -665,7 +701,7 @@ Status launch_stage(Plan* p, int stage, const T* f0, typename Cx<T>::type* F, co
     const bool planes = stage == 0 || stage == 5;
     Status s = sizeof(T) == 4 ? (planes ? fast_planes_f32(a, err) : fast_other_f32(a, err))
                               : (planes ? fast_planes_f64(a, err) : fast_other_f64(a, err));
-    g_launches += (stage == 3 && p->reps_quad && !q_step) ? 2 : 1;  // regroup + gather
+    ++g_launches;
     return s;
   }
   switch (stage) {
@@ -831,6 +867,148 @@ static long q_of_channel_point(const PlanTables& T, int c, int x, int y, int z) 
   if (!T.centered) return x + static_cast<long>(T.M[0]) * (y + static_cast<long>(T.M[1]) * z);
   const auto& o = T.offsets[c];
   return (2 * x + o[0]) + static_cast<long>(T.M[0]) * ((2 * y + o[1]) + static_cast<long>(T.M[1]) * (2 * z + o[2]));
+}
+
+// Fibers of the inverse gather (k_inv_fiber).  Orbits are taken in order; an orbit not
+// yet served opens a fiber whose taps are its own alias row, and the fiber also serves the
+// orbit of each image R_b^T q whose row, written out as a linear form in the spectrum
+// (index, conjugation, phase), equals the fiber's Walsh-Hadamard row; where an operation
+// takes h to -h, conj F(h) = e^{2 pi i h.t / N} F(h) of a real symmetric field first writes
+// conjugated terms as plain ones.  The two gathers then agree for every such field, and
+// operation lists that are no group fall back to one fiber per orbit.  Fibers are ordered
+// by 4 x 4 x 4 blocks of their first spectral point: a permutation of the axes relates the
+// taps of neighbouring fibers, so a block keeps every tap's reads within a few sectors.
+// Returns the fiber count; tables are [m][fiber].
+static int build_fibers(const PlanTables& T, const std::vector<int2>& expand, std::vector<uint2>* taps,
+                        std::vector<uint2>* outs) {
+  const int d = T.d, P = T.P;
+  const size_t no = T.orbit_rep.size();
+  const long hvol = static_cast<long>(T.H[0]) * T.H[1] * T.H[2];
+  // parity classes in the order of the aliases (first axis of stride 2 fastest)
+  auto class_of = [&](const long* t) {
+    int c = 0, w = 1;
+    for (int k = 0; k < 3; ++k)
+      if (T.L[k] == 2) { c += w * static_cast<int>(t[k] & 1); w *= 2; }
+    return c;
+  };
+  std::vector<int> cls(d);
+  for (int b = 0; b < d; ++b) {
+    const long t[3] = {T.rep_ops[b].t[0], T.rep_ops[b].t[1], T.rep_ops[b].t[2]};
+    cls[b] = class_of(t);
+  }
+  // phase numerator c with conj F(h) = e^{2 pi i c / P} F(h), or -1.  The inversion, where
+  // the list has it, takes every h to -h.
+  std::vector<long> friedel(T.spec.size(), -1);
+  const SymOp* inversion = nullptr;
+  for (const auto& op : T.ops) {
+    bool neg = true;
+    for (int i = 0; i < 3; ++i)
+      for (int k = 0; k < 3; ++k) neg = neg && op.R[i][k] == (i == k ? (T.N[i] > 1 ? -1 : op.R[i][i]) : 0);
+    if (neg) { inversion = &op; break; }
+  }
+  for (size_t s = 0; s < T.spec.size(); ++s) {
+    const auto& h = T.spec[s].h;
+    const SymOp* found = inversion;
+    for (size_t o = 0; o < T.ops.size() && !found; ++o) {
+      bool neg = true;
+      for (int k = 0; k < 3 && neg; ++k) {
+        long v = h[k];
+        for (int i = 0; i < 3; ++i) v += static_cast<long>(T.ops[o].R[i][k]) * h[i];
+        neg = floor_mod(v, T.N[k]) == 0;
+      }
+      if (neg) found = &T.ops[o];
+    }
+    if (!found) continue;
+    long c = 0;
+    for (int k = 0; k < 3; ++k) c += static_cast<long>(h[k]) * found->t[k] * (P / T.N[k]);
+    friedel[s] = floor_mod(c, P);
+  }
+  std::vector<char> served(no, 0);
+  std::vector<uint2> ft, fo;  // d entries per fiber
+  std::vector<uint64_t> row(d), form(d);  // (index | conjugate) << 32 | phase
+  auto word = [&](size_t k) {
+    const int sp = T.inv_spec[k];
+    return static_cast<uint32_t>(sp < 0 ? -sp : sp) | (sp < 0 ? 0x80000000u : 0u);
+  };
+  auto term = [&](uint32_t w, long j) {  // 0 for an extinct tap
+    if (!w) return uint64_t{0};
+    if (w >> 31) {
+      const long c = friedel[(w & 0x7FFFFFFFu) - 1];
+      if (c >= 0) { w &= 0x7FFFFFFFu; j += c; }
+    }
+    return (static_cast<uint64_t>(w) << 32) | static_cast<uint64_t>(floor_mod(j, P));
+  };
+  for (size_t o = 0; o < no; ++o) {
+    if (served[o]) continue;
+    long m = T.orbit_rep[o], q[3];
+    q[0] = m % T.M[0]; m /= T.M[0]; q[1] = m % T.M[1]; q[2] = m / T.M[1];
+    ft.resize(ft.size() + d);
+    fo.resize(fo.size() + d, make_uint2(0u, 0u));
+    uint2* tp = &ft[ft.size() - d];
+    uint2* op = &fo[fo.size() - d];
+    for (int a = 0; a < d; ++a) tp[a] = make_uint2(word(o * d + a), static_cast<uint32_t>(T.inv_phase[o * d + a]));
+    for (int b = 0; b < d; ++b) {
+      long idx[3], jt = 0;
+      for (int k = 0; k < 3; ++k) {
+        long v = 0;
+        for (int i = 0; i < 3; ++i) v += static_cast<long>(T.rep_ops[b].R[i][k]) * q[i];
+        idx[k] = floor_mod(v, T.M[k]);
+        jt += q[k] * T.rep_ops[b].t[k] * (P / T.N[k]);
+      }
+      long pos;
+      if (T.centered) {
+        const int c = T.chan_of_parity[(idx[0] & 1) + 2 * (idx[1] & 1) + 4 * (idx[2] & 1)];
+        if (c < 0) continue;
+        pos = c * hvol + ((idx[2] >> 1) * T.H[1] + (idx[1] >> 1)) * T.H[0] + (idx[0] >> 1);
+      } else {
+        pos = (idx[2] * T.H[1] + idx[1]) * T.H[0] + idx[0];
+      }
+      const int2 ex = expand[pos];
+      if (ex.x < 0 || served[ex.x]) continue;
+      const long jo = floor_mod(jt - ex.y, P);
+      // Walsh-Hadamard row b times the output phase, against the orbit's own alias row.
+      bool sharable = P % 2 == 0 || cls[b] == 0;
+      for (int a = 0; a < d && sharable; ++a) {
+        const int flip = __builtin_popcount(cls[b] & a) & 1;
+        form[a] = term(tp[a].x, static_cast<long>(tp[a].y) + jo + (flip ? P / 2 : 0));
+        const size_t k = static_cast<size_t>(ex.x) * d + a;
+        row[a] = term(word(k), T.inv_phase[k]);
+      }
+      if (!sharable) continue;
+      std::sort(form.begin(), form.end());
+      std::sort(row.begin(), row.end());
+      if (form != row) continue;
+      served[ex.x] = 1;
+      op[cls[b]] = make_uint2(static_cast<uint32_t>(ex.x) + 1u, static_cast<uint32_t>(jo));
+    }
+    if (!served[o]) {  // the orbit itself: sum of its row, no phase
+      served[o] = 1;
+      op[0] = make_uint2(static_cast<uint32_t>(o) + 1u, 0u);
+    }
+  }
+  const size_t nf = ft.size() / d;
+  std::vector<std::pair<uint64_t, size_t>> order(nf);
+  for (size_t f = 0; f < nf; ++f) {
+    uint64_t key = ~0ull;
+    for (int a = 0; a < d; ++a)
+      if (const uint32_t w = ft[f * d + a].x & 0x7FFFFFFFu) {
+        const auto& h = T.spec[w - 1].h;
+        key = 0;
+        for (int k = 0; k < 3; ++k) key = (key << 10) | static_cast<uint64_t>(h[k] >> 2);
+        for (int k = 0; k < 3; ++k) key = (key << 2) | static_cast<uint64_t>(h[k] & 3);
+        break;
+      }
+    order[f] = {key, f};
+  }
+  std::sort(order.begin(), order.end());
+  taps->resize(nf * d);
+  outs->resize(nf * d);
+  for (size_t f = 0; f < nf; ++f)
+    for (int a = 0; a < d; ++a) {
+      (*taps)[a * nf + f] = ft[order[f].second * d + a];
+      (*outs)[a * nf + f] = fo[order[f].second * d + a];
+    }
+  return static_cast<int>(nf);
 }
 
 Status plan_device_init(Plan* p, std::string* err) {
@@ -999,37 +1177,28 @@ Status plan_device_init(Plan* p, std::string* err) {
   if ((st = alloc(&p->d_work_T, p->lanes * p->w_lane_bytes, "channel workspace")) != Status::kOk) return st;
   if ((st = alloc(&p->d_work_F, B * T.spec.size() * cs, "spectrum workspace")) != Status::kOk) return st;
   if ((st = alloc(&p->d_work_E, B * mvol * rs, "interaction workspace")) != Status::kOk) return st;
-  // Packed alias rows (spec+1 in 20 bits, conj, phase in 11 bits) for the quad gather.
-  std::vector<uint32_t> inv_pk;
   p->reps_quad = p->fast_h && T.spec.size() < (1u << 20) - 1 && T.P <= 2048 && T.orbit_rep.size() < (1u << 21);
+  std::vector<uint2> fib_taps, fib_outs;
   if (p->reps_quad) {
-    inv_pk.resize(T.inv_spec.size());
-    for (size_t k = 0; k < inv_pk.size(); ++k) {
-      const int sp = T.inv_spec[k];
-      const uint32_t a = static_cast<uint32_t>(sp < 0 ? -sp : sp);
-      inv_pk[k] = a | (sp < 0 ? (1u << 20) : 0u) | (static_cast<uint32_t>(T.inv_phase[k]) << 21);
-    }
-    if ((st = alloc(&p->d_inv_pk, inv_pk.size() * 4, "packed inverse table")) != Status::kOk) return st;
+    p->n_fib = build_fibers(T, expand, &fib_taps, &fib_outs);
+    if ((st = alloc(&p->d_fib_taps, fib_taps.size() * sizeof(uint2), "fiber taps")) != Status::kOk) return st;
+    if ((st = alloc(&p->d_fib_outs, fib_outs.size() * sizeof(uint2), "fiber outputs")) != Status::kOk) return st;
   }
   if (p->fast_h) {
-    // The quad path reads the expansion entries packed in 32 bits (orbit | phase << 21).
+    // Packed expansion entries (orbit | phase << 21) where they fit 32 bits.
     if ((st = alloc(&p->d_expand, expand.size() * (p->reps_quad ? 4 : sizeof(int2)), "expansion table")) != Status::kOk)
       return st;
-    // Wide groups (16 FP32 / 8 FP64 fields per line) once a chunk fills one group; the
-    // fused cluster kernels read the quad layout, so CFFT_CLUSTER keeps quads.
+    // Rows of 64 bytes (8 FP32 / 4 FP64 slots) once a chunk fills one; the fused cluster
+    // kernels read rows of 2 slots, so CFFT_CLUSTER keeps those.
     const size_t gw = 128 / cs;
     const char* wide_env = std::getenv("CFFT_WIDE");
     const char* cl_env = std::getenv("CFFT_CLUSTER");
     const bool cluster_wanted = p->tune.cluster >= 0 ? p->tune.cluster > 0 : (cl_env && std::atoi(cl_env) > 0);
     const bool wide_wanted = p->tune.wide >= 0 ? p->tune.wide > 0 : !(wide_env && wide_env[0] == '0');
     p->reps_wide = p->reps_quad && chunk >= gw && wide_wanted && !cluster_wanted;
-    const size_t chunk4 = p->reps_wide ? (chunk + gw - 1) / gw * gw : (chunk + 3) / 4 * 4;  // whole groups of fields
+    const size_t chunk4 = p->reps_wide ? (chunk + gw - 1) / gw * gw : (chunk + 3) / 4 * 4;  // whole rows of slots
     p->g0r_lane_bytes = (((p->reps_quad ? chunk4 : chunk + 1) * T.orbit_rep.size() * cs + 255) / 256) * 256;
     if ((st = alloc(&p->d_g0r, p->lanes * p->g0r_lane_bytes, "representative workspace")) != Status::kOk) return st;
-    if (p->reps_quad) {
-      p->ft_lane_bytes = ((chunk4 * T.spec.size() * cs + 255) / 256) * 256;
-      if ((st = alloc(&p->d_ft, p->lanes * p->ft_lane_bytes, "grouped spectra")) != Status::kOk) return st;
-    }
   }
   // Q-matrix step (M2Q / M7): runs on the compile-time sized kernels only.
   if (p->qmode) {
@@ -1104,10 +1273,12 @@ Status plan_device_init(Plan* p, std::string* err) {
   } else if (p->fast_h) {
     CFFT_CUDA(cudaMemcpy(p->d_expand, expand.data(), expand.size() * sizeof(int2), cudaMemcpyHostToDevice), "upload expansion");
   }
-  if (p->reps_quad)
-    CFFT_CUDA(cudaMemcpy(p->d_inv_pk, inv_pk.data(), inv_pk.size() * 4, cudaMemcpyHostToDevice), "upload packed table");
+  if (p->n_fib) {
+    CFFT_CUDA(cudaMemcpy(p->d_fib_taps, fib_taps.data(), fib_taps.size() * sizeof(uint2), cudaMemcpyHostToDevice), "upload fiber taps");
+    CFFT_CUDA(cudaMemcpy(p->d_fib_outs, fib_outs.data(), fib_outs.size() * sizeof(uint2), cudaMemcpyHostToDevice), "upload fiber outputs");
+  }
   if (p->fast_h && p->rep_diag8 && !p->qmode) {
-    Status zs = build_zrecon_units(p, err);
+    Status zs = build_zrecon_units(p, g, err);
     if (zs != Status::kOk) return zs;
   }
   // Orbit expansion writes only alive positions; channel positions never written stay zero.
@@ -1238,8 +1409,8 @@ Status plan_upload_kernel(Plan* p, std::string* err) {
 void plan_device_free(Plan* p) {
   void** bufs[] = {&p->d_geom, &p->d_tables, &p->d_spec_h, &p->d_K, &p->d_orbit_rep, &p->d_inv_spec,
                    &p->d_inv_phase, &p->d_img_mask, &p->d_fill_map, &p->d_work_T, &p->d_work_F,
-                   &p->d_work_E, &p->d_stage_in, &p->d_stage_out, &p->d_expand, &p->d_g0r, &p->d_inv_pk, &p->d_ft,
-                   &p->d_qt, &p->d_gt, &p->d_work_Q, &p->d_zr_units, &p->d_zr_pts, &p->d_qsep};
+                   &p->d_work_E, &p->d_stage_in, &p->d_stage_out, &p->d_expand, &p->d_g0r, &p->d_fib_taps, &p->d_fib_outs,
+                   &p->d_qt, &p->d_gt, &p->d_work_Q, &p->d_zr_units, &p->d_zr_pts, &p->d_zr_pq, &p->d_qsep};
   for (void** b : bufs)
     if (*b) { cudaFree(*b); *b = nullptr; }
   if (p->h_status) { cudaFreeHost(p->h_status); p->h_status = nullptr; p->d_status = nullptr; }

@@ -44,10 +44,13 @@ struct Plan {
   void* d_stage_out = nullptr;
   void* d_expand = nullptr;     // fast path: per channel position (orbit index, phase numerator)
   void* d_g0r = nullptr;        // fast path: G0 at orbit representatives (per lane)
-  void* d_ft = nullptr;         // packed backward path: spectra regrouped in quads of fields (per lane)
-  void* d_inv_pk = nullptr;     // fast path: packed alias table for the shared-memory gather
+  void* d_fib_taps = nullptr;   // inverse gather by fibers: d x n_fib taps (uint2, k_inv_fiber)
+  void* d_fib_outs = nullptr;   // and d x n_fib outputs
+  int n_fib = 0;
   void* d_zr_units = nullptr;   // fused z FFT + gather: uint4 per unit (c | ya | yb, first point, count)
-  void* d_zr_pts = nullptr;     // fused z FFT + gather: spectral indices grouped by unit
+  void* d_zr_pts = nullptr;     // fused z FFT + gather: (spectral index, packed h) grouped by unit
+  void* d_zr_pq = nullptr;      // fused z FFT + gather: tap-pair weights [4][point] (two complex each)
+  int zr_npts = 0;
   void* own_stream = nullptr;
   static constexpr int kMaxLanes = 4;
   void* lane_stream[kMaxLanes] = {};  // concurrent chunk lanes (fork/join on the caller's stream)
@@ -60,7 +63,7 @@ struct Plan {
   void* d2h_stream = nullptr;
   void* ev_in[kHostPieces] = {};
   void* ev_done[kHostPieces] = {};
-  size_t w_lane_bytes = 0, g0r_lane_bytes = 0, ft_lane_bytes = 0;
+  size_t w_lane_bytes = 0, g0r_lane_bytes = 0;
   size_t workspace_bytes = 0;
   // launch geometry
   int threads_xy = 0, threads_z = 0;
@@ -70,8 +73,8 @@ struct Plan {
   int cent_type = 0;            // plane-kernel centring (0 plain, 1 I, 2 F, 3 C, 4 A)
   bool rep_perm = false;        // representative ops are signed permutations
   bool rep_diag8 = false;       // representative ops are the 8 diagonal sign matrices
-  bool reps_quad = false;       // packed alias rows; fields gathered and expanded in quads
-  bool reps_wide = false;       // the same in groups of 128 / sizeof(complex) fields (one line per point)
+  bool reps_quad = false;       // packed expansion entries; representatives in rows of 2 slots
+  bool reps_wide = false;       // the same in rows of 64 bytes (8 FP32 / 4 FP64 slots)
   bool zrecon = false;          // forward z FFT fused with the diagonal-sign gather (stage 6)
   int zr_units = 0;             // units of the fused kernel (channel + mirrored row pair)
   bool cluster = false;         // fused cluster kernels: fold+xyz FFT and expand+xyz IFFT+unfold

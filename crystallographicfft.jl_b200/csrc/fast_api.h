@@ -17,11 +17,12 @@ struct FastArgs {
   const void* K = nullptr;
   const void* inv_spec = nullptr;
   const void* inv_phase = nullptr;
-  const void* inv_pk = nullptr;
+  const void* fib_taps = nullptr;  // inverse gather by fibers: taps and outputs (uint2)
+  const void* fib_outs = nullptr;
+  int n_fib = 0;
   const void* expand = nullptr;
   void* W = nullptr;      // channel workspace of this lane
   void* G0R = nullptr;    // representative workspace of this lane
-  void* FT = nullptr;     // quad-grouped spectra of this lane (packed backward path)
   // call operands
   const void* f0 = nullptr;
   void* F = nullptr;
@@ -32,10 +33,12 @@ struct FastArgs {
   int stage = 0, nb = 0, H = 0, n_ch = 1, centered = 0, cent_type = 0, d = 1;
   int n_spec = 0, n_orbits = 0;
   bool use_K = false, rep_diag8 = false, rep_perm = false, reps_quad = false;
-  bool reps_wide = false;  // backward gather in groups of 128 / sizeof(complex) fields
+  bool reps_wide = false;  // representatives in rows of 64 bytes (8 FP32 / 4 FP64 slots), else 2 slots
   // Stage 6 (fused z FFT + diagonal-sign gather): unit table and spectral points.
   const void* zr_units = nullptr;
-  const void* zr_pts = nullptr;
+  const void* zr_pts = nullptr;   // (spectral index, packed h) per point, in unit order
+  const void* zr_pq = nullptr;    // weights of the four tap pairs per point
+  int n_spec_pts = 0;             // points in the unit lists
   int zr_n_units = 0;
   bool cluster = false;   // fused cluster kernels for stages 0 (with 1) and 5 (with 4)
   int cluster_ctas = 8;   // CTAs per cluster (8, or 16 where the device allows it)

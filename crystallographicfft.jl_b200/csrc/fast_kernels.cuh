@@ -132,18 +132,36 @@ template <int CT> struct Cent {
 // builds X = G_a + i G_b and the unfold reads field a from the real part and field b
 // from the imaginary part.  This halves the FFT work and the workspace traffic.
 
-// Row / column FFTs of nch padded planes for a group of threads (gtid of gnth).
-template <typename C, bool INV, int H>
+// Place of column x in a row that is written or read VW consecutive values per thread:
+// value l of thread m sits at l * (H / VW) + m, so the lanes of a warp access
+// neighbouring words (natural order makes them VW-way bank conflicts).  The x-line pass,
+// one row per thread, takes either order at no cost.
+template <int H, int VW> constexpr __host__ __device__ int fold_pos(int x) { return (x % VW) * (H / VW) + x / VW; }
+
+// Item e of the vector fold and unfold: columns ix0 .. ix0 + VW - 1 of row iy.  The rows a
+// warp touches lie H / (rows per warp) apart: with the odd row stride their words then
+// fall into different banks (adjacent rows overlap in all but one).
+template <int H, int VW> __device__ __forceinline__ void fold_item(int e, int* ix0, int* iy) {
+  constexpr int PR = H / VW;                                  // items per row
+  constexpr int RW = PR < 32 && 32 % PR == 0 && H % (32 / PR) == 0 ? 32 / PR : 1;  // rows per warp
+  const int r = e / PR;
+  *ix0 = (e % PR) * VW;
+  *iy = (r % RW) * (H / RW) + r / RW;
+}
+
+// Row / column FFTs of nch padded planes for a group of threads (gtid of gnth); rows are
+// read in fold_pos<H, PI> order and left in fold_pos<H, PO> order.
+template <typename C, bool INV, int H, int PI = 1, int PO = 1>
 __device__ __forceinline__ void group_rows(C* buf, int nlines, int tid, int nth) {
   constexpr int S = H + 1;
   for (int l = tid; l < nlines; l += nth) {
     C* p = buf + l * S;
     C v[H];
 #pragma unroll
-    for (int i = 0; i < H; ++i) v[i] = p[i];
+    for (int i = 0; i < H; ++i) v[i] = p[fold_pos<H, PI>(i)];
     reg_fft<C, INV, H>(v);
 #pragma unroll
-    for (int i = 0; i < H; ++i) p[i] = v[i];
+    for (int i = 0; i < H; ++i) p[fold_pos<H, PO>(i)] = v[i];
   }
 }
 template <typename C, bool INV, int H>
@@ -163,8 +181,8 @@ __device__ __forceinline__ void group_cols(C* buf, int nlines, int tid, int nth)
 // Fold of VW consecutive x values (ix0 .. ix0 + VW - 1) of channel row iy: the eight
 // octant values of fields a and b (va[k], vb[k], octant k = kx + 2 ky + 4 kz) go through
 // the WHT8, each alive channel takes its fold twiddle, and the results land in the
-// padded planes at buf.
-template <typename T, int H, int CT, int VW>
+// padded planes at buf (PV > 1: columns at fold_pos<H, PV>).
+template <typename T, int H, int CT, int VW, int PV = 1>
 __device__ __forceinline__ void fold_emit(const T (&va)[8][VW], const T (&vb)[8][VW], int ix0, int iy,
                                           const typename Cx<T>::type* __restrict__ ftx,
                                           typename Cx<T>::type ftz, typename Cx<T>::type* buf) {
@@ -189,7 +207,7 @@ __device__ __forceinline__ void fold_emit(const T (&va)[8][VW], const T (&vb)[8]
       if (o & 1) w = tx;
       if (o & 2) w = cmul(w, ty);
       if (o & 4) w = cmul(w, ftz);
-      buf[c * PL + iy * S + ix] = o ? cmul(p8[o], w) : p8[o];
+      buf[c * PL + iy * S + fold_pos<H, PV>(ix)] = o ? cmul(p8[o], w) : p8[o];
     }
   }
 }
@@ -198,7 +216,7 @@ __device__ __forceinline__ void fold_emit(const T (&va)[8][VW], const T (&vb)[8]
 // the nch padded planes at buf (channel c at buf + c * H * (H + 1)), with the fold
 // twiddles e^{-2 pi i off.n / M} and the interaction factors E when given.  Work is
 // spread over threads tid of nth.
-template <typename T, int H, int CT>
+template <typename T, int H, int CT, int PV = 1>
 __device__ __forceinline__ void fold_plane(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
                                            const T* __restrict__ srca, const T* __restrict__ srcb,
                                            const T* __restrict__ Ea, const T* __restrict__ Eb, bool has_b, bool USE_E,
@@ -214,7 +232,7 @@ __device__ __forceinline__ void fold_plane(const DevGeom* __restrict__ g, const 
       T va = srca[zoff + e];
       T vb = has_b ? srcb[zoff + e] : zero;
       if (USE_E) { va *= Ea[zoff + e]; if (has_b) vb *= Eb[zoff + e]; }
-      buf[(e / H) * S + (e % H)] = mk<C>(va, vb);
+      buf[(e / H) * S + fold_pos<H, PV>(e % H)] = mk<C>(va, vb);
     }
   } else {
     constexpr int M = 2 * H;
@@ -226,7 +244,8 @@ __device__ __forceinline__ void fold_plane(const DevGeom* __restrict__ g, const 
                      (!USE_E || reinterpret_cast<uintptr_t>(Ea) % 16 == 0);
     if (vec) {
       for (int e = tid; e < H * H / VW; e += nth) {
-        const int ix0 = (e % (H / VW)) * VW, iy = e / (H / VW);
+        int ix0, iy;
+        fold_item<H, VW>(e, &ix0, &iy);
         T va[8][VW], vb[8][VW];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -249,7 +268,7 @@ __device__ __forceinline__ void fold_plane(const DevGeom* __restrict__ g, const 
             }
           }
         }
-        fold_emit<T, H, CT, VW>(va, vb, ix0, iy, ftx, ftz, buf);
+        fold_emit<T, H, CT, VW, PV>(va, vb, ix0, iy, ftx, ftz, buf);
       }
     } else {
       for (int e = tid; e < H * H; e += nth) {
@@ -272,17 +291,28 @@ __device__ __forceinline__ void fold_plane(const DevGeom* __restrict__ g, const 
           if (o & 1) w = tx;
           if (o & 2) w = cmul(w, ty);
           if (o & 4) w = cmul(w, ftz);
-          buf[c * PL + iy * S + ix] = cmul(mk<C>(va[o], vb[o]), w);
+          buf[c * PL + iy * S + fold_pos<H, PV>(ix)] = cmul(mk<C>(va[o], vb[o]), w);
         }
       }
     }
   }
 }
 
+// v / V for the inverse transform's normalisation.  1/V rounded to FP32 is off by 7.5e-9
+// for edges with a factor 3, the same way in every step of a contour loop (7.5e-7 after a
+// hundred); its remainder as a second term makes the product correct to a rounding, which
+// does not accumulate.  Powers of two have no remainder.
+template <typename T, int V> __device__ __forceinline__ T div_const(T v) {
+  constexpr T hi = static_cast<T>(1.0 / V);
+  constexpr T lo = sizeof(T) == 4 ? static_cast<T>(1.0 / V - static_cast<double>(hi)) : static_cast<T>(0);
+  if constexpr (lo == static_cast<T>(0)) return v * hi;
+  else return fma(v, hi, v * lo);
+}
+
 // Unfold of the nch inverse-transformed planes at buf (channel z-plane iz) into the two
 // fields of the slot: conjugate fold twiddle, inverse WHT8 / 8, real part -> field a,
 // imaginary part -> field b, times E when given.
-template <typename T, int H, int CT, bool VEC = false>
+template <typename T, int H, int CT, bool VEC = false, int PV = 1>
 __device__ __forceinline__ void unfold_plane(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
                                              const typename Cx<T>::type* buf, T* __restrict__ dsta, T* __restrict__ dstb,
                                              const T* __restrict__ Ea, const T* __restrict__ Eb, bool has_b, bool USE_E,
@@ -291,21 +321,19 @@ __device__ __forceinline__ void unfold_plane(const DevGeom* __restrict__ g, cons
   constexpr int S = H + 1;
   constexpr int PL = H * S;
   constexpr int nch = Cent<CT>::n;
-  const size_t hvol = static_cast<size_t>(H) * H * H;
-  const size_t mvol = static_cast<size_t>(g->M[0]) * g->M[1] * g->M[2];
   if constexpr (CT == 0) {
-    const T scale = static_cast<T>(1.0 / static_cast<double>(mvol));
+    constexpr int V = H * H * H;
     const size_t zoff = static_cast<size_t>(iz) * H * H;
     for (int e = tid; e < H * H; e += nth) {
-      const C x = buf[(e / H) * S + (e % H)];
-      T va = x.x * scale, vb = x.y * scale;
+      const C x = buf[(e / H) * S + fold_pos<H, PV>(e % H)];
+      T va = div_const<T, V>(x.x), vb = div_const<T, V>(x.y);
       if (USE_E) { va *= Ea[zoff + e]; if (has_b) vb *= Eb[zoff + e]; }
       dsta[zoff + e] = va;
       if (has_b) dstb[zoff + e] = vb;
     }
   } else {
     constexpr int M = 2 * H;
-    const T scale = static_cast<T>(1.0 / (8.0 * static_cast<double>(hvol)));
+    constexpr int V = 8 * H * H * H;
     const C* ftx = tables + g->ftw_off[0];
     const C ftz = tables[g->ftw_off[2] + iz];
     constexpr int VW = 16 / static_cast<int>(sizeof(T));  // elements per 16-byte vector
@@ -315,7 +343,8 @@ __device__ __forceinline__ void unfold_plane(const DevGeom* __restrict__ g, cons
     if (vec) {
       // VW consecutive x values per thread; each octant row piece leaves as one 16-byte store.
       for (int e = tid; e < H * H / VW; e += nth) {
-        const int ix0 = (e % (H / VW)) * VW, iy = e / (H / VW);
+        int ix0, iy;
+        fold_item<H, VW>(e, &ix0, &iy);
         const C ty = ftx[iy];
         T oa[8][VW], ob[8][VW];
 #pragma unroll
@@ -332,14 +361,14 @@ __device__ __forceinline__ void unfold_plane(const DevGeom* __restrict__ g, cons
             if (o & 1) w = tx;
             if (o & 2) w = cmul(w, ty);
             if (o & 4) w = cmul(w, ftz);
-            const C y = cmulc(buf[c * PL + iy * S + ix], w);
+            const C y = cmulc(buf[c * PL + iy * S + fold_pos<H, PV>(ix)], w);
             va[o] = y.x;
             vb[o] = y.y;
           }
           wht8(va);
           wht8(vb);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) { oa[k][l] = va[k] * scale; ob[k][l] = vb[k] * scale; }
+          for (int k = 0; k < 8; ++k) { oa[k][l] = div_const<T, V>(va[k]); ob[k][l] = div_const<T, V>(vb[k]); }
         }
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -373,7 +402,7 @@ __device__ __forceinline__ void unfold_plane(const DevGeom* __restrict__ g, cons
           if (o & 1) w = tx;
           if (o & 2) w = cmul(w, ty);
           if (o & 4) w = cmul(w, ftz);
-          const C y = cmulc(buf[c * PL + iy * S + ix], w);  // x * conj(w)
+          const C y = cmulc(buf[c * PL + iy * S + fold_pos<H, PV>(ix)], w);  // x * conj(w)
           va[o] = y.x;
           vb[o] = y.y;
         }
@@ -382,7 +411,7 @@ __device__ __forceinline__ void unfold_plane(const DevGeom* __restrict__ g, cons
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const int idx = ((iz + ((k >> 2) & 1) * H) * M + iy + ((k >> 1) & 1) * H) * M + ix + (k & 1) * H;
-          T a = va[k] * scale, bq = vb[k] * scale;
+          T a = div_const<T, V>(va[k]), bq = div_const<T, V>(vb[k]);
           if (USE_E) { a *= Ea[idx]; if (has_b) bq *= Eb[idx]; }
           dsta[idx] = a;
           if (has_b) dstb[idx] = bq;
@@ -413,55 +442,11 @@ __device__ __forceinline__ void y_lines_to_workspace(const C* buf, C* __restrict
   }
 }
 
-// Forward plane kernel, cubic H: fold (or plain load) of two fields + x FFT + y FFT
-// -> W[slot][c][z][y][x].
-template <typename T, int H, int CT>
-__global__ void k_plane_fwd_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
-                              const T* __restrict__ f0, const T* __restrict__ E, typename Cx<T>::type* __restrict__ W,
-                              int nfields) {
-  pdl_enter();
-  using C = typename Cx<T>::type;
-  constexpr int nch = Cent<CT>::n;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* buf = reinterpret_cast<C*>(smem_raw);
-  const int iz = blockIdx.x, slot = blockIdx.y;
-  const int fa = 2 * slot;
-  const bool has_b = fa + 1 < nfields;
-  const bool USE_E = E != nullptr;  // warp-uniform
-  const int tid = threadIdx.x, nth = blockDim.x;
-  const size_t mvol = static_cast<size_t>(g->M[0]) * g->M[1] * g->M[2];
-  const T* srca = f0 + static_cast<size_t>(fa) * mvol;
-  const T* Ea = USE_E ? E + static_cast<size_t>(fa) * mvol : nullptr;
-  fold_plane<T, H, CT>(g, tables, srca, srca + mvol, Ea, USE_E ? Ea + mvol : nullptr, has_b, USE_E, iz, buf, tid, nth);
-  __syncthreads();
-  group_rows<C, false, H>(buf, nch * H, tid, nth);   // x lines
-  __syncthreads();
-  constexpr int HV = H * H * H;
-  y_lines_to_workspace<C, H, nch>(buf, W + static_cast<size_t>(slot) * nch * HV + iz * H * H, tid, nth);
-}
-
-// Backward plane kernel, cubic H: inverse x/y FFT of W[slot][c][iz] + unfold of the two
-// fields (real part -> field a, imaginary part -> field b).
-template <typename T, int H, int CT, bool VEC>
-__global__ void k_plane_bwd_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
-                              const typename Cx<T>::type* __restrict__ W, const T* __restrict__ E, T* __restrict__ f0,
-                              int nfields) {
-  pdl_enter();
-  using C = typename Cx<T>::type;
-  constexpr int S = H + 1;
-  constexpr int PL = H * S;
-  constexpr int nch = Cent<CT>::n;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* buf = reinterpret_cast<C*>(smem_raw);
-  const int iz = blockIdx.x, slot = blockIdx.y;
-  const int fa = 2 * slot;
-  const bool has_b = fa + 1 < nfields;
-  const bool USE_E = E != nullptr;  // warp-uniform
-  const int tid = threadIdx.x, nth = blockDim.x;
-  constexpr int HV = H * H * H;
-  // y lines straight from the workspace into registers (coalesced across x), inverse
-  // FFT, into shared memory; then the x lines there.
-  const C* src0 = W + static_cast<size_t>(slot) * nch * HV + iz * H * H;
+// y lines of the nch planes at src0 (channel stride H^3) straight into registers (coalesced
+// across x), inverse FFT, into the padded planes at buf.
+template <typename C, int H, int nch>
+__device__ __forceinline__ void inverse_y_lines(const C* __restrict__ src0, C* buf, int tid, int nth) {
+  constexpr int S = H + 1, PL = H * S, HV = H * H * H;
   for (int l = tid; l < nch * H; l += nth) {
     const int c = l / H, x = l % H;
     const C* q = src0 + static_cast<size_t>(c) * HV + x;
@@ -473,19 +458,480 @@ __global__ void k_plane_bwd_h(const DevGeom* __restrict__ g, const typename Cx<T
 #pragma unroll
     for (int i = 0; i < H; ++i) p[i * S] = v[i];
   }
-  __syncthreads();
-  // Last read of these workspace planes: drop their lines from L2 without a write-back.
+}
+// After the last read of those planes: drop their lines from L2 without a write-back.
+template <typename C, int H, int nch>
+__device__ __forceinline__ void discard_planes(const C* src0, int tid, int nth) {
   if constexpr ((H * H * sizeof(C)) % 128 == 0) {
-    constexpr int LPP = static_cast<int>(H * H * sizeof(C) / 128);
+    constexpr int HV = H * H * H, LPP = static_cast<int>(H * H * sizeof(C) / 128);
     for (int i = tid; i < nch * LPP; i += nth)
       discard_l2_line(reinterpret_cast<const char*>(src0 + static_cast<size_t>(i / LPP) * HV) + (i % LPP) * 128);
   }
-  group_rows<C, true, H>(buf, nch * H, tid, nth);
+}
+
+// Values per thread of the centred fold and unfold's vector path (the fold_pos order of
+// their rows); 1 where that path does not apply.
+template <typename T, int H, int CT> constexpr int row_vec() {
+  constexpr int v = 16 / static_cast<int>(sizeof(T));
+  return CT != 0 && H % v == 0 ? v : 1;
+}
+
+// Threads of the line-per-thread plane kernels: one per line, in warps, at least two warps;
+// two warps more where that saves the fold a round (H = 24: 144 items on 160 threads instead
+// of 96 or 128).  Measured, Ia-3d 96^3 FP32 contour steps of 256 fields, us for three: 637 /
+// 680 / 620 / 693 with 96 / 128 / 160 / 192 threads; Im-3m 64^3 FP32 round trips of 256
+// fields: 40.7 / 43.9 with 64 / 128; Pmmm 64^3 FP64, 256 fields: 217 / 229 with 64 / 128.
+template <typename T> inline int plane_line_threads(int H, int nch, bool folded) {
+  constexpr int v = 16 / static_cast<int>(sizeof(T));
+  const int base = std::max(64, ((nch * H + 31) / 32) * 32);
+  const int items = H * H / (H % v == 0 ? v : 1);
+  const auto rounds = [&](int t) { return (items + t - 1) / t; };
+  return folded && rounds(base + 64) < rounds(base) && rounds(base + 64) <= 2 ? base + 64 : base;
+}
+
+// Forward plane kernel, cubic H: fold (or plain load) of two fields + x FFT + y FFT
+// -> W[slot][c][z][y][x].
+template <typename T, int H, int CT>
+__global__ void k_plane_fwd_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+                              const T* __restrict__ f0, const T* __restrict__ E, typename Cx<T>::type* __restrict__ W,
+                              int nfields) {
+  pdl_enter();
+  using C = typename Cx<T>::type;
+  constexpr int nch = Cent<CT>::n, PV = row_vec<T, H, CT>();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* buf = reinterpret_cast<C*>(smem_raw);
+  const int iz = blockIdx.x, slot = blockIdx.y;
+  const int fa = 2 * slot;
+  const bool has_b = fa + 1 < nfields;
+  const bool USE_E = E != nullptr;  // warp-uniform
+  const int tid = threadIdx.x, nth = blockDim.x;
+  const size_t mvol = static_cast<size_t>(g->M[0]) * g->M[1] * g->M[2];
+  const T* srca = f0 + static_cast<size_t>(fa) * mvol;
+  const T* Ea = USE_E ? E + static_cast<size_t>(fa) * mvol : nullptr;
+  fold_plane<T, H, CT, PV>(g, tables, srca, srca + mvol, Ea, USE_E ? Ea + mvol : nullptr, has_b, USE_E, iz, buf, tid, nth);
+  __syncthreads();
+  group_rows<C, false, H, PV, 1>(buf, nch * H, tid, nth);   // x lines
+  __syncthreads();
+  constexpr int HV = H * H * H;
+  y_lines_to_workspace<C, H, nch>(buf, W + static_cast<size_t>(slot) * nch * HV + iz * H * H, tid, nth);
+}
+
+// Backward plane kernel, cubic H: inverse x/y FFT of W[slot][c][iz] + unfold of the two
+// fields (real part -> field a, imaginary part -> field b).
+template <typename T, int H, int CT>
+__global__ void k_plane_bwd_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+                              const typename Cx<T>::type* __restrict__ W, const T* __restrict__ E, T* __restrict__ f0,
+                              int nfields) {
+  pdl_enter();
+  using C = typename Cx<T>::type;
+  constexpr int nch = Cent<CT>::n, PV = row_vec<T, H, CT>();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* buf = reinterpret_cast<C*>(smem_raw);
+  const int iz = blockIdx.x, slot = blockIdx.y;
+  const int fa = 2 * slot;
+  const bool has_b = fa + 1 < nfields;
+  const bool USE_E = E != nullptr;  // warp-uniform
+  const int tid = threadIdx.x, nth = blockDim.x;
+  constexpr int HV = H * H * H;
+  const C* src0 = W + static_cast<size_t>(slot) * nch * HV + iz * H * H;
+  inverse_y_lines<C, H, nch>(src0, buf, tid, nth);
+  __syncthreads();
+  discard_planes<C, H, nch>(src0, tid, nth);
+  group_rows<C, true, H, 1, PV>(buf, nch * H, tid, nth);
   __syncthreads();
   const size_t mvol = static_cast<size_t>(g->M[0]) * g->M[1] * g->M[2];
   T* dsta = f0 + static_cast<size_t>(fa) * mvol;
   const T* Ea = USE_E ? E + static_cast<size_t>(fa) * mvol : nullptr;
-  unfold_plane<T, H, CT, VEC>(g, tables, buf, dsta, dsta + mvol, Ea, USE_E ? Ea + mvol : nullptr, has_b, USE_E, iz, tid, nth);
+  unfold_plane<T, H, CT, true, PV>(g, tables, buf, dsta, dsta + mvol, Ea, USE_E ? Ea + mvol : nullptr, has_b, USE_E, iz, tid, nth);
+}
+
+// ---------------------------------------------------------------- split lines
+// A line of H = A x B points is transformed by two register passes through shared
+// memory, in place: pass 1 takes the B butterflies of A points {j + B r}, multiplies
+// output k1 by e^{-2 pi i j k1 / H} and writes it back to position j + B k1; pass 2 takes
+// the A butterflies of B points {B k1 + j} and leaves frequency k1 + A k2 at position
+// B k1 + k2 (line_pos).  A butterfly holds at most 8 values, so a plane is worked by
+// four to eight times the threads of a line-per-thread kernel, at about half the
+// registers: the plane and z kernels wait on memory, not on arithmetic, and need warps.
+template <int H> constexpr int split_a() { return H == 12 || H == 16 ? 4 : H == 24 ? 6 : H >= 32 ? 8 : H; }
+template <int H> constexpr int split_b() { return H / split_a<H>(); }
+template <int H> __device__ __forceinline__ int line_pos(int k) {
+  constexpr int A = split_a<H>(), B = split_b<H>();
+  return B == 1 ? k : (k % A) * B + k / A;
+}
+
+// Twiddles e^{-2 pi i k / H} of the plan's tables into shared memory (lanes of a warp mostly
+// share an index, but not for every H: constant memory would replay those reads).
+template <typename C, int H>
+__device__ __forceinline__ void load_line_twiddles(const DevGeom* __restrict__ g, const C* __restrict__ tables, C* tw) {
+  if constexpr (split_b<H>() > 1)
+    for (int i = threadIdx.x; i < H; i += blockDim.x) tw[i] = __ldg(tables + g->tw_off[0] + i);
+}
+
+// Butterfly j of pass 1 on the values v (already loaded): DFT_A and the twiddles.
+template <typename C, bool INV, int H>
+__device__ __forceinline__ void split_pass1(C (&v)[split_a<H>()], int j, const C* tw) {
+  constexpr int A = split_a<H>();
+  reg_fft<C, INV, A>(v);
+  if constexpr (split_b<H>() > 1) {
+#pragma unroll
+    for (int k = 1; k < A; ++k) {
+      const C t = tw[j * k];
+      v[k] = INV ? cmulc(v[k], t) : cmul(v[k], t);
+    }
+  }
+}
+
+// In-place passes over `nlines` lines (line l at base(l), element stride ES) by all
+// threads; consecutive threads take consecutive lines.
+template <typename C, bool INV, int H, int ES, typename Base>
+__device__ __forceinline__ void split_pass1_smem(C* buf, int nlines, Base base, const C* tw) {
+  constexpr int A = split_a<H>(), B = split_b<H>();
+  for (int i = threadIdx.x; i < nlines * B; i += blockDim.x) {
+    const int j = i / nlines;
+    C* p = buf + base(i - j * nlines) + j * ES;
+    C v[A];
+#pragma unroll
+    for (int r = 0; r < A; ++r) v[r] = p[r * B * ES];
+    split_pass1<C, INV, H>(v, j, tw);
+#pragma unroll
+    for (int r = 0; r < A; ++r) p[r * B * ES] = v[r];
+  }
+}
+template <typename C, bool INV, int H, int ES, typename Base>
+__device__ __forceinline__ void split_pass2_smem(C* buf, int nlines, Base base) {
+  constexpr int A = split_a<H>(), B = split_b<H>();
+  if constexpr (B > 1) {
+    for (int i = threadIdx.x; i < nlines * A; i += blockDim.x) {
+      const int k1 = i / nlines;
+      C* p = buf + base(i - k1 * nlines) + k1 * B * ES;
+      C v[B];
+#pragma unroll
+      for (int r = 0; r < B; ++r) v[r] = p[r * ES];
+      reg_fft<C, INV, B>(v);
+#pragma unroll
+      for (int r = 0; r < B; ++r) p[r * ES] = v[r];
+    }
+  }
+}
+
+// Values per thread and octant row of the fold and the unfold: 8-byte accesses (two
+// floats, one double).  Wider ones need twice the registers for the eight octants of two
+// fields, which costs the resident warps more than the wider accesses give.
+template <typename T> constexpr int fold_width() { return 8 / static_cast<int>(sizeof(T)); }
+template <typename T, int VW> __device__ __forceinline__ void vw_load_stream(T (&o)[VW], const T* p) {
+  if constexpr (VW == 2 && sizeof(T) == 4) {
+    const float2 v = __ldcs(reinterpret_cast<const float2*>(p));
+    o[0] = v.x; o[1] = v.y;
+  } else {
+#pragma unroll
+    for (int l = 0; l < VW; ++l) o[l] = __ldcs(p + l);
+  }
+}
+template <typename T, int VW> __device__ __forceinline__ void vw_load(T (&o)[VW], const T* p) {
+  if constexpr (VW == 2 && sizeof(T) == 4) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    o[0] = v.x; o[1] = v.y;
+  } else {
+#pragma unroll
+    for (int l = 0; l < VW; ++l) o[l] = p[l];
+  }
+}
+template <typename T, int VW> __device__ __forceinline__ void vw_store_stream(T* p, const T (&o)[VW]) {
+  if constexpr (VW == 2 && sizeof(T) == 4) __stcs(reinterpret_cast<float2*>(p), make_float2(o[0], o[1]));
+  else {
+#pragma unroll
+    for (int l = 0; l < VW; ++l) __stcs(p + l, o[l]);
+  }
+}
+
+// Fold (or plain load) of the two fields of a slot at channel z-plane iz, VW consecutive
+// x values per thread and step, into the nch planes at buf (row stride H + 1).
+template <typename T, int H, int CT, int VW>
+__device__ __forceinline__ void fold_rows(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+                                          const T* __restrict__ srca, const T* __restrict__ srcb,
+                                          const T* __restrict__ Ea, const T* __restrict__ Eb, bool has_b, bool USE_E,
+                                          int iz, typename Cx<T>::type* buf) {
+  using C = typename Cx<T>::type;
+  constexpr int S = H + 1;
+  const T zero = static_cast<T>(0);
+  if constexpr (CT == 0) {
+    const int zoff = iz * H * H;
+    for (int e = threadIdx.x; e < H * H / VW; e += blockDim.x) {
+      const int ix0 = (e % (H / VW)) * VW, iy = e / (H / VW);
+      const int idx = zoff + iy * H + ix0;
+      T va[VW], vb[VW], ea[VW];
+      vw_load_stream<T, VW>(va, srca + idx);
+#pragma unroll
+      for (int l = 0; l < VW; ++l) vb[l] = zero;
+      if (has_b) vw_load_stream<T, VW>(vb, srcb + idx);
+      if (USE_E) {
+        vw_load<T, VW>(ea, Ea + idx);
+#pragma unroll
+        for (int l = 0; l < VW; ++l) va[l] *= ea[l];
+        if (has_b) {
+          vw_load<T, VW>(ea, Eb + idx);
+#pragma unroll
+          for (int l = 0; l < VW; ++l) vb[l] *= ea[l];
+        }
+      }
+#pragma unroll
+      for (int l = 0; l < VW; ++l) buf[iy * S + ix0 + l] = mk<C>(va[l], vb[l]);
+    }
+  } else {
+    constexpr int M = 2 * H;
+    const C* ftx = tables + g->ftw_off[0];
+    const C ftz = tables[g->ftw_off[2] + iz];
+    for (int e = threadIdx.x; e < H * H / VW; e += blockDim.x) {
+      const int ix0 = (e % (H / VW)) * VW, iy = e / (H / VW);
+      T va[8][VW], vb[8][VW];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int idx = ((iz + ((k >> 2) & 1) * H) * M + iy + ((k >> 1) & 1) * H) * M + ix0 + (k & 1) * H;
+        vw_load_stream<T, VW>(va[k], srca + idx);
+#pragma unroll
+        for (int l = 0; l < VW; ++l) vb[k][l] = zero;
+        if (has_b) vw_load_stream<T, VW>(vb[k], srcb + idx);
+      }
+      if (USE_E) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int idx = ((iz + ((k >> 2) & 1) * H) * M + iy + ((k >> 1) & 1) * H) * M + ix0 + (k & 1) * H;
+          T ea[VW];
+          vw_load<T, VW>(ea, Ea + idx);
+#pragma unroll
+          for (int l = 0; l < VW; ++l) va[k][l] *= ea[l];
+          if (has_b) {
+            vw_load<T, VW>(ea, Eb + idx);
+#pragma unroll
+            for (int l = 0; l < VW; ++l) vb[k][l] *= ea[l];
+          }
+        }
+      }
+      fold_emit<T, H, CT, VW>(va, vb, ix0, iy, ftx, ftz, buf);
+    }
+  }
+}
+
+// Unfold of the nch inverse-transformed planes at buf (x and y in line_pos order) into
+// the two fields of the slot: conjugate fold twiddle, inverse WHT8 / 8, real part ->
+// field a, imaginary part -> field b, times E when given.
+template <typename T, int H, int CT, int VW>
+__device__ __forceinline__ void unfold_rows(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+                                            const typename Cx<T>::type* buf, T* __restrict__ dsta, T* __restrict__ dstb,
+                                            const T* __restrict__ Ea, const T* __restrict__ Eb, bool has_b, bool USE_E,
+                                            int iz) {
+  using C = typename Cx<T>::type;
+  constexpr int S = H + 1;
+  constexpr int PL = H * S;
+  constexpr int nch = Cent<CT>::n;
+  if constexpr (CT == 0) {
+    constexpr int V = H * H * H;
+    for (int e = threadIdx.x; e < H * H / VW; e += blockDim.x) {
+      const int ix0 = (e % (H / VW)) * VW, iy = e / (H / VW);
+      const int idx = iz * H * H + iy * H + ix0;
+      T va[VW], vb[VW], ea[VW];
+#pragma unroll
+      for (int l = 0; l < VW; ++l) {
+        const C x = buf[line_pos<H>(iy) * S + line_pos<H>(ix0 + l)];
+        va[l] = div_const<T, V>(x.x);
+        vb[l] = div_const<T, V>(x.y);
+      }
+      if (USE_E) {
+        vw_load<T, VW>(ea, Ea + idx);
+#pragma unroll
+        for (int l = 0; l < VW; ++l) va[l] *= ea[l];
+        if (has_b) {
+          vw_load<T, VW>(ea, Eb + idx);
+#pragma unroll
+          for (int l = 0; l < VW; ++l) vb[l] *= ea[l];
+        }
+      }
+      vw_store_stream<T, VW>(dsta + idx, va);
+      if (has_b) vw_store_stream<T, VW>(dstb + idx, vb);
+    }
+  } else {
+    constexpr int M = 2 * H;
+    constexpr int V = 8 * H * H * H;
+    const C* ftx = tables + g->ftw_off[0];
+    const C ftz = tables[g->ftw_off[2] + iz];
+    for (int e = threadIdx.x; e < H * H / VW; e += blockDim.x) {
+      const int ix0 = (e % (H / VW)) * VW, iy = e / (H / VW);
+      const C ty = ftx[iy];
+      const C* row = buf + line_pos<H>(iy) * S;
+      T oa[8][VW], ob[8][VW];
+#pragma unroll
+      for (int l = 0; l < VW; ++l) {
+        const C tx = ftx[ix0 + l];
+        const int px = line_pos<H>(ix0 + l);
+        C p8[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) p8[k] = mk<C>(static_cast<T>(0), static_cast<T>(0));
+#pragma unroll
+        for (int c = 0; c < nch; ++c) {
+          const int o = Cent<CT>::off(c);
+          C w = mk<C>(static_cast<T>(1), static_cast<T>(0));
+          if (o & 1) w = tx;
+          if (o & 2) w = cmul(w, ty);
+          if (o & 4) w = cmul(w, ftz);
+          p8[o] = o ? cmulc(row[c * PL + px], w) : row[c * PL + px];
+        }
+        wht8c(p8);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { oa[k][l] = div_const<T, V>(p8[k].x); ob[k][l] = div_const<T, V>(p8[k].y); }
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int idx = ((iz + ((k >> 2) & 1) * H) * M + iy + ((k >> 1) & 1) * H) * M + ix0 + (k & 1) * H;
+        if (USE_E) {
+          T ea[VW];
+          vw_load<T, VW>(ea, Ea + idx);
+#pragma unroll
+          for (int l = 0; l < VW; ++l) oa[k][l] *= ea[l];
+          if (has_b) {
+            vw_load<T, VW>(ea, Eb + idx);
+#pragma unroll
+            for (int l = 0; l < VW; ++l) ob[k][l] *= ea[l];
+          }
+        }
+        vw_store_stream<T, VW>(dsta + idx, oa[k]);
+        if (has_b) vw_store_stream<T, VW>(dstb + idx, ob[k]);
+      }
+    }
+  }
+}
+
+// Threads of the split plane kernels: enough for the pass-1 butterflies in one to three
+// rounds, on the plain path also for the plane's values in two, at most 512.
+template <int H, int CT> constexpr int split_threads() {
+  constexpr int n = CT == 0 && H * H / 2 > H * split_b<H>() ? H * H / 2 : Cent<CT>::n * H * split_b<H>();
+  constexpr int t = n <= 512 ? n : (n + 1) / 2 <= 512 ? (n + 1) / 2 : (n + 2) / 3;
+  return t < 64 ? 64 : ((t + 31) / 32) * 32;
+}
+template <typename T, int H, int CT> constexpr int split_blocks() {
+  constexpr int by_threads = (sizeof(T) == 4 ? 1024 : 768) / split_threads<H, CT>();
+  constexpr int by_smem = static_cast<int>((220 * 1024) / (Cent<CT>::n * H * (H + 1) * 2 * sizeof(T) + 1024));
+  constexpr int b = by_threads < by_smem ? by_threads : by_smem;
+  return b < 1 ? 1 : b > 8 ? 8 : b;
+}
+
+// Forward plane kernel, cubic H: fold (or plain load) of two fields + x FFT + y FFT
+// -> W[slot][c][z][y][x].
+template <typename T, int H, int CT>
+__global__ void __launch_bounds__(split_threads<H, CT>(), split_blocks<T, H, CT>())
+k_plane_fwd_s(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+              const T* __restrict__ f0, const T* __restrict__ E, typename Cx<T>::type* __restrict__ W, int nfields) {
+  pdl_enter();
+  using C = typename Cx<T>::type;
+  constexpr int nch = Cent<CT>::n, S = H + 1, PL = H * S, A = split_a<H>(), B = split_b<H>(), HV = H * H * H;
+  constexpr int VW = H % fold_width<T>() == 0 ? fold_width<T>() : 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* buf = reinterpret_cast<C*>(smem_raw);
+  C* tw = buf + nch * PL;
+  load_line_twiddles<C, H>(g, tables, tw);
+  const int iz = blockIdx.x, slot = blockIdx.y;
+  const int fa = 2 * slot;
+  const bool has_b = fa + 1 < nfields;
+  const bool USE_E = E != nullptr;  // warp-uniform
+  constexpr size_t mvol = static_cast<size_t>(CT ? 8 : 1) * HV;
+  const T* srca = f0 + static_cast<size_t>(fa) * mvol;
+  const T* Ea = USE_E ? E + static_cast<size_t>(fa) * mvol : nullptr;
+  const T* Eb = USE_E ? Ea + mvol : nullptr;
+  // Rows hold an even number of values, so the caller's base decides the alignment.
+  if (VW == 1 || ((reinterpret_cast<uintptr_t>(f0) | reinterpret_cast<uintptr_t>(E)) & 7u) == 0)
+    fold_rows<T, H, CT, VW>(g, tables, srca, srca + mvol, Ea, Eb, has_b, USE_E, iz, buf);
+  else
+    fold_rows<T, H, CT, 1>(g, tables, srca, srca + mvol, Ea, Eb, has_b, USE_E, iz, buf);
+  __syncthreads();
+  auto row = [](int l) { return l * S; };                          // line (c, y)
+  auto col = [](int l) { return (l / H) * PL + (l % H); };         // line (c, x position)
+  split_pass1_smem<C, false, H, 1>(buf, nch * H, row, tw);
+  __syncthreads();
+  if constexpr (B > 1) {
+    split_pass2_smem<C, false, H, 1>(buf, nch * H, row);
+    __syncthreads();
+    split_pass1_smem<C, false, H, S>(buf, nch * H, col, tw);
+    __syncthreads();
+  }
+  // Last pass straight to the workspace: butterfly k1 of column (c, x position) holds the
+  // rows k1 + A r.
+  C* dst0 = W + static_cast<size_t>(slot) * nch * HV + iz * H * H;
+  constexpr int R = B > 1 ? B : A, NB = H / R;
+  for (int i = threadIdx.x; i < nch * H * NB; i += blockDim.x) {
+    const int k1 = i / (nch * H), l = i - k1 * (nch * H);
+    const int c = l / H, px = l % H;
+    const C* p = buf + c * PL + px + k1 * R * S;
+    C v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = p[r * S];
+    reg_fft<C, false, R>(v);
+    const int kx = B > 1 ? px / B + A * (px % B) : px;
+    C* d = dst0 + static_cast<size_t>(c) * HV + k1 * H + kx;
+#pragma unroll
+    for (int r = 0; r < R; ++r) d[r * NB * H] = v[r];
+  }
+}
+
+// Backward plane kernel, cubic H: inverse x/y FFT of W[slot][c][iz] + unfold of the two
+// fields (real part -> field a, imaginary part -> field b).
+template <typename T, int H, int CT>
+__global__ void __launch_bounds__(split_threads<H, CT>(), split_blocks<T, H, CT>())
+k_plane_bwd_s(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+              const typename Cx<T>::type* __restrict__ W, const T* __restrict__ E, T* __restrict__ f0, int nfields) {
+  pdl_enter();
+  using C = typename Cx<T>::type;
+  constexpr int nch = Cent<CT>::n, S = H + 1, PL = H * S, A = split_a<H>(), B = split_b<H>(), HV = H * H * H;
+  constexpr int VW = H % fold_width<T>() == 0 ? fold_width<T>() : 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* buf = reinterpret_cast<C*>(smem_raw);
+  C* tw = buf + nch * PL;
+  load_line_twiddles<C, H>(g, tables, tw);
+  const int iz = blockIdx.x, slot = blockIdx.y;
+  const int fa = 2 * slot;
+  const bool has_b = fa + 1 < nfields;
+  const bool USE_E = E != nullptr;  // warp-uniform
+  __syncthreads();
+  // First pass of the y lines straight from the workspace (coalesced across x).
+  const C* src0 = W + static_cast<size_t>(slot) * nch * HV + iz * H * H;
+  for (int i = threadIdx.x; i < nch * H * B; i += blockDim.x) {
+    const int j = i / (nch * H), l = i - j * (nch * H);
+    const int c = l / H, x = l % H;
+    const C* q = src0 + static_cast<size_t>(c) * HV + j * H + x;
+    C v[A];
+#pragma unroll
+    for (int r = 0; r < A; ++r) v[r] = q[r * B * H];
+    split_pass1<C, true, H>(v, j, tw);
+    C* p = buf + c * PL + j * S + x;
+#pragma unroll
+    for (int r = 0; r < A; ++r) p[r * B * S] = v[r];
+  }
+  __syncthreads();
+  // Last read of these workspace planes: drop their lines from L2 without a write-back.
+  if constexpr ((H * H * sizeof(C)) % 128 == 0) {
+    constexpr int LPP = static_cast<int>(H * H * sizeof(C) / 128);
+    for (int i = threadIdx.x; i < nch * LPP; i += blockDim.x)
+      discard_l2_line(reinterpret_cast<const char*>(src0 + static_cast<size_t>(i / LPP) * HV) + (i % LPP) * 128);
+  }
+  auto row = [](int l) { return l * S; };
+  auto col = [](int l) { return (l / H) * PL + (l % H); };
+  if constexpr (B > 1) {
+    split_pass2_smem<C, true, H, S>(buf, nch * H, col);
+    __syncthreads();
+  }
+  split_pass1_smem<C, true, H, 1>(buf, nch * H, row, tw);
+  __syncthreads();
+  if constexpr (B > 1) {
+    split_pass2_smem<C, true, H, 1>(buf, nch * H, row);
+    __syncthreads();
+  }
+  constexpr size_t mvol = static_cast<size_t>(CT ? 8 : 1) * HV;
+  T* dsta = f0 + static_cast<size_t>(fa) * mvol;
+  const T* Ea = USE_E ? E + static_cast<size_t>(fa) * mvol : nullptr;
+  const T* Eb = USE_E ? Ea + mvol : nullptr;
+  if (VW == 1 || ((reinterpret_cast<uintptr_t>(f0) | reinterpret_cast<uintptr_t>(E)) & 7u) == 0)
+    unfold_rows<T, H, CT, VW>(g, tables, buf, dsta, dsta + mvol, Ea, Eb, has_b, USE_E, iz);
+  else
+    unfold_rows<T, H, CT, 1>(g, tables, buf, dsta, dsta + mvol, Ea, Eb, has_b, USE_E, iz);
 }
 
 #include "tma_planes.cuh"
@@ -891,49 +1337,103 @@ __global__ void k_recon_diag8(const DevGeom* __restrict__ g, const typename Cx<T
 // operations (the taps of a spectral point h read G0 at the sign images of h, which lie
 // in one channel c on the rows y = p1 >> ls and its mirror y' = m1 >> ls).  A CTA
 // takes one unit (channel c and a mirrored pair of channel rows y_a, y_b; y_b < 0 when
-// the unit has one row) and ZR_SLOTS workspace slots:
-//   1. thread (slot, row, x) loads the z line W[slot][c][z][y_row][x] (coalesced across
-//      x), transforms it in registers and keeps it in shared memory [slot][row][x][z];
+// the unit has one row) and SL workspace slots:
+//   1. the z lines W[slot][c][z][y_row][x] (coalesced across x) are transformed and kept
+//      in shared memory [slot][row][x][z];
 //   2. the unit's spectral points (a list built at plan time) are gathered from shared
 //      memory as in k_recon_diag8 and written to F.
 // The transposed workspace of the separate z kernel is never written or read back.
 // Unit entry: x = c | y_a << 8 | (y_b + 1) << 16, y = first point, z = point count.
-template <int H> constexpr int zr_threads(int slots) { return slots * 2 * H < 32 ? 32 : ((slots * 2 * H + 31) / 32) * 32; }
-template <typename T, int H, int SL, bool USE_K>
-__global__ void k_fft_z_recon_diag8(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
-                                    const uint32_t* __restrict__ spec_h, const T* __restrict__ K,
-                                    const uint4* __restrict__ units, const uint32_t* __restrict__ pts,
-                                    const typename Cx<T>::type* __restrict__ W, typename Cx<T>::type* __restrict__ F,
-                                    int nfields) {
+// Points: pts[i] = (spectral index, packed h); weights pq[2 sg][i] = Pw, pq[2 sg + 1][i] = Qw
+// of the four Hermitian tap pairs (sg, 7 - sg): looking the eight phases up per point instead costs
+// eight divergent table reads for values that every slot and both fields share.
+// SPLIT: lines of two passes (see split_pass1) instead of one line per thread, for FP64 and
+// H = 48, where a line per thread leaves 8 to 11 warps on an SM, and for small launches.
+template <typename T, int H> constexpr bool zr_split() { return sizeof(T) == 8 || H > 32; }
+template <int H, int SL, bool SPLIT> constexpr int zr_threads() {
+  constexpr int n = SL * 2 * H * (SPLIT ? split_b<H>() : 1);
+  return n <= 64 ? 64 : SPLIT && n > 256 ? 256 : ((n + 31) / 32) * 32;
+}
+template <typename T, int H, int SL, bool SPLIT>
+__global__ void __launch_bounds__(zr_threads<H, SL, SPLIT>())
+k_fft_z_recon_diag8(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+                    const T* __restrict__ K, const uint4* __restrict__ units, const uint2* __restrict__ pts,
+                    const typename Cx<T>::type* __restrict__ pq, int npts,
+                    const typename Cx<T>::type* __restrict__ W, typename Cx<T>::type* __restrict__ F, int nfields) {
   pdl_enter();
   using C = typename Cx<T>::type;
-  constexpr int S = H + 1;
-  constexpr int HV = H * H * H;
+  constexpr int S = H + 1, HV = H * H * H, NTH = zr_threads<H, SL, SPLIT>(), NL = SL * 2 * H;
   constexpr int RS = H * S;  // one row of (x, z) lines
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);  // [slot][row][x][z] padded
-  __shared__ int sTP[8][3];
-  const int tid = threadIdx.x, nth = blockDim.x;
-  if (tid < 24) sTP[tid / 3][tid % 3] = g->rep_tp[g->sign_op[tid / 3]][tid % 3];
+  const int tid = threadIdx.x;
   const uint4 un = units[blockIdx.x];
   const int c = static_cast<int>(un.x & 0xFFu), ya = static_cast<int>((un.x >> 8) & 0xFFu);
   const int yb = static_cast<int>((un.x >> 16) & 0xFFu) - 1;
   const int slot0 = blockIdx.y * SL;
   const int nslots = (nfields + 1) / 2;
   const int nch = g->n_ch;
-  if (tid < SL * 2 * H) {
-    const int k = tid / (2 * H), r = (tid / H) & 1, x = tid % H;
-    const int slot = slot0 + k;
-    const int y = r ? yb : ya;
-    if (slot < nslots && y >= 0) {
-      const C* src = W + (static_cast<size_t>(slot) * nch + c) * HV + y * H + x;
-      C v[H];
+  if constexpr (!SPLIT) {
+    if (tid < NL) {
+      const int k = tid / (2 * H), r = (tid / H) & 1, x = tid % H;
+      const int slot = slot0 + k;
+      const int y = r ? yb : ya;
+      if (slot < nslots && y >= 0) {
+        const C* src = W + (static_cast<size_t>(slot) * nch + c) * HV + y * H + x;
+        C v[H];
 #pragma unroll
-      for (int z = 0; z < H; ++z) v[z] = src[static_cast<size_t>(z) * H * H];
-      reg_fft<C, false, H>(v);
-      C* row = buf + (k * 2 + r) * RS + x * S;
+        for (int z = 0; z < H; ++z) v[z] = src[static_cast<size_t>(z) * H * H];
+        reg_fft<C, false, H>(v);
+        C* row = buf + (k * 2 + r) * RS + x * S;
 #pragma unroll
-      for (int z = 0; z < H; ++z) row[z] = v[z];
+        for (int z = 0; z < H; ++z) row[z] = v[z];
+      }
+    }
+  } else {
+    constexpr int A = split_a<H>(), B = split_b<H>();
+    C* tw = buf + SL * 2 * RS;
+    load_line_twiddles<C, H>(g, tables, tw);
+    if constexpr (B > 1) __syncthreads();
+    for (int i = tid; i < NL * B; i += NTH) {
+      const int l = i % NL, j = i / NL;
+      const int k = l / (2 * H), r = (l / H) & 1, x = l % H;
+      const int slot = slot0 + k, y = r ? yb : ya;
+      if (slot < nslots && y >= 0) {
+        const C* src = W + (static_cast<size_t>(slot) * nch + c) * HV + y * H + x + j * H * H;
+        C v[A];
+#pragma unroll
+        for (int q = 0; q < A; ++q) v[q] = src[static_cast<size_t>(q) * B * H * H];
+        split_pass1<C, false, H>(v, j, tw);
+        C* row = buf + l * S + j;
+#pragma unroll
+        for (int q = 0; q < A; ++q) row[q * B] = v[q];
+      }
+    }
+    if constexpr (B > 1) {
+      // Pass 2 through registers, so the lines come out in natural order for the gather.
+      constexpr int R2 = (NL * A + NTH - 1) / NTH;
+      C v[R2][B];
+      __syncthreads();
+#pragma unroll
+      for (int t = 0; t < R2; ++t) {
+        const int i = tid + t * NTH, l = i % NL, k1 = i / NL;
+        if (k1 < A) {
+          const C* row = buf + l * S + k1 * B;
+#pragma unroll
+          for (int q = 0; q < B; ++q) v[t][q] = row[q];
+          reg_fft<C, false, B>(v[t]);
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int t = 0; t < R2; ++t) {
+        const int i = tid + t * NTH, l = i % NL, k1 = i / NL;
+        if (k1 < A) {
+          C* row = buf + l * S + k1;
+#pragma unroll
+          for (int q = 0; q < B; ++q) row[q * A] = v[t][q];
+        }
+      }
     }
   }
   __syncthreads();
@@ -941,7 +1441,7 @@ __global__ void k_fft_z_recon_diag8(const DevGeom* __restrict__ g, const typenam
   // again: drop its lines from L2 (rows that fill whole 128-byte lines only).
   if constexpr ((H * sizeof(C)) % 128 == 0) {
     constexpr int LPR = static_cast<int>(H * sizeof(C) / 128);
-    for (int i = tid; i < SL * 2 * H * LPR; i += nth) {
+    for (int i = tid; i < SL * 2 * H * LPR; i += NTH) {
       const int li = i % LPR, z = (i / LPR) % H, r = (i / (LPR * H)) & 1, k = i / (LPR * H * 2);
       const int slot = slot0 + k, y = r ? yb : ya;
       if (slot < nslots && y >= 0)
@@ -953,13 +1453,17 @@ __global__ void k_fft_z_recon_diag8(const DevGeom* __restrict__ g, const typenam
   const int M = cen ? 2 * H : H;
   const int ls = cen ? 1 : 0;
   const int ns = g->n_spec;
-  const C* ph = tables + g->ph_off;
-  const int P = g->P, pmask = g->pmask;
-  const T half = static_cast<T>(0.5);
   const int nvalid = min(SL, nslots - slot0);
-  for (int i = tid; i < static_cast<int>(un.z); i += nth) {
-    const uint32_t sidx = __ldg(pts + un.y + i);
-    const uint32_t hp = __ldg(spec_h + sidx);
+  for (int i = tid; i < static_cast<int>(un.z); i += NTH) {
+    const uint2 pt = __ldg(pts + un.y + i);
+    C Pw[4], Qw[4];
+#pragma unroll
+    for (int sg = 0; sg < 4; ++sg) {
+      const C* p = pq + static_cast<size_t>(2 * sg) * npts + un.y + i;
+      Pw[sg] = __ldg(p);
+      Qw[sg] = __ldg(p + npts);
+    }
+    const uint32_t sidx = pt.x, hp = pt.y;
     const int h0 = static_cast<int>(hp & 1023u), h1 = static_cast<int>((hp >> 10) & 1023u), h2 = static_cast<int>((hp >> 20) & 1023u);
     const int p0 = cen ? mod_m<2 * H>(h0) : mod_m<H>(h0);
     const int p1 = cen ? mod_m<2 * H>(h1) : mod_m<H>(h1);
@@ -968,24 +1472,7 @@ __global__ void k_fft_z_recon_diag8(const DevGeom* __restrict__ g, const typenam
     const int X0[2] = {(p0 >> ls) * S, (m0 >> ls) * S};
     const int X1[2] = {((p1 >> ls) != ya) * RS, ((m1 >> ls) != ya) * RS};
     const int X2[2] = {p2 >> ls, m2 >> ls};
-    C Pw[4], Qw[4];
-    {
-      C w[8];
-#pragma unroll
-      for (int sg = 0; sg < 8; ++sg) {
-        int j = h0 * sTP[sg][0] + h1 * sTP[sg][1] + h2 * sTP[sg][2];
-        j = pmask >= 0 ? (j & pmask) : ((j % P) + P) % P;
-        w[sg] = ph[j];
-      }
-      // Hermitian tap pairs (sg, 7 - sg), as in k_recon_diag8.
-#pragma unroll
-      for (int sg = 0; sg < 4; ++sg) {
-        const C u = w[sg], v = w[7 - sg];
-        Pw[sg] = mk<C>(half * (u.x + v.x), half * (u.y + v.y));
-        Qw[sg] = mk<C>(half * (v.y - u.y), half * (u.x - v.x));
-      }
-    }
-    const T kk = USE_K ? K[sidx] : static_cast<T>(1);
+    const T kk = K ? K[sidx] : static_cast<T>(1);
 #pragma unroll
     for (int k = 0; k < SL; ++k) {
       if (k >= nvalid) break;
@@ -1004,7 +1491,7 @@ __global__ void k_fft_z_recon_diag8(const DevGeom* __restrict__ g, const typenam
         accb.x = fma(a2, Pw[sg].x, fma(b2, Qw[sg].x, accb.x));
         accb.y = fma(a2, Pw[sg].y, fma(b2, Qw[sg].y, accb.y));
       }
-      if (USE_K) { acca = cscale(acca, kk); accb = cscale(accb, kk); }
+      if (K) { acca = cscale(acca, kk); accb = cscale(accb, kk); }
       const int fa = 2 * (slot0 + k);
       F[static_cast<size_t>(fa) * ns + sidx] = acca;
       if (fa + 1 < nfields) F[static_cast<size_t>(fa + 1) * ns + sidx] = accb;
@@ -1059,165 +1546,213 @@ __global__ void k_inv_recon_reps(const DevGeom* __restrict__ g, const typename C
   }
 }
 
-template <int D>
-__device__ __forceinline__ void load_alias_row(const uint32_t* __restrict__ inv_pk, int o, uint32_t (&e)[D]) {
-  if constexpr (D == 8) {
-    const uint4* p4 = reinterpret_cast<const uint4*>(inv_pk + static_cast<size_t>(o) * 8);
-    const uint4 u0 = __ldg(p4), u1 = __ldg(p4 + 1);
-    e[0] = u0.x; e[1] = u0.y; e[2] = u0.z; e[3] = u0.w; e[4] = u1.x; e[5] = u1.y; e[6] = u1.z; e[7] = u1.w;
-  } else if constexpr (D == 4) {
-    const uint4 u0 = __ldg(reinterpret_cast<const uint4*>(inv_pk + static_cast<size_t>(o) * 4));
-    e[0] = u0.x; e[1] = u0.y; e[2] = u0.z; e[3] = u0.w;
-  } else {
+// Walsh-Hadamard transform of D = 1, 2, 4 or 8 complex values.
+template <typename C, int D> __device__ __forceinline__ void wht_d(C (&v)[D]) {
 #pragma unroll
-    for (int a = 0; a < D; ++a) e[a] = __ldg(inv_pk + static_cast<size_t>(o) * D + a);
-  }
+  for (int s = 1; s < D; s <<= 1)
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+      if (!(i & s)) { const C a = v[i], b = v[i + s]; v[i] = cadd(a, b); v[i + s] = csub(a, b); }
 }
 
-// Four complex values (fields 4g .. 4g+3 of one spectral point or orbit) as 16-byte
-// vector loads / stores: 32 bytes for float, 64 for double.
-template <typename C>
-__device__ __forceinline__ void load_quad(const C* __restrict__ p, C (&v)[4]) {
-  if constexpr (sizeof(C) == 8) {
-    const float4 u0 = __ldg(reinterpret_cast<const float4*>(p)), u1 = __ldg(reinterpret_cast<const float4*>(p) + 1);
-    v[0] = mk<C>(u0.x, u0.y); v[1] = mk<C>(u0.z, u0.w); v[2] = mk<C>(u1.x, u1.y); v[3] = mk<C>(u1.z, u1.w);
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = __ldg(p + k);
-  }
-}
-template <typename C>
-__device__ __forceinline__ void store_quad(C* __restrict__ p, const C (&v)[4]) {
-  if constexpr (sizeof(C) == 8) {
-    reinterpret_cast<float4*>(p)[0] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
-    reinterpret_cast<float4*>(p)[1] = make_float4(v[2].x, v[2].y, v[3].x, v[3].y);
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) p[k] = v[k];
-  }
-}
-
-// Regroup the spectra of nb fields into quads: FT[q][s][k] = F[4q + k][s] (zero past
-// the last field), so one gather of a spectral point serves four fields with one
-// fully used 32-byte sector (float).  Coalesced on both sides; two spectral points per
-// thread, read as one 16-byte vector per field where the row allows it.
-template <typename T>
-__global__ void k_group_spectra(const typename Cx<T>::type* __restrict__ F, typename Cx<T>::type* __restrict__ FT,
-                                int ns, int nb) {
+// ---------------------------------------------------------------- inverse gather by fibers
+// The d aliases q + M m of a subgrid frequency q (its fiber) determine G0 at all d
+// images R_b^T q of the representative operations at once:
+//   e^{-2 pi i q.t_b / N} G0(R_b^T q) = (1/d) sum_m (-1)^{m . t_b} F(q + M m),
+// a Walsh-Hadamard transform of the d values, because the translations t_b run through
+// the parity classes once each.  One fiber therefore serves up to d orbits: its d spectrum
+// values are loaded once instead of once per orbit, and the d x d phases become d + d.
+// Taps (fiber-fastest, [m][fiber]): x = spectral index + 1 | conjugate << 31 (0: extinct),
+// y = phase numerator j, F(q + M m) = e^{2 pi i j / P} F[x] (conjugated first where
+// flagged).  Outputs ([b][fiber]): x = orbit + 1 (0: none), y = phase numerator.
+//
+// Each spectrum value is read about once, so the gather reads F field by field as the
+// caller stores it: a warp takes 32 fibers of one workspace slot, whose taps are near
+// neighbours in the spectral order.  The slot inputs X = G_a + i G_b of the L slots of a
+// group are exchanged through shared memory and leave as whole rows G0P[group][orbit][L]
+// for the expansion.  Im-3m 128^3 FP32, 64 fields: 7.5 + 15.0 us (regroup of the spectra
+// and one gather per orbit, 8 x the loads) before.
+constexpr int kFibers = 32;
+template <typename T, int D, int L>
+__global__ void __launch_bounds__(kFibers * L)
+k_inv_fiber(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+            const uint2* __restrict__ taps, const uint2* __restrict__ outs, int nf,
+            const typename Cx<T>::type* __restrict__ F, typename Cx<T>::type* __restrict__ G0P, int nb) {
   pdl_enter();
   using C = typename Cx<T>::type;
-  const int s0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
-  if (s0 >= ns) return;
-  const bool two = s0 + 1 < ns;
-  const int q = blockIdx.y;
-  const C z = mk<C>(static_cast<T>(0), static_cast<T>(0));
-  C v[2][4];
+  constexpr int RS = L + 1;
+  __shared__ C tile[D * kFibers * RS];
+  const int lane = threadIdx.x % kFibers, j = threadIdx.x / kFibers;
+  const int f0 = blockIdx.x * kFibers, f = f0 + lane;
+  const int gq = blockIdx.y;
+  const int fa = 2 * (gq * L + j);
+  const C* ph = tables + g->ph_off;
+  const int ns = g->n_spec;
+  const C zero = mk<C>(static_cast<T>(0), static_cast<T>(0));
+  C x[D];
+  if (f < nf && fa < nb) {
+    const C* Fa = F + static_cast<size_t>(fa) * ns;
+    const bool has_b = fa + 1 < nb;
+    uint2 t[D];
+    C va[D], vb[D];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int f = 4 * q + k;
-    const C* row = F + static_cast<size_t>(f) * ns + s0;
-    bool done = f >= nb;
-    if (done) { v[0][k] = z; v[1][k] = z; }
-    if constexpr (sizeof(C) == 8) {
-      if (!done && two && (reinterpret_cast<uintptr_t>(row) & 15u) == 0) {
-        const float4 u = __ldg(reinterpret_cast<const float4*>(row));
-        v[0][k] = make_float2(u.x, u.y);
-        v[1][k] = make_float2(u.z, u.w);
-        done = true;
+    for (int m = 0; m < D; ++m) t[m] = __ldg(taps + static_cast<size_t>(m) * nf + f);
+#pragma unroll
+    for (int m = 0; m < D; ++m) {
+      const uint32_t sp = t[m].x & 0x7FFFFFFFu;
+      va[m] = sp ? __ldg(Fa + sp - 1) : zero;
+      vb[m] = sp && has_b ? __ldg(Fa + ns + sp - 1) : zero;
+    }
+#pragma unroll
+    for (int m = 0; m < D; ++m) {
+      const T sg = (t[m].x >> 31) ? static_cast<T>(-1) : static_cast<T>(1);
+      const C v = mk<C>(va[m].x - sg * vb[m].y, sg * va[m].y + vb[m].x);
+      x[m] = cmulc(v, ph[t[m].y]);
+    }
+    wht_d<C, D>(x);
+  } else {
+#pragma unroll
+    for (int m = 0; m < D; ++m) x[m] = zero;
+  }
+  if (f < nf) {
+    const T inv_d = static_cast<T>(1.0 / static_cast<double>(D));
+#pragma unroll
+    for (int b = 0; b < D; ++b) {
+      const uint2 o = __ldg(outs + static_cast<size_t>(b) * nf + f);
+      if (o.x) tile[(b * kFibers + lane) * RS + j] = cscale(cmulc(x[b], ph[o.y]), inv_d);
+    }
+  }
+  __syncthreads();
+  const int no = g->n_orbits;
+  const int cnt = min(kFibers, nf - f0);
+  C* dst = G0P + static_cast<size_t>(gq) * no * L;
+#pragma unroll
+  for (int e = threadIdx.x; e < D * kFibers * L; e += kFibers * L) {
+    const int k = e % L, fb = (e / L) % kFibers, b = e / (L * kFibers);
+    if (fb < cnt) {
+      const uint32_t o = __ldg(outs + static_cast<size_t>(b) * nf + f0 + fb).x;
+      if (o) dst[static_cast<size_t>(o - 1) * L + k] = tile[(b * kFibers + fb) * RS + k];
+    }
+  }
+}
+
+// ---------------------------------------------------------------- orbit expansion + inverse z FFT
+// X(R^T q) = X(q_o) e^{2 pi i j / P} at every channel point from the packed entries (orbit
+// in bits 0-20, phase numerator in bits 21-31) and the rows G0P[group][orbit][L], then the
+// inverse z FFT -> W[slot][c][z][y][x].  A CTA takes one (y, c) and LS of the group's L
+// slots.  The lanes of a row fetch it in 16-byte pieces; the values meet their z lines in
+// shared memory, so the workspace stores run along x (storing straight from the fetching
+// lanes splits every store over eight slots).  SPLIT: lines of two passes (see
+// split_pass1), for FP64 and small launches, where one thread per line leaves too few
+// warps.
+template <typename C> constexpr int wide_slots() { return static_cast<int>(64 / sizeof(C)); }  // 8 FP32, 4 FP64
+template <typename C, int H, int L> constexpr int expand_slots() {
+  int ls = L;
+  while (ls > 2 && ls * H * H * static_cast<int>(sizeof(C)) > 72 * 1024) ls /= 2;
+  return ls;
+}
+template <int H> constexpr int expand_plane() { return ((H * H + 7) / 8) * 8 + 2; }
+template <typename C, int H, int LS> constexpr int expand_threads() {
+  constexpr int items = H * H * LS * static_cast<int>(sizeof(C)) / 16;
+  constexpr int t = items / 4 > LS * H ? items / 4 : LS * H;
+  return t <= 64 ? 64 : t >= 256 ? 256 : ((t + 31) / 32) * 32;
+}
+template <typename T, int H, int L, int LS, bool SPLIT>
+__global__ void __launch_bounds__(expand_threads<typename Cx<T>::type, H, LS>())
+k_expand_ifft_z(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+                const uint32_t* __restrict__ ETP, const typename Cx<T>::type* __restrict__ G0P,
+                typename Cx<T>::type* __restrict__ W, int nfields) {
+  pdl_enter();
+  using C = typename Cx<T>::type;
+  constexpr int HV = H * H * H, PS = expand_plane<H>(), NTH = expand_threads<C, H, LS>();
+  constexpr int SPV = 16 / static_cast<int>(sizeof(C)), NP = LS / SPV;  // slots per 16 bytes, pieces per row
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* buf = reinterpret_cast<C*>(smem_raw);  // [slot][z][x]
+  C* tw = buf + LS * PS;
+  if constexpr (SPLIT) load_line_twiddles<C, H>(g, tables, tw);
+  const int y = blockIdx.x, c = blockIdx.y, gq = blockIdx.z / (L / LS), part = blockIdx.z % (L / LS);
+  const int slot0 = gq * L + part * LS;
+  if (2 * slot0 >= nfields) return;
+  const uint32_t* et = ETP + static_cast<size_t>(c) * HV + y * H;
+  const C* rp = G0P + static_cast<size_t>(gq) * g->n_orbits * L + part * LS;
+  const C* ph = tables + g->ph_off;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < H * H * NP; i += NTH) {
+    const int p = i % NP, x = (i / NP) % H, z = i / (NP * H);
+    const uint32_t t = __ldg(et + z * H * H + x);
+    const C* src = rp + static_cast<size_t>(L) * (t & 0x1FFFFFu) + p * SPV;
+    const C w = ph[t >> 21];
+    C* d = buf + (p * SPV) * PS + z * H + x;
+    if constexpr (SPV == 2) {
+      const float4 u = __ldg(reinterpret_cast<const float4*>(src));
+      d[0] = cmulc(mk<C>(u.x, u.y), w);
+      d[PS] = cmulc(mk<C>(u.z, u.w), w);
+    } else {
+      d[0] = cmulc(__ldg(src), w);
+    }
+  }
+  __syncthreads();
+  C* dst = W + (static_cast<size_t>(slot0) * g->n_ch + c) * HV + y * H;
+  const size_t sstride = static_cast<size_t>(g->n_ch) * HV;
+  const int live = min(LS, (nfields + 1) / 2 - slot0);
+  if constexpr (!SPLIT) {
+    for (int i = threadIdx.x; i < LS * H; i += NTH) {
+      const int x = i % H, j = i / H;
+      const C* p = buf + j * PS + x;
+      C v[H];
+#pragma unroll
+      for (int z = 0; z < H; ++z) v[z] = p[z * H];
+      reg_fft<C, true, H>(v);
+      if (j < live) {
+        C* d = dst + j * sstride + x;
+#pragma unroll
+        for (int z = 0; z < H; ++z) d[z * H * H] = v[z];
       }
     }
-    if (!done) {
-      v[0][k] = __ldg(row);
-      v[1][k] = two ? __ldg(row + 1) : z;
+  } else {
+    constexpr int A = split_a<H>(), B = split_b<H>(), R = B > 1 ? B : A, NB = H / R;
+    if constexpr (B > 1) {
+      for (int i = threadIdx.x; i < LS * H * B; i += NTH) {
+        const int x = i % H, j = (i / H) % LS, jj = i / (H * LS);
+        C* p = buf + j * PS + jj * H + x;
+        C v[A];
+#pragma unroll
+        for (int r = 0; r < A; ++r) v[r] = p[r * B * H];
+        split_pass1<C, true, H>(v, jj, tw);
+#pragma unroll
+        for (int r = 0; r < A; ++r) p[r * B * H] = v[r];
+      }
+      __syncthreads();
+    }
+    for (int i = threadIdx.x; i < LS * H * NB; i += NTH) {
+      const int x = i % H, j = (i / H) % LS, k1 = i / (H * LS);
+      if (j >= live) continue;
+      const C* p = buf + j * PS + k1 * R * H + x;
+      C v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = p[r * H];
+      reg_fft<C, true, R>(v);
+      C* d = dst + j * sstride + static_cast<size_t>(k1) * H * H + x;
+#pragma unroll
+      for (int r = 0; r < R; ++r) d[static_cast<size_t>(r) * NB * H * H] = v[r];
     }
   }
-  store_quad(FT + (static_cast<size_t>(q) * ns + s0) * 4, v[0]);
-  if (two) store_quad(FT + (static_cast<size_t>(q) * ns + s0 + 1) * 4, v[1]);
 }
 
-// Backward inverse reconstruction for a quad of fields:
-//   G0(q_o) = (1/d) sum_a ph_a F(spec_a)   (F conjugated where flagged)
-// from the packed alias rows (spec+1 in bits 0-19, conj in bit 20, phase numerator in
-// bits 21-31; 0 = no alias).  Two consecutive lanes take one orbit: lane k reads fields
-// 4q + 2k and 4q + 2k + 1, one 16-byte half (float) of the spectral point's 32-byte
-// quad in FT, so every alias gather of a warp reads whole quads and the two fields of
-// a workspace slot sit in the same lane.  The d loads of a lane are independent and in
-// flight together.  Lane k stores the slot input X = G_a + i G_b of its pair as
-// G0P[q][o][k] (pair 0: fields 4q, 4q+1; pair 1: fields 4q+2, 4q+3).
-template <typename T, int D>
-__global__ void __launch_bounds__(256)
-k_inv_recon_quad(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
-                 const uint32_t* __restrict__ inv_pk, const typename Cx<T>::type* __restrict__ FT,
-                 typename Cx<T>::type* __restrict__ G0P) {
-  pdl_enter();
-  using C = typename Cx<T>::type;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int no = g->n_orbits;
-  const int o = t >> 1, k = t & 1;
-  if (o >= no) return;
-  const int q = blockIdx.y;
-  const C* ft = FT + static_cast<size_t>(q) * g->n_spec * 4 + 2 * k;
-  const C* ph = tables + g->ph_off;
-  uint32_t e[D];
-  load_alias_row<D>(inv_pk, o, e);
-  C v[D][2];
-#pragma unroll
-  for (int a = 0; a < D; ++a) {
-    const uint32_t sp = e[a] & 0xFFFFFu;
-    const C* src = ft + static_cast<size_t>(sp ? sp - 1 : 0) * 4;
-    if constexpr (sizeof(C) == 8) {
-      const float4 u = __ldg(reinterpret_cast<const float4*>(src));
-      v[a][0] = mk<C>(u.x, u.y);
-      v[a][1] = mk<C>(u.z, u.w);
-    } else {
-      v[a][0] = __ldg(src);
-      v[a][1] = __ldg(src + 1);
-    }
-  }
-  const T zero = static_cast<T>(0);
-  T re[2] = {zero, zero}, im[2] = {zero, zero};
-#pragma unroll
-  for (int a = 0; a < D; ++a) {
-    // term = v conj(w), or conj(v) conj(w) when flagged: with s = -1 if flagged,
-    // re = v.x w.x + v.y (s w.y), im = v.y (s w.x) - v.x w.y.
-    C w = ph[e[a] >> 21];
-    if ((e[a] & 0xFFFFFu) == 0) w = mk<C>(zero, zero);
-    const T sg = ((e[a] >> 20) & 1u) ? static_cast<T>(-1) : static_cast<T>(1);
-    const T cA = w.x, cB = sg * w.y, cC = sg * w.x, cD = -w.y;
-#pragma unroll
-    for (int f = 0; f < 2; ++f) {
-      re[f] = fma(v[a][f].x, cA, fma(v[a][f].y, cB, re[f]));
-      im[f] = fma(v[a][f].y, cC, fma(v[a][f].x, cD, im[f]));
-    }
-  }
-  const T inv_d = static_cast<T>(1.0 / static_cast<double>(D));
-  // X = G_a + i G_b; fields past the batch were zero-filled.
-  G0P[(static_cast<size_t>(q) * no + o) * 2 + k] = mk<C>(inv_d * (re[0] - im[1]), inv_d * (im[0] + re[1]));
-}
-
-// Backward orbit expansion + inverse z FFT for a quad of fields (two workspace
-// slots): the two halves of the CTA build the z lines of slots 2q and 2q+1 at the same
-// (y, x) positions, X_slot(R^T q) = X_slot(q_o) e^{+2 pi i j / P}, from the packed
-// expansion entries (orbit in bits 0-20, phase numerator in bits 21-31) and the
-// combined representatives G0P[q][o][pair]; both halves read the same entries and
-// 16-byte pairs (the second read hits L1).  The line is transformed in registers and
-// stored coalesced across x.  No shared memory.  A CTA covers YB y values.
+// The same for rows of two slots (small batches), one z line per thread straight from the
+// gather to the workspace, no shared memory: half of a CTA takes each slot, YB rows y.
 template <typename T, int H, int YB>
-__global__ void k_expand4_ifft_z_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
-                                   const uint32_t* __restrict__ ETP, const typename Cx<T>::type* __restrict__ G0P,
-                                   typename Cx<T>::type* __restrict__ W, int nfields) {
+__global__ void k_expand2_ifft_z(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+                                 const uint32_t* __restrict__ ETP, const typename Cx<T>::type* __restrict__ G0P,
+                                 typename Cx<T>::type* __restrict__ W, int nfields) {
   pdl_enter();
   using C = typename Cx<T>::type;
   constexpr int HV = H * H * H;
   constexpr int kHalf = ((YB * H + 31) / 32) * 32;
-  const int y0 = blockIdx.x * YB, c = blockIdx.y, q = blockIdx.z;
+  const int c = blockIdx.y, q = blockIdx.z;
   const int half = threadIdx.x / kHalf, r = threadIdx.x % kHalf;
-  const int slot = 2 * q + half;
-  if (2 * slot >= nfields) return;
-  const int ny = min(YB, H - y0);
-  const int yy = r / H, x = r % H;
-  if (yy >= ny) return;
-  const int y = y0 + yy;
+  const int slot = 2 * q + half, y = blockIdx.x * YB + r / H, x = r % H;
+  if (2 * slot >= nfields || r >= YB * H || y >= H) return;
   const uint32_t* et = ETP + static_cast<size_t>(c) * HV + y * H + x;
   const C* rp = G0P + static_cast<size_t>(q) * g->n_orbits * 2 + half;
   const C* ph = tables + g->ph_off;
@@ -1226,125 +1761,6 @@ __global__ void k_expand4_ifft_z_h(const DevGeom* __restrict__ g, const typename
   for (int z = 0; z < H; ++z) {
     const uint32_t t = __ldg(et + z * H * H);
     v[z] = cmulc(__ldg(rp + 2 * static_cast<size_t>(t & 0x1FFFFFu)), ph[t >> 21]);
-  }
-  reg_fft<C, true, H>(v);
-  C* dst = W + (static_cast<size_t>(slot) * g->n_ch + c) * HV + y * H + x;
-#pragma unroll
-  for (int z = 0; z < H; ++z) dst[z * H * H] = v[z];
-}
-
-// ---------------------------------------------------------------- wide backward gather
-// Field groups of GW = 128 / sizeof(complex) fields (16 in FP32, 8 in FP64): the
-// spectrum of a group keeps the GW values of one spectral point in one 128-byte line,
-// FT[g][s][k] = F[GW g + k][s], and the orbit representatives of a group keep their
-// GW / 2 workspace-slot inputs in one line, G0P[g][o][j] = X of slot GW/2 g + j.  Each
-// random gather of a warp then fetches whole lines that serve GW fields, a quarter of
-// the L1 wavefronts per useful byte of the quad layout.
-template <typename C> constexpr int wide_fields() { return static_cast<int>(128 / sizeof(C)); }
-constexpr int kWideTile = 128;  // spectral points per CTA of the regroup
-
-// Regroup of the spectra of nb fields into groups of GW: a CTA moves a tile of
-// kWideTile spectral points x GW fields through shared memory (row stride GW + 1, so
-// both phases are free of bank conflicts); reads are coalesced along each field's
-// row, writes are whole lines.  Fields past nb are zero.
-template <typename T>
-__global__ void __launch_bounds__(256) k_group_spectra_w(const typename Cx<T>::type* __restrict__ F,
-                                                         typename Cx<T>::type* __restrict__ FT, int ns, int nb) {
-  pdl_enter();
-  using C = typename Cx<T>::type;
-  constexpr int GW = wide_fields<C>(), SP = kWideTile, RS = GW + 1;
-  __shared__ C tile[SP * RS];
-  const int s0 = blockIdx.x * SP, gq = blockIdx.y;
-  const int np = min(SP, ns - s0);
-  const C z = mk<C>(static_cast<T>(0), static_cast<T>(0));
-  for (int e = threadIdx.x; e < SP * GW; e += blockDim.x) {
-    const int f = e / SP, i = e % SP;
-    const int field = gq * GW + f;
-    tile[i * RS + f] = (i < np && field < nb) ? __ldg(F + static_cast<size_t>(field) * ns + s0 + i) : z;
-  }
-  __syncthreads();
-  C* out = FT + (static_cast<size_t>(gq) * ns + s0) * GW;
-  for (int e = threadIdx.x; e < np * GW; e += blockDim.x) out[e] = tile[(e / GW) * RS + (e % GW)];
-}
-
-// Backward inverse reconstruction for a group of GW fields: as k_inv_recon_quad, with
-// GW / 2 lanes per orbit; lane j reads fields GW g + 2j and GW g + 2j + 1 (two
-// consecutive complex of the spectral point's line), so the lanes of an orbit read
-// each tap's line whole, and stores the slot input X = G_a + i G_b as G0P[g][o][j].
-template <typename T, int D>
-__global__ void __launch_bounds__(256)
-k_inv_recon_w(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
-              const uint32_t* __restrict__ inv_pk, const typename Cx<T>::type* __restrict__ FT,
-              typename Cx<T>::type* __restrict__ G0P) {
-  pdl_enter();
-  using C = typename Cx<T>::type;
-  constexpr int GW = wide_fields<C>(), L = GW / 2;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int no = g->n_orbits;
-  const int o = t / L, j = t % L;
-  if (o >= no) return;
-  const int gq = blockIdx.y;
-  const C* ft = FT + static_cast<size_t>(gq) * g->n_spec * GW + 2 * j;
-  const C* ph = tables + g->ph_off;
-  uint32_t e[D];
-  load_alias_row<D>(inv_pk, o, e);
-  C v[D][2];
-#pragma unroll
-  for (int a = 0; a < D; ++a) {
-    const uint32_t sp = e[a] & 0xFFFFFu;
-    const C* src = ft + static_cast<size_t>(sp ? sp - 1 : 0) * GW;
-    if constexpr (sizeof(C) == 8) {
-      const float4 u = __ldg(reinterpret_cast<const float4*>(src));
-      v[a][0] = mk<C>(u.x, u.y);
-      v[a][1] = mk<C>(u.z, u.w);
-    } else {
-      v[a][0] = __ldg(src);
-      v[a][1] = __ldg(src + 1);
-    }
-  }
-  const T zero = static_cast<T>(0);
-  T re[2] = {zero, zero}, im[2] = {zero, zero};
-#pragma unroll
-  for (int a = 0; a < D; ++a) {
-    C w = ph[e[a] >> 21];
-    if ((e[a] & 0xFFFFFu) == 0) w = mk<C>(zero, zero);
-    const T sg = ((e[a] >> 20) & 1u) ? static_cast<T>(-1) : static_cast<T>(1);
-    const T cA = w.x, cB = sg * w.y, cC = sg * w.x, cD = -w.y;
-#pragma unroll
-    for (int f = 0; f < 2; ++f) {
-      re[f] = fma(v[a][f].x, cA, fma(v[a][f].y, cB, re[f]));
-      im[f] = fma(v[a][f].y, cC, fma(v[a][f].x, cD, im[f]));
-    }
-  }
-  const T inv_d = static_cast<T>(1.0 / static_cast<double>(D));
-  G0P[(static_cast<size_t>(gq) * no + o) * L + j] = mk<C>(inv_d * (re[0] - im[1]), inv_d * (im[0] + re[1]));
-}
-
-// Backward orbit expansion + inverse z FFT for a group of GW fields (GW / 2 slots): a
-// CTA takes one (y, c, group); thread (x, j) builds the z line of slot GW/2 g + j at
-// (y, x) from the packed expansion entries and G0P[g][orbit][j] (the GW / 2 lanes of
-// one x read one orbit's line), transforms it in registers and stores it to
-// W[slot][c][z][y][x].  Launched with GW / 2 * H threads.
-template <typename T, int H>
-__global__ void __launch_bounds__(wide_fields<typename Cx<T>::type>() / 2 * H)
-k_expand_w_ifft_z_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
-                    const uint32_t* __restrict__ ETP, const typename Cx<T>::type* __restrict__ G0P,
-                    typename Cx<T>::type* __restrict__ W, int nfields) {
-  pdl_enter();
-  using C = typename Cx<T>::type;
-  constexpr int GW = wide_fields<C>(), L = GW / 2, HV = H * H * H;
-  const int y = blockIdx.x, c = blockIdx.y, gq = blockIdx.z;
-  const int j = threadIdx.x % L, x = threadIdx.x / L;
-  const int slot = gq * L + j;
-  if (2 * slot >= nfields) return;
-  const uint32_t* et = ETP + static_cast<size_t>(c) * HV + y * H + x;
-  const C* rp = G0P + static_cast<size_t>(gq) * g->n_orbits * L + j;
-  const C* ph = tables + g->ph_off;
-  C v[H];
-#pragma unroll
-  for (int z = 0; z < H; ++z) {
-    const uint32_t t = __ldg(et + z * H * H);
-    v[z] = cmulc(__ldg(rp + static_cast<size_t>(L) * (t & 0x1FFFFFu)), ph[t >> 21]);
   }
   reg_fft<C, true, H>(v);
   C* dst = W + (static_cast<size_t>(slot) * g->n_ch + c) * HV + y * H + x;
@@ -1459,6 +1875,7 @@ __global__ void k_qsep_ifft_z_h(const DevGeom* __restrict__ g, const typename Cx
 }
 
 constexpr int kMaxDynSmemFast = 227 * 1024;
+constexpr int kSMs = 148;  // B200: the unit of the launch-size rules
 
 // Programmatic dependent launch of the fast-path kernels (off with CFFT_PDL=0): each
 // kernel of a lane may launch while its predecessor in the stream is finishing, and
@@ -1693,7 +2110,9 @@ Status fast_unit_init(std::string* err) {
         for (int ct = 0; ct < 5; ++ct) {
           CFFT_FOR_CT(ct, {
             cudaFuncSetAttribute(k_plane_fwd_h<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
-            cudaFuncSetAttribute(k_plane_bwd_h<T, HH, CTT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
+            cudaFuncSetAttribute(k_plane_bwd_h<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
+            cudaFuncSetAttribute(k_plane_fwd_s<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
+            cudaFuncSetAttribute(k_plane_bwd_s<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
             // The bulk-copy kernels also hold a little static shared memory, so their
             // dynamic limit is their exact need; a refusal is reported.
             cudaError_t te = cudaSuccess;
@@ -1728,12 +2147,16 @@ Status fast_unit_init(std::string* err) {
         // share above 48 KB (FP64, 4 slots) needs the attribute, so failures are reported.
         {
           constexpr int kZr = kMaxDynSmemFast - 1024;
-          cudaError_t ze = cudaFuncSetAttribute(k_fft_z_recon_diag8<T, HH, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kZr);
-          if (ze == cudaSuccess) ze = cudaFuncSetAttribute(k_fft_z_recon_diag8<T, HH, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kZr);
-          if (ze == cudaSuccess) ze = cudaFuncSetAttribute(k_fft_z_recon_diag8<T, HH, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kZr);
-          if (ze == cudaSuccess) ze = cudaFuncSetAttribute(k_fft_z_recon_diag8<T, HH, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kZr);
+          constexpr bool SP = zr_split<T, HH>();
+          cudaError_t ze = cudaFuncSetAttribute(k_fft_z_recon_diag8<T, HH, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kZr);
+          if (ze == cudaSuccess) ze = cudaFuncSetAttribute(k_fft_z_recon_diag8<T, HH, 2, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kZr);
+          if (ze == cudaSuccess) ze = cudaFuncSetAttribute(k_fft_z_recon_diag8<T, HH, 4, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kZr);
           if (ze != cudaSuccess) return fast_cuda(ze, "fused z FFT + gather shared-memory attribute", err);
         }
+        using CC = typename Cx<T>::type;
+        cudaFuncSetAttribute(k_expand_ifft_z<T, HH, wide_slots<CC>(), expand_slots<CC, HH, wide_slots<CC>()>(), sizeof(T) == 8>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
+        cudaFuncSetAttribute(k_expand_ifft_z<T, HH, 2, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
         cudaFuncSetAttribute(k_expand_ifft_z_h<T, HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
       }
     });
@@ -1817,9 +2240,15 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
       if (ce != cudaSuccess) return fast_cuda(ce, "fused cluster launch", err);
       return fast_cuda(cudaGetLastError(), "fused cluster launch", err);
     }
-    const int thr_plane = std::max(128, ((nch * H + 31) / 32) * 32);
+    const int thr_plane = plane_line_threads<T>(H, nch, a.cent_type != 0);
     const size_t smem_plane = static_cast<size_t>(nch) * H * (H + 1) * cs;
     const int ntasks = nslots * H;
+    // Split lines while the launch has at most one CTA per SM: then the length of a thread's
+    // chain counts, beyond that the extra shared-memory passes do.  Ia-3d 96^3 FP32, three
+    // contour steps of 2 / 32 fields: 69 / 140 us against 84 / 140 with a line per thread; of
+    // Im-3m 128^3, 32 fields (256 CTAs): 58.9 against 56.5.  Above H = 32 the plane takes a
+    // whole SM either way and the split loses at every size.
+    const bool split = ntasks <= kSMs && H <= 32;
     auto al16 = [](const void* p) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     const int tmode = a.tma >= 0 ? a.tma : tma_mode();
     const bool tma = al16(f0) && al16(E) && al16(f0_out) && al16(W) && (tmode & (a.stage == 0 ? 1 : 2));
@@ -1848,7 +2277,9 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
               done = true;
             }
           }
-          if (!done)
+          if (!done && split)
+            launch_k(k_plane_fwd_s<T, HH, CTT>, dim3(H, nslots), split_threads<HH, CTT>(), smem_plane + HH * cs, st, g, tab, f0, E, W, nb);
+          else if (!done)
             launch_k(k_plane_fwd_h<T, HH, CTT>, dim3(H, nslots), thr_plane, smem_plane, st, g, tab, f0, E, W, nb);
         });
       });
@@ -1867,8 +2298,10 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
               done = true;
             }
           }
-          if (!done)
-            launch_k(k_plane_bwd_h<T, HH, CTT, true>, dim3(H, nslots), thr_plane, smem_plane, st, g, tab, W, E, f0_out, nb);
+          if (!done && split)
+            launch_k(k_plane_bwd_s<T, HH, CTT>, dim3(H, nslots), split_threads<HH, CTT>(), smem_plane + HH * cs, st, g, tab, W, E, f0_out, nb);
+          else if (!done)
+            launch_k(k_plane_bwd_h<T, HH, CTT>, dim3(H, nslots), thr_plane, smem_plane, st, g, tab, W, E, f0_out, nb);
         });
       });
     }
@@ -1914,56 +2347,50 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
         break;
       }
       case 6: {
-        // fused z FFT + diagonal-sign gather, ZR_SLOTS workspace slots per CTA
-        const int sl = a.zr_slots == 2 || a.zr_slots == 4 ? a.zr_slots : zr_slots();
-        const T* K = static_cast<const T*>(a.K);
-        const uint32_t* sh = static_cast<const uint32_t*>(a.spec_h);
+        // Fused z FFT + diagonal-sign gather.  One slot per CTA (split lines) while that
+        // gives at most two CTAs per SM; else 4 slots per CTA in FP32 (2 on request).  FP64 and
+        // H = 48 split their lines: 2 slots where the units hold many points, whose weights the
+        // slots share (Pmmm 64^3 FP64, 256 fields, round trip: 211 / 212 / 218 us with 2 / 1 / 4), 1
+        // else (Im-3m 96^3 FP64, 64 fields: 64.3 / 66.9 / 67.5 with 1 / 2 / 4).
+        const T* K = a.use_K ? static_cast<const T*>(a.K) : nullptr;
         const uint4* un = static_cast<const uint4*>(a.zr_units);
-        const uint32_t* pt = static_cast<const uint32_t*>(a.zr_pts);
+        const uint2* pt = static_cast<const uint2*>(a.zr_pts);
+        const C* pq = static_cast<const C*>(a.zr_pq);
         const C* Wc = W;
         CFFT_FOR_H(H, {
-          const size_t sm = static_cast<size_t>(sl) * 2 * HH * (HH + 1) * cs;
+          constexpr bool SP = zr_split<T, HH>();
+          const int sl = a.zr_slots == 2 || a.zr_slots == 4 ? a.zr_slots
+                         : a.zr_n_units * nslots <= 2 * kSMs ? 1 : SP ? (a.n_spec_pts > 512 * a.zr_n_units ? 2 : 1) : zr_slots();
+          const size_t sm = (static_cast<size_t>(sl) * 2 * HH * (HH + 1) + HH) * cs;
           const dim3 gzr(a.zr_n_units, (nslots + sl - 1) / sl);
-          if (sl == 4) {
-            if (a.use_K) launch_k(k_fft_z_recon_diag8<T, HH, 4, true>, gzr, zr_threads<HH>(4), sm, st, g, tab, sh, K, un, pt, Wc, F, nb);
-            else launch_k(k_fft_z_recon_diag8<T, HH, 4, false>, gzr, zr_threads<HH>(4), sm, st, g, tab, sh, nullptr, un, pt, Wc, F, nb);
-          } else {
-            if (a.use_K) launch_k(k_fft_z_recon_diag8<T, HH, 2, true>, gzr, zr_threads<HH>(2), sm, st, g, tab, sh, K, un, pt, Wc, F, nb);
-            else launch_k(k_fft_z_recon_diag8<T, HH, 2, false>, gzr, zr_threads<HH>(2), sm, st, g, tab, sh, nullptr, un, pt, Wc, F, nb);
-          }
+          if (sl == 1)
+            launch_k(k_fft_z_recon_diag8<T, HH, 1, true>, gzr, zr_threads<HH, 1, true>(), sm, st, g, tab, K, un, pt, pq, a.n_spec_pts, Wc, F, nb);
+          else if (sl == 4)
+            launch_k(k_fft_z_recon_diag8<T, HH, 4, SP>, gzr, zr_threads<HH, 4, SP>(), sm, st, g, tab, K, un, pt, pq, a.n_spec_pts, Wc, F, nb);
+          else
+            launch_k(k_fft_z_recon_diag8<T, HH, 2, SP>, gzr, zr_threads<HH, 2, SP>(), sm, st, g, tab, K, un, pt, pq, a.n_spec_pts, Wc, F, nb);
         });
         break;
       }
       case 3: {
         const int no = a.n_orbits;
-        if (a.reps_wide) {
-          constexpr int GW = wide_fields<C>();
-          const int ng = (nb + GW - 1) / GW;
-          C* FT = static_cast<C*>(a.FT);
-          launch_k(k_group_spectra_w<T>, dim3((a.n_spec + kWideTile - 1) / kWideTile, ng), 256, 0, st, Fin, FT,
-                   a.n_spec, nb);
-          const dim3 gw((GW / 2 * no + 255) / 256, ng);
-          const uint32_t* pk = static_cast<const uint32_t*>(a.inv_pk);
-          switch (a.d) {
-            case 1: launch_k(k_inv_recon_w<T, 1>, gw, 256, 0, st, g, tab, pk, FT, G0R); break;
-            case 2: launch_k(k_inv_recon_w<T, 2>, gw, 256, 0, st, g, tab, pk, FT, G0R); break;
-            case 4: launch_k(k_inv_recon_w<T, 4>, gw, 256, 0, st, g, tab, pk, FT, G0R); break;
-            default: launch_k(k_inv_recon_w<T, 8>, gw, 256, 0, st, g, tab, pk, FT, G0R); break;
-          }
-          break;
-        }
         if (a.reps_quad) {
-          const int nq = (nb + 3) / 4;
-          C* FT = static_cast<C*>(a.FT);
-          launch_k(k_group_spectra<T>, dim3((a.n_spec + 511) / 512, nq), 256, 0, st, Fin, FT, a.n_spec, nb);
-          const dim3 gq((2 * no + 255) / 256, nq);
-          const uint32_t* pk = static_cast<const uint32_t*>(a.inv_pk);
-          switch (a.d) {
-            case 1: launch_k(k_inv_recon_quad<T, 1>, gq, 256, 0, st, g, tab, pk, FT, G0R); break;
-            case 2: launch_k(k_inv_recon_quad<T, 2>, gq, 256, 0, st, g, tab, pk, FT, G0R); break;
-            case 4: launch_k(k_inv_recon_quad<T, 4>, gq, 256, 0, st, g, tab, pk, FT, G0R); break;
-            default: launch_k(k_inv_recon_quad<T, 8>, gq, 256, 0, st, g, tab, pk, FT, G0R); break;
-          }
+          const uint2* tp = static_cast<const uint2*>(a.fib_taps);
+          const uint2* fo = static_cast<const uint2*>(a.fib_outs);
+          const int fb = (a.n_fib + kFibers - 1) / kFibers;
+#define CFFT_INV_FIBER(LL)                                                                                          \
+  {                                                                                                                 \
+    const dim3 gf(fb, (nslots + (LL) - 1) / (LL));                                                                  \
+    switch (a.d) {                                                                                                  \
+      case 1: launch_k(k_inv_fiber<T, 1, LL>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
+      case 2: launch_k(k_inv_fiber<T, 2, LL>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
+      case 4: launch_k(k_inv_fiber<T, 4, LL>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
+      default: launch_k(k_inv_fiber<T, 8, LL>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
+    }                                                                                                               \
+  }
+          if (a.reps_wide) CFFT_INV_FIBER(wide_slots<C>())
+          else CFFT_INV_FIBER(2)
+#undef CFFT_INV_FIBER
           break;
         }
         launch_k(k_inv_recon_reps<T>, dim3((no + 127) / 128, (nslots + kRepSlots - 1) / kRepSlots), 128, 0, st, 
@@ -1987,15 +2414,20 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
           break;
         }
         CFFT_FOR_H(H, {
+          const uint32_t* et = static_cast<const uint32_t*>(a.expand);
+          // Rows of two slots: split lines through shared memory for launches of at most one CTA
+          // per SM (Im-3m 128^3 FP32, one field, round trip 19.6 against 21.6 us; 8 fields 32.1
+          // against 29.8), never above H = 32 (192^3, one field: 44.0 against 30.8).
           if (a.reps_wide) {
-            constexpr int GW = wide_fields<C>();
-            launch_k(k_expand_w_ifft_z_h<T, HH>, dim3(HH, nch, (nb + GW - 1) / GW), GW / 2 * HH, 0, st, g, tab,
-                     static_cast<const uint32_t*>(a.expand), G0R, W, nb);
-          } else if (a.reps_quad) {
-            // two y values per CTA (128 threads at H = 32): 5 CTAs per SM at this kernel's registers
+            constexpr int L = wide_slots<C>(), LS = expand_slots<C, HH, L>();
+            launch_k(k_expand_ifft_z<T, HH, L, LS, sizeof(T) == 8>, dim3(HH, nch, (nslots + L - 1) / L * (L / LS)),
+                     expand_threads<C, HH, LS>(), (expand_plane<HH>() * LS + HH) * sizeof(C), st, g, tab, et, G0R, W, nb);
+          } else if (a.reps_quad && (HH > 32 || HH * nch * ((nslots + 1) / 2) > kSMs)) {
             constexpr int half = ((2 * HH + 31) / 32) * 32;
-            launch_k(k_expand4_ifft_z_h<T, HH, 2>, dim3((HH + 1) / 2, nch, (nb + 3) / 4), 2 * half, 0, st, 
-                g, tab, static_cast<const uint32_t*>(a.expand), G0R, W, nb);
+            launch_k(k_expand2_ifft_z<T, HH, 2>, dim3((HH + 1) / 2, nch, (nslots + 1) / 2), 2 * half, 0, st, g, tab, et, G0R, W, nb);
+          } else if (a.reps_quad) {
+            launch_k(k_expand_ifft_z<T, HH, 2, 2, true>, dim3(HH, nch, (nslots + 1) / 2), expand_threads<C, HH, 2>(),
+                     (expand_plane<HH>() * 2 + HH) * sizeof(C), st, g, tab, et, G0R, W, nb);
           } else
             launch_k(k_expand_ifft_z_h<T, HH>, gz, thr_z, smem_z, st, g, tab, static_cast<const int2*>(a.expand), G0R, W);
         });

@@ -1,0 +1,59 @@
+"""The compile-time sized kernels at the edges of their dispatch: small launches (split
+lines, rows of two slots), full rows of representatives with a remainder, every channel
+edge, all centrings, and groups with screw axes, glides and no inversion centre, where the
+fibers of the inverse gather carry phases and conjugated taps.  Each field is a seeded
+combination of two symmetric oracle fields, so its spectrum is the same combination of two
+FP64 full-grid FFTs (test/runtests.jl:199-216, test/test_centered_backward.jl:31-70).
+
+Tolerances: the worst-case growth of a radix-r FFT pass is a few roundings, so a transform of
+n points is within about 4 log2(n) eps of the largest value; 4 x 17 x 1.2e-7 = 8e-6 for FP32
+at 48^3 points and 1.5e-14 for FP64, and the round trip doubles that.  The bars are 1e-5 and
+2e-13, and twice that for the round trip."""
+import numpy as np
+import pytest
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("no CUDA device", allow_module_level=True)
+
+TOL = {4: 1e-5, 8: 2e-13}
+
+
+def check(cf, O, prep, sg, N, precision, batch):
+    ps = [prep(sg, N, seed=s) for s in (31, 32)]
+    plan = cf.KRFFTPlan(ps[0]["spec"], ps[0]["ops_s"], precision=precision, max_batch=batch)
+    ospec = O.calc_spectral_asu(ps[0]["oops"], len(N), N)
+    bases = np.stack([O.pack_stride(p["u"], plan.L) for p in ps])
+    truths = np.stack([O.spectrum_on_asu(p["u"], ospec) for p in ps])
+    coef = np.random.default_rng(batch).standard_normal((batch, 2))
+    f0 = np.tensordot(coef, bases, 1)
+    order = (0,) + tuple(range(len(N), 0, -1))
+    x = torch.tensor(np.ascontiguousarray(f0.transpose(order)), device="cuda",
+                     dtype=torch.float32 if precision == 4 else torch.float64)
+    F = plan.forward(x)
+    back = plan.backward(F).cpu().numpy().reshape(x.shape)
+    F = F.cpu().numpy().reshape(batch, -1)
+    for b in range(batch):
+        assert rel_err(F[b], coef[b] @ truths) < TOL[precision], b
+        assert rel_err(back[b], f0[b].T) < 2 * TOL[precision], b
+    plan.close()
+
+
+@pytest.mark.parametrize("precision", [4, 8])
+@pytest.mark.parametrize("sg,n,batch", [(229, 16, 1), (229, 24, 3), (229, 32, 33), (230, 48, 2), (229, 48, 17), (227, 64, 9),
+                                        (230, 64, 36), (225, 96, 5), (229, 96, 1), (47, 32, 70), (221, 48, 19)])
+def test_channel_edges(cf, O, prep, sg, n, batch, precision):
+    check(cf, O, prep, sg, (n, n, n), precision, batch)
+
+
+@pytest.mark.parametrize("sg", [2, 16, 19, 23, 24, 62, 92, 96, 122, 141, 198, 199, 205, 212, 214, 220, 228])
+def test_fiber_phases(cf, O, prep, sg):
+    check(cf, O, prep, sg, (16, 16, 16), 8, 11)
+
+
+def test_largest_edge(cf, O, prep):
+    check(cf, O, prep, 221, (96, 96, 96), 4, 3)  # plain lattice, 48 points per line
