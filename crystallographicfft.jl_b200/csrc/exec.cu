@@ -691,11 +691,12 @@ Status launch_stage(Plan* p, int stage, const T* f0, typename Cx<T>::type* F, co
       a.q_step = true;
       a.QT = p->d_qt;
       a.GT = p->d_gt;
-      a.qsep = p->qsep;
       a.QS = p->d_qsep;
-      C* WQ = reinterpret_cast<C*>(static_cast<char*>(p->d_work_Q) + lane * p->w_lane_bytes);
-      if (stage == 4) a.W2 = WQ;
-      else if (stage == 5) a.W = WQ;
+      if (!p->qsep) {
+        C* WQ = reinterpret_cast<C*>(static_cast<char*>(p->d_work_Q) + lane * p->w_lane_bytes);
+        if (stage == 4) a.W2 = WQ;
+        else if (stage == 5) a.W = WQ;
+      }
     }
     a.stream = st;
     const bool planes = stage == 0 || stage == 5;
@@ -769,8 +770,11 @@ Status run_chunks(Plan* p, bool fwd, bool bwd, const T* f0, typename Cx<T>::type
     auto* Fc = F + b0 * ns;
     if (fwd && bwd && use_K && p->qmode) {
       // Q-matrix diffusion step: forward transform to G0, Q-multiply + inverse z FFT,
-      // inverse x/y FFT + unfold (no spectral-ASU round trip).
+      // inverse x/y FFT + unfold (no spectral-ASU round trip); separable plans do both z
+      // transforms and the multiply in one stage.
       for (int s : {0, 1, 4, 5}) {
+        if (p->qsep && s == 1) continue;
+        if (p->qsep && s == 4) s = 7;
         Status r = launch_stage<T>(p, s, fin, Fc, Fc, fout, Ec, false, nb, ls, err, lane, true);
         if (r != Status::kOk) return r;
       }
@@ -1207,7 +1211,6 @@ Status plan_device_init(Plan* p, std::string* err) {
       return Status::kUnsupported;
     }
     const size_t np = static_cast<size_t>(T.n_ch) * hvol;
-    if ((st = alloc(&p->d_work_Q, p->lanes * p->w_lane_bytes, "Q workspace")) != Status::kOk) return st;
     // Separable Q-multiply (_is_pmmm_like, src/q_fused_krfft.jl:431-454): M2Q plan, d = 8,
     // L = (2, 2, 2), diagonal representatives listed in parity-class order with
     // translations 0 or N - 1, and an orthogonal cell (K factorises per axis).
@@ -1231,6 +1234,7 @@ Status plan_device_init(Plan* p, std::string* err) {
     if (p->qsep) {
       if ((st = alloc(&p->d_qsep, static_cast<size_t>(9) * T.M[0] * cs, "separable Q factors")) != Status::kOk) return st;
     } else {
+      if ((st = alloc(&p->d_work_Q, p->lanes * p->w_lane_bytes, "Q workspace")) != Status::kOk) return st;
       if ((st = alloc(&p->d_qt, T.d * np * cs, "Q coefficients")) != Status::kOk) return st;
       if ((st = alloc(&p->d_gt, T.d * np * 4, "Q gather")) != Status::kOk) return st;
     }

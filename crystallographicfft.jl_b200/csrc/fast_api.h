@@ -42,13 +42,13 @@ struct FastArgs {
   int zr_n_units = 0;
   bool cluster = false;   // fused cluster kernels for stages 0 (with 1) and 5 (with 4)
   int cluster_ctas = 8;   // CTAs per cluster (8, or 16 where the device allows it)
-  // Q-matrix step: stage 4 reads W (forward G0, z-fastest) and writes W2
+  // Q-matrix step: stage 4 reads W (forward G0, z-fastest) and writes W2; a separable plan
+  // runs stage 7 in place on W instead of stages 1 and 4
   bool q_step = false;
   const void* QT = nullptr;   // d x n_ch x H^3 coefficients
   const void* GT = nullptr;   // d x n_ch x H^3 int32 workspace indices (-1: extinct)
   void* W2 = nullptr;
-  bool qsep = false;          // separable Q-multiply (Pmmm-like plans)
-  const void* QS = nullptr;   // its 1-D twiddles and kernel factors
+  const void* QS = nullptr;   // 1-D twiddles and kernel factors of the separable Q-multiply
   void* stream = nullptr;
   // bounded device waits of the persistent bulk-copy kernels: limit, and the plan's
   // status word that a wait which runs out sets to CFFT_ERR_TIMEOUT

@@ -1657,6 +1657,56 @@ template <typename C, int H, int LS> constexpr int expand_threads() {
   constexpr int t = items / 4 > LS * H ? items / 4 : LS * H;
   return t <= 64 ? 64 : t >= 256 ? 256 : ((t + 31) / 32) * 32;
 }
+// Inverse z FFT of LS planes [slot][z][x] (expand_plane apart) in shared memory, stored for
+// the first `live` slots to dst + slot * sstride + z * H * H + x.
+template <typename C, int H, int LS, bool SPLIT>
+__device__ __forceinline__ void inverse_z_planes(C* buf, const C* tw, C* __restrict__ dst, size_t sstride, int live) {
+  constexpr int PS = expand_plane<H>();
+  const int tid = threadIdx.x, nth = blockDim.x;
+  if constexpr (!SPLIT) {
+    for (int i = tid; i < LS * H; i += nth) {
+      const int x = i % H, j = i / H;
+      const C* p = buf + j * PS + x;
+      C v[H];
+#pragma unroll
+      for (int z = 0; z < H; ++z) v[z] = p[z * H];
+      reg_fft<C, true, H>(v);
+      if (j < live) {
+        C* d = dst + j * sstride + x;
+#pragma unroll
+        for (int z = 0; z < H; ++z) d[z * H * H] = v[z];
+      }
+    }
+  } else {
+    constexpr int A = split_a<H>(), B = split_b<H>(), R = B > 1 ? B : A, NB = H / R;
+    if constexpr (B > 1) {
+      for (int i = tid; i < LS * H * B; i += nth) {
+        const int x = i % H, j = (i / H) % LS, jj = i / (H * LS);
+        C* p = buf + j * PS + jj * H + x;
+        C v[A];
+#pragma unroll
+        for (int r = 0; r < A; ++r) v[r] = p[r * B * H];
+        split_pass1<C, true, H>(v, jj, tw);
+#pragma unroll
+        for (int r = 0; r < A; ++r) p[r * B * H] = v[r];
+      }
+      __syncthreads();
+    }
+    for (int i = tid; i < LS * H * NB; i += nth) {
+      const int x = i % H, j = (i / H) % LS, k1 = i / (H * LS);
+      if (j >= live) continue;
+      const C* p = buf + j * PS + k1 * R * H + x;
+      C v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = p[r * H];
+      reg_fft<C, true, R>(v);
+      C* d = dst + j * sstride + static_cast<size_t>(k1) * H * H + x;
+#pragma unroll
+      for (int r = 0; r < R; ++r) d[static_cast<size_t>(r) * NB * H * H] = v[r];
+    }
+  }
+}
+
 template <typename T, int H, int L, int LS, bool SPLIT>
 __global__ void __launch_bounds__(expand_threads<typename Cx<T>::type, H, LS>())
 k_expand_ifft_z(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
@@ -1692,51 +1742,9 @@ k_expand_ifft_z(const DevGeom* __restrict__ g, const typename Cx<T>::type* __res
     }
   }
   __syncthreads();
-  C* dst = W + (static_cast<size_t>(slot0) * g->n_ch + c) * HV + y * H;
-  const size_t sstride = static_cast<size_t>(g->n_ch) * HV;
   const int live = min(LS, (nfields + 1) / 2 - slot0);
-  if constexpr (!SPLIT) {
-    for (int i = threadIdx.x; i < LS * H; i += NTH) {
-      const int x = i % H, j = i / H;
-      const C* p = buf + j * PS + x;
-      C v[H];
-#pragma unroll
-      for (int z = 0; z < H; ++z) v[z] = p[z * H];
-      reg_fft<C, true, H>(v);
-      if (j < live) {
-        C* d = dst + j * sstride + x;
-#pragma unroll
-        for (int z = 0; z < H; ++z) d[z * H * H] = v[z];
-      }
-    }
-  } else {
-    constexpr int A = split_a<H>(), B = split_b<H>(), R = B > 1 ? B : A, NB = H / R;
-    if constexpr (B > 1) {
-      for (int i = threadIdx.x; i < LS * H * B; i += NTH) {
-        const int x = i % H, j = (i / H) % LS, jj = i / (H * LS);
-        C* p = buf + j * PS + jj * H + x;
-        C v[A];
-#pragma unroll
-        for (int r = 0; r < A; ++r) v[r] = p[r * B * H];
-        split_pass1<C, true, H>(v, jj, tw);
-#pragma unroll
-        for (int r = 0; r < A; ++r) p[r * B * H] = v[r];
-      }
-      __syncthreads();
-    }
-    for (int i = threadIdx.x; i < LS * H * NB; i += NTH) {
-      const int x = i % H, j = (i / H) % LS, k1 = i / (H * LS);
-      if (j >= live) continue;
-      const C* p = buf + j * PS + k1 * R * H + x;
-      C v[R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = p[r * H];
-      reg_fft<C, true, R>(v);
-      C* d = dst + j * sstride + static_cast<size_t>(k1) * H * H + x;
-#pragma unroll
-      for (int r = 0; r < R; ++r) d[static_cast<size_t>(r) * NB * H * H] = v[r];
-    }
-  }
+  inverse_z_planes<C, H, LS, SPLIT>(buf, tw, W + (static_cast<size_t>(slot0) * g->n_ch + c) * HV + y * H,
+                                    static_cast<size_t>(g->n_ch) * HV, live);
 }
 
 // The same for rows of two slots (small batches), one z line per thread straight from the
@@ -1772,27 +1780,29 @@ __global__ void k_expand2_ifft_z(const DevGeom* __restrict__ g, const typename C
 // 870-895): for every channel point (c, x, y, z) of a slot, q its subgrid position,
 //   Y'(q) = sum_b Q_b(q) G0(R_b^T q mod M)
 // with G0 gathered from the forward workspace WT (z-fastest; index -1 marks a parity
-// class without a channel, where G0 = 0), assembled as the z line of (c, y, x), inverse z
-// FFT in registers, stored W2[slot][c][z][y][x] for the inverse plane kernel.  Both
-// fields of the slot (G0_a + i G0_b) go through the same complex-linear map.
+// class without a channel, where G0 = 0), then the inverse z FFT, stored
+// W2[slot][c][z][y][x] for the inverse plane kernel.  Both fields of the slot
+// (G0_a + i G0_b) go through the same complex-linear map.  A CTA takes one (y, c, slot), a
+// thread one point at a time: the d gathers of a point are independent, but a thread that
+// gathers a whole line makes H of them wait for one another.
 template <typename T, int H>
-__global__ void k_qmul_ifft_z_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ QT,
-                                const int32_t* __restrict__ GT, const typename Cx<T>::type* __restrict__ WT,
-                                typename Cx<T>::type* __restrict__ W2) {
+__global__ void __launch_bounds__(expand_threads<typename Cx<T>::type, H, 2>())
+k_qmul_ifft_z_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+                const typename Cx<T>::type* __restrict__ QT, const int32_t* __restrict__ GT,
+                const typename Cx<T>::type* __restrict__ WT, typename Cx<T>::type* __restrict__ W2) {
   pdl_enter();
   using C = typename Cx<T>::type;
   constexpr int HV = H * H * H;
-  const int y0 = blockIdx.x * kZB, c = blockIdx.y, slot = blockIdx.z;
-  const int ny = min(kZB, H - y0);
-  const int yy = threadIdx.x / H, x = threadIdx.x % H;
-  if (yy >= ny) return;
-  const int y = y0 + yy;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* buf = reinterpret_cast<C*>(smem_raw);  // [z][x]
+  C* tw = buf + expand_plane<H>();
+  load_line_twiddles<C, H>(g, tables, tw);
+  const int y = blockIdx.x, c = blockIdx.y, slot = blockIdx.z;
   const int d = g->d;
   const size_t np = static_cast<size_t>(g->n_ch) * HV;
   const C* wt = WT + static_cast<size_t>(slot) * g->n_ch * HV;
-  C v[H];
-#pragma unroll
-  for (int z = 0; z < H; ++z) {
+  for (int i = threadIdx.x; i < H * H; i += blockDim.x) {
+    const int x = i % H, z = i / H;
     const size_t pos = static_cast<size_t>(c) * HV + (z * H + y) * H + x;
     C acc = mk<C>(static_cast<T>(0), static_cast<T>(0));
 #pragma unroll
@@ -1802,12 +1812,10 @@ __global__ void k_qmul_ifft_z_h(const DevGeom* __restrict__ g, const typename Cx
         if (gi >= 0) acc = cadd(acc, cmul(__ldg(QT + b * np + pos), __ldg(wt + gi)));
       }
     }
-    v[z] = acc;
+    buf[z * H + x] = acc;
   }
-  reg_fft<C, true, H>(v);
-  C* dst = W2 + (static_cast<size_t>(slot) * g->n_ch + c) * HV + y * H + x;
-#pragma unroll
-  for (int z = 0; z < H; ++z) dst[z * H * H] = v[z];
+  __syncthreads();
+  inverse_z_planes<C, H, 1, true>(buf, tw, W2 + (static_cast<size_t>(slot) * g->n_ch + c) * HV + y * H, 0, 1);
 }
 
 // Separable Q-multiply of the M2Q step for Pmmm-like plans (_q_multiply_separable!,
@@ -1815,63 +1823,144 @@ __global__ void k_qmul_ifft_z_h(const DevGeom* __restrict__ g, const typename Cx
 // the representatives diag(s) with translations 0 or -1, and an orthogonal cell.  Then
 // B = WHT8 diag(tw^alpha) and the first row of Q = B^-1 diag(K) B gives
 //   Y'(q) = (1/8) sum_m K(q + M alpha_m) [WHT8 (tw^alpha_a(q) Y(s_a q mod M))]_m,
-// tw_d(q) = e^{2 pi i q_d / N_d}, K(h) = prod_d exp(-ds (2 pi h_c,d / a_d)^2).  Nothing is
-// tabulated per point: QS holds the 1-D twiddles (3 x H complex) and the 1-D kernel
-// factors (3 x 2H, real parts).  Same line structure as k_qmul_ifft_z_h (plain path,
-// one channel, H = M): the z line of (y, x) is assembled, inverse z FFT, stored to W2.
+// tw_d(q) = e^{2 pi i q_d / N_d}, K(h) = prod_d exp(-ds (2 pi h_c,d / a_d)^2).  The eight
+// images s_a q form a closed set on which the spectrum only changes by the twiddle, so
+//   Y'(s_a q) = conj(tw^alpha_a(q)) / 8 [WHT8 (K WHT8 (tw^alpha Y))]_a
+// maps the eight values in place: one pair of transforms per eight points instead of
+// one gather of eight per point.  The images lie on the channel rows y and -y and the
+// lines x and -x, so a CTA that holds those lines does the whole middle of the step: forward
+// z FFT, the map, inverse z FFT, in place on the workspace W[slot][z][y][x] (plain path, one
+// channel, H = M).  Blocks: rows y <= H / 2, PP pairs of lines (x, -x), slots; fewer pairs
+// per block while the launch would not fill the SMs.  The lines stay in line_pos order
+// between the transforms, whose passes run in reverse on the way back.  Pm-3m 48^3 FP64,
+// 4 fields: 5 us z FFT + 20 us gather (and its second workspace) before.
+// QS holds the 1-D twiddles (3 x H complex) and the 1-D kernel factors (3 x 2H, real parts).
+constexpr int kSepThreads = 128;
 template <typename T, int H>
-__global__ void k_qsep_ifft_z_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ QS,
-                                const typename Cx<T>::type* __restrict__ WT, typename Cx<T>::type* __restrict__ W2) {
+__global__ void __launch_bounds__(kSepThreads)
+k_qsep_z(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+         const typename Cx<T>::type* __restrict__ QS, typename Cx<T>::type* __restrict__ W, int PP) {
   pdl_enter();
   using C = typename Cx<T>::type;
-  constexpr int HV = H * H * H;
-  const int y0 = blockIdx.x * kZB, slot = blockIdx.z;
-  const int ny = min(kZB, H - y0);
-  const int yy = threadIdx.x / H, x = threadIdx.x % H;
-  if (yy >= ny) return;
-  const int y = y0 + yy;
-  const C* wt = WT + static_cast<size_t>(slot) * HV;
-  const C* tw = QS;              // tw[d * H + q]
-  const C* kf = QS + 3 * H;      // kf[d * 2H + h].x
-  int neg[8];                    // bit d: axis d negated by representative a
+  constexpr int HV = H * H * H, S = H + 1, A = split_a<H>(), B = split_b<H>(), HP = H / 2 + 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* buf = reinterpret_cast<C*>(smem_raw);  // [row][side][pair][z]
+  C* tw = buf + 4 * PP * S;
+  load_line_twiddles<C, H>(g, tables, tw);
+  const int y = blockIdx.x, ym = y ? H - y : 0, rows = ym == y ? 1 : 2;
+  const int p0 = blockIdx.y * PP, np = min(PP, HP - p0), slot = blockIdx.z;
+  const int lines = rows * 2 * np;
+  C* Ws = W + static_cast<size_t>(slot) * HV;
+  // line l: row r, side (x or -x), pair p; -1 where the line is its own mirror image
+  auto line = [&](int l, int* off) {
+    const int r = l / (2 * np), m = l - r * 2 * np, side = m / np, k = m - side * np, p = p0 + k;
+    if (side && (p == 0 || 2 * p == H)) return -1;
+    *off = (r ? ym : y) * H + (side ? H - p : p);
+    return ((r * 2 + side) * PP + k) * S;
+  };
+  if constexpr (B > 1) __syncthreads();
+  for (int i = threadIdx.x; i < lines * B; i += kSepThreads) {
+    const int j = i / lines;
+    int off = 0;
+    const int at = line(i - j * lines, &off);
+    if (at < 0) continue;
+    const C* src = Ws + off + j * H * H;
+    C v[A];
 #pragma unroll
-  for (int a = 0; a < 8; ++a)
-    neg[a] = (g->rep_R[a][0] < 0 ? 1 : 0) | (g->rep_R[a][4] < 0 ? 2 : 0) | (g->rep_R[a][8] < 0 ? 4 : 0);
-  const int xm = x ? H - x : 0, ym = y ? H - y : 0;
-  const C twx = tw[x], twy = tw[H + y];
-  const T kx0 = kf[x].x, kx1 = kf[x + H].x, ky0 = kf[2 * H + y].x, ky1 = kf[2 * H + y + H].x;
-  const C txy = cmul(twx, twy);
-  C v[H];
+    for (int r = 0; r < A; ++r) v[r] = src[r * B * H * H];
+    split_pass1<C, false, H>(v, j, tw);
+    C* row = buf + at + j;
 #pragma unroll
-  for (int z = 0; z < H; ++z) {
-    const int zm = z ? H - z : 0;
-    const C twz = tw[2 * H + z];
-    C p[8];
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      const int gx = (neg[a] & 1) ? xm : x, gy = (neg[a] & 2) ? ym : y, gz = (neg[a] & 4) ? zm : z;
-      p[a] = wt[(gx * H + gy) * H + gz];
-    }
-    p[1] = cmul(p[1], twx);
-    p[2] = cmul(p[2], twy);
-    p[3] = cmul(p[3], txy);
-    p[4] = cmul(p[4], twz);
-    p[5] = cmul(p[5], cmul(twx, twz));
-    p[6] = cmul(p[6], cmul(twy, twz));
-    p[7] = cmul(p[7], cmul(txy, twz));
-    wht8c(p);
-    const T kz0 = kf[4 * H + z].x, kz1 = kf[4 * H + z + H].x;
-    const T k00 = kx0 * ky0, k10 = kx1 * ky0, k01 = kx0 * ky1, k11 = kx1 * ky1;
-    const T km[8] = {k00 * kz0, k10 * kz0, k01 * kz0, k11 * kz0, k00 * kz1, k10 * kz1, k01 * kz1, k11 * kz1};
-    C acc = cscale(p[0], km[0]);
-#pragma unroll
-    for (int m = 1; m < 8; ++m) acc = cadd(acc, cscale(p[m], km[m]));
-    v[z] = cscale(acc, static_cast<T>(0.125));
+    for (int r = 0; r < A; ++r) row[r * B] = v[r];
   }
-  reg_fft<C, true, H>(v);
-  C* dst = W2 + static_cast<size_t>(slot) * HV + y * H + x;
+  __syncthreads();
+  if constexpr (B > 1) {
+    for (int i = threadIdx.x; i < lines * A; i += kSepThreads) {
+      const int k1 = i / lines;
+      int off = 0;
+      const int at = line(i - k1 * lines, &off);
+      if (at < 0) continue;
+      C* row = buf + at + k1 * B;
+      C v[B];
 #pragma unroll
-  for (int z = 0; z < H; ++z) dst[z * H * H] = v[z];
+      for (int r = 0; r < B; ++r) v[r] = row[r];
+      reg_fft<C, false, B>(v);
+#pragma unroll
+      for (int r = 0; r < B; ++r) row[r] = v[r];
+    }
+    __syncthreads();
+  }
+  {
+    const C* tq = QS;          // tq[d * H + q]
+    const C* kf = QS + 3 * H;  // kf[d * 2H + h].x
+    int img[8];                // representative a negates the axes of bit set img[a]
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+      img[a] = (g->rep_R[a][0] < 0 ? 1 : 0) | (g->rep_R[a][4] < 0 ? 2 : 0) | (g->rep_R[a][8] < 0 ? 4 : 0);
+    const C twy = tq[H + y];
+    const T ky0 = kf[2 * H + y].x, ky1 = kf[2 * H + y + H].x;
+    for (int i = threadIdx.x; i < np * HP; i += kSepThreads) {
+      const int k = i / HP, z = i - k * HP, p = p0 + k;
+      const int zm = z ? H - z : 0;
+      const bool sx = p == 0 || 2 * p == H, sy = rows == 1, sz = zm == z;
+      const int xo[2] = {k * S, sx ? k * S : (PP + k) * S}, yo[2] = {0, sy ? 0 : 2 * PP * S};
+      const int zo[2] = {line_pos<H>(z), line_pos<H>(zm)};
+      const C twx = tq[p], twz = tq[2 * H + z];
+      const C txy = cmul(twx, twy), txz = cmul(twx, twz), tyz = cmul(twy, twz), txyz = cmul(txy, twz);
+      const C t8[8] = {mk<C>(static_cast<T>(1), static_cast<T>(0)), twx, twy, txy, twz, txz, tyz, txyz};
+      const T kx0 = kf[p].x, kx1 = kf[p + H].x, kz0 = kf[4 * H + z].x, kz1 = kf[4 * H + z + H].x;
+      const T e = static_cast<T>(0.125);
+      const T k00 = e * kx0 * ky0, k10 = e * kx1 * ky0, k01 = e * kx0 * ky1, k11 = e * kx1 * ky1;
+      const T km[8] = {k00 * kz0, k10 * kz0, k01 * kz0, k11 * kz0, k00 * kz1, k10 * kz1, k01 * kz1, k11 * kz1};
+      C v[8];
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        v[a] = buf[xo[img[a] & 1] + yo[(img[a] >> 1) & 1] + zo[(img[a] >> 2) & 1]];
+        if (a) v[a] = cmul(v[a], t8[a]);
+      }
+      wht8c(v);
+#pragma unroll
+      for (int a = 0; a < 8; ++a) v[a] = cscale(v[a], km[a]);
+      wht8c(v);
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        const int m = img[a];
+        if (((m & 1) && sx) || ((m & 2) && sy) || ((m & 4) && sz)) continue;  // the same point again
+        buf[xo[m & 1] + yo[(m >> 1) & 1] + zo[(m >> 2) & 1]] = a ? cmulc(v[a], t8[a]) : v[a];
+      }
+    }
+  }
+  __syncthreads();
+  if constexpr (B > 1) {
+    for (int i = threadIdx.x; i < lines * A; i += kSepThreads) {
+      const int k1 = i / lines;
+      int off = 0;
+      const int at = line(i - k1 * lines, &off);
+      if (at < 0) continue;
+      C* row = buf + at + k1 * B;
+      C v[B];
+#pragma unroll
+      for (int r = 0; r < B; ++r) v[r] = row[r];
+      reg_fft<C, true, B>(v);
+#pragma unroll
+      for (int r = 0; r < B; ++r) row[r] = r ? cmulc(v[r], tw[r * k1]) : v[r];
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < lines * B; i += kSepThreads) {
+    const int j = i / lines;
+    int off = 0;
+    const int at = line(i - j * lines, &off);
+    if (at < 0) continue;
+    const C* row = buf + at + j;
+    C v[A];
+#pragma unroll
+    for (int r = 0; r < A; ++r) v[r] = row[r * B];
+    reg_fft<C, true, A>(v);
+    C* dst = Ws + off + j * H * H;
+#pragma unroll
+    for (int r = 0; r < A; ++r) dst[r * B * H * H] = v[r];
+  }
 }
 
 constexpr int kMaxDynSmemFast = 227 * 1024;
@@ -2157,6 +2246,7 @@ Status fast_unit_init(std::string* err) {
         cudaFuncSetAttribute(k_expand_ifft_z<T, HH, wide_slots<CC>(), expand_slots<CC, HH, wide_slots<CC>()>(), sizeof(T) == 8>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
         cudaFuncSetAttribute(k_expand_ifft_z<T, HH, 2, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
+        cudaFuncSetAttribute(k_qsep_z<T, HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
         cudaFuncSetAttribute(k_expand_ifft_z_h<T, HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
       }
     });
@@ -2372,6 +2462,15 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
         });
         break;
       }
+      case 7:  // forward z FFT + separable Q-multiply + inverse z FFT, in place on W
+        CFFT_FOR_H(H, {
+          constexpr int HP = HH / 2 + 1;
+          const int want = (2 * kSMs + HP * nslots - 1) / (HP * nslots);  // blocks per row that give two CTAs per SM
+          const int pp = std::max(2, (HP + want - 1) / want);
+          launch_k(k_qsep_z<T, HH>, dim3(HP, (HP + pp - 1) / pp, nslots), kSepThreads,
+                   (static_cast<size_t>(4) * pp * (HH + 1) + HH) * sizeof(C), st, g, tab, static_cast<const C*>(a.QS), W, pp);
+        });
+        break;
       case 3: {
         const int no = a.n_orbits;
         if (a.reps_quad) {
@@ -2398,18 +2497,11 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
         break;
       }
       default:
-        if (a.q_step && a.qsep) {
-          CFFT_FOR_H(H, {
-            launch_k(k_qsep_ifft_z_h<T, HH>, gz, thr_z, 0, st, g, static_cast<const C*>(a.QS), W,
-                     static_cast<C*>(a.W2));
-          });
-          break;
-        }
         if (a.q_step) {
           CFFT_FOR_H(H, {
-            launch_k(k_qmul_ifft_z_h<T, HH>, gz, thr_z, 0, st, g, static_cast<const C*>(a.QT),
-                                                         static_cast<const int32_t*>(a.GT), W,
-                                                         static_cast<C*>(a.W2));
+            launch_k(k_qmul_ifft_z_h<T, HH>, dim3(HH, nch, nslots), expand_threads<C, HH, 2>(),
+                     (expand_plane<HH>() + HH) * sizeof(C), st, g, tab, static_cast<const C*>(a.QT),
+                     static_cast<const int32_t*>(a.GT), W, static_cast<C*>(a.W2));
           });
           break;
         }

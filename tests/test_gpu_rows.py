@@ -12,7 +12,7 @@ at 48^3 points and 1.5e-14 for FP64, and the round trip doubles that.  The bars 
 import numpy as np
 import pytest
 
-from conftest import rel_err
+from conftest import q_plan, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +57,21 @@ def test_fiber_phases(cf, O, prep, sg):
 
 def test_largest_edge(cf, O, prep):
     check(cf, O, prep, 221, (96, 96, 96), 4, 3)  # plain lattice, 48 points per line
+
+
+@pytest.mark.parametrize("sg,n,batch,precision", [(47, 8, 1, 8), (47, 12, 3, 8), (200, 16, 2, 4), (221, 24, 40, 8), (47, 48, 2, 4),
+                                                  (123, 64, 7, 8), (47, 96, 3, 4)])
+def test_separable_step(cf, O, prep, sg, n, batch, precision):
+    # both z transforms and the Q-multiply in one kernel: blocks of few and of all line pairs
+    N, lat = (n, n, n), np.diag([1.0, 1.0, 1.3]) if sg == 123 else np.diag([1.0, 1.3, 0.8]) if sg == 47 else np.eye(3)
+    p = prep(sg, N, seed=33)
+    plan = q_plan(cf, p, cf.PATH_M2Q, 0.01, lat, precision=precision, max_batch=batch)
+    assert plan.info.exec_path & 64
+    f0 = O.pack_stride(p["u"], plan.L).T
+    want = O.fullgrid_reference(p["u"], N, 0.01, lat, plan.L).T
+    scale = np.arange(1, batch + 1).reshape(-1, 1, 1, 1)
+    q = torch.tensor(scale * f0, device="cuda", dtype=torch.float32 if precision == 4 else torch.float64)
+    plan.scft_step(q)
+    for b in range(batch):
+        assert rel_err(q[b].cpu().numpy(), (b + 1) * want) < 2 * TOL[precision], b
+    plan.close()
