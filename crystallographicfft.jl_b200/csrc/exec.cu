@@ -451,25 +451,74 @@ __global__ void k_block_scale(const int32_t* __restrict__ dims, const long long*
   }
 }
 
+// Stride-L subgrid of whole-grid fields: one row (y, z) of a field per block row, threads
+// along x.
 template <typename T>
-__global__ void k_full_to_sub(const T* __restrict__ u, T* __restrict__ f0, int N1, int N2, int L1, int L2, int L3,
-                              int M1, int M2, size_t mvol, size_t nvol, int B) {
-  const size_t tot = mvol * B;
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < tot; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const size_t b = i / mvol, r = i % mvol;
-    const size_t x = r % M1, y = (r / M1) % M2, z = r / (static_cast<size_t>(M1) * M2);
-    f0[i] = u[b * nvol + (z * L3 * N2 + y * L2) * N1 + x * L1];
+__global__ void __launch_bounds__(256) k_full_to_sub(const T* __restrict__ u, T* __restrict__ f0, int N1, int N2, int L1, int L2,
+                                                     int L3, int M1, int M2, int M3, size_t mvol, size_t nvol) {
+  const int y = blockIdx.x * blockDim.y + threadIdx.y, z = blockIdx.y, b = blockIdx.z;
+  if (y >= M2) return;
+  const T* src = u + b * nvol + (static_cast<size_t>(z) * L3 * N2 + static_cast<size_t>(y) * L2) * N1;
+  T* dst = f0 + b * mvol + (static_cast<size_t>(z) * M2 + y) * M1;
+  for (int x = threadIdx.x; x < M1; x += blockDim.x) dst[x] = src[x * L1];
+}
+
+// Symmetry fill: u(r) = f0(fill_map(r)).  A thread takes VW neighbouring points (VW = 4 with
+// 16-byte aligned map rows and even field sizes) of up to kFillFields fields: the map entries
+// are read once for all of them and the stores are vectors.
+constexpr int kFillFields = 4;
+template <typename T, int VW>
+__global__ void __launch_bounds__(256) k_sub_to_full(const T* __restrict__ f0, const int32_t* __restrict__ fill_map,
+                                                     T* __restrict__ u, size_t mvol, size_t nvol, int B) {
+  const size_t r = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * VW;
+  if (r >= nvol) return;
+  int m[VW];
+  if constexpr (VW == 4) {
+    const int4 v = __ldg(reinterpret_cast<const int4*>(fill_map + r));
+    m[0] = v.x; m[1] = v.y; m[2] = v.z; m[3] = v.w;
+  } else {
+    m[0] = __ldg(fill_map + r);
+  }
+  const int b0 = blockIdx.y * kFillFields;
+#pragma unroll
+  for (int k = 0; k < kFillFields; ++k) {
+    if (b0 + k >= B) break;
+    const T* f = f0 + (b0 + k) * mvol;
+    T v[VW];
+#pragma unroll
+    for (int l = 0; l < VW; ++l) v[l] = __ldg(f + m[l]);
+    T* d = u + (b0 + k) * nvol + r;
+    if constexpr (VW == 4) {
+      vstore<T>(d, v);
+      if constexpr (sizeof(T) == 8) vstore<T>(d + 2, v + 2);
+    } else {
+      *d = v[0];
+    }
   }
 }
 
-template <typename T>
-__global__ void k_sub_to_full(const T* __restrict__ f0, const int32_t* __restrict__ fill_map, T* __restrict__ u,
-                              size_t mvol, size_t nvol, int B) {
-  const size_t tot = nvol * B;
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < tot; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const size_t b = i / nvol, r = i % nvol;
-    u[i] = f0[b * mvol + fill_map[r]];
+// _build_fill_map (src/q_fused_krfft.jl:733-783): for each grid point the first operation that
+// lands it on the stride-L subgrid; `missing` counts the points that none does.  ops: 12
+// words per operation (R row-major, t).
+__global__ void __launch_bounds__(256) k_fill_map(const int32_t* __restrict__ ops, int n_ops, int N1, int N2, int N3, int L1,
+                                                  int L2, int L3, int M1, int M2, int32_t* __restrict__ map, int* __restrict__ missing) {
+  const int N[3] = {N1, N2, N3}, L[3] = {L1, L2, L3};
+  const long n = static_cast<long>(N1) * N2 * N3, i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int X[3] = {static_cast<int>(i % N1), static_cast<int>((i / N1) % N2), static_cast<int>(i / (static_cast<long>(N1) * N2))};
+  for (int o = 0; o < n_ops; ++o) {
+    const int32_t* op = ops + 12 * o;
+    int s[3];
+    bool on = true;
+    for (int d = 0; d < 3 && on; ++d) {
+      int v = (op[3 * d] * X[0] + op[3 * d + 1] * X[1] + op[3 * d + 2] * X[2] + op[9 + d]) % N[d];
+      if (v < 0) v += N[d];
+      on = v % L[d] == 0;
+      s[d] = v / L[d];
+    }
+    if (on) { map[i] = s[0] + M1 * (s[1] + M2 * s[2]); return; }
   }
+  atomicAdd(missing, 1);
 }
 
 // ---------------------------------------------------------------- host helpers
@@ -666,7 +715,8 @@ Status launch_stage(Plan* p, int stage, const T* f0, typename Cx<T>::type* F, co
   const C* tab = static_cast<const C*>(p->d_tables);
   C* W = reinterpret_cast<C*>(static_cast<char*>(p->d_work_T) + lane * p->w_lane_bytes);
   const PlanTables& T_ = p->T;
-  if (p->fast_h > 0) {
+  if (p->fast_h > 0 || p->general) {
+    if (p->general && (stage == 1 || stage == 4) && T_.H[2] <= 1) return Status::kOk;  // one z plane
     if (p->cluster && (stage == 1 || stage == 4)) return Status::kOk;  // fused into stages 0 and 5
     FastArgs a;
     a.geom = p->d_geom; a.tables = p->d_tables; a.spec_h = p->d_spec_h; a.K = p->d_K;
@@ -700,7 +750,8 @@ Status launch_stage(Plan* p, int stage, const T* f0, typename Cx<T>::type* F, co
     }
     a.stream = st;
     const bool planes = stage == 0 || stage == 5;
-    Status s = sizeof(T) == 4 ? (planes ? fast_planes_f32(a, err) : fast_other_f32(a, err))
+    Status s = p->general && stage != 3 ? (sizeof(T) == 4 ? general_f32(a, p->gen, err) : general_f64(a, p->gen, err))
+               : sizeof(T) == 4 ? (planes ? fast_planes_f32(a, err) : fast_other_f32(a, err))
                               : (planes ? fast_planes_f64(a, err) : fast_other_f64(a, err));
     ++g_launches;
     return s;
@@ -873,6 +924,38 @@ static long q_of_channel_point(const PlanTables& T, int c, int x, int y, int z) 
   return (2 * x + o[0]) + static_cast<long>(T.M[0]) * ((2 * y + o[1]) + static_cast<long>(T.M[1]) * (2 * z + o[2]));
 }
 
+// n = A x B with A >= B, both radices of the general kernels, the closest to square.
+static bool general_split(int n, int* A, int* B) {
+  auto radix = [](int r) { return r <= 6 || r == 8 || r == 9 || r == 10 || r == 12 || r == 15 || r == 16; };
+  if (n <= 10 && radix(n)) { *A = n; *B = 1; return true; }
+  for (int a = 2; a <= 16; ++a)
+    if (n % a == 0 && n / a <= a && radix(a) && radix(n / a)) { *A = a; *B = n / a; return true; }
+  return false;
+}
+
+static void fill_general(const DevGeom& g, const PlanTables& T, GenShape* s) {
+  auto mul = [](int d) { return d == 1 ? 0u : static_cast<uint32_t>(((1ull << 32) + d - 1) / d); };
+  s->nch = T.n_ch; s->centered = T.centered ? 1 : 0; s->d = T.d; s->P = T.P;
+  s->n_spec = static_cast<int>(T.spec.size());
+  s->n_orbits = static_cast<int>(T.orbit_rep.size());
+  s->S = T.H[0] | 1;
+  s->ph = g.ph_off;
+  s->hvol = s->mvol = 1;
+  for (int k = 0; k < 8; ++k) s->chan[k] = T.centered ? T.chan_of_parity[k] : (k == 0 ? 0 : -1);
+  for (int d = 0; d < 3; ++d) {
+    s->H[d] = T.H[d]; s->M[d] = T.M[d]; s->N[d] = T.N[d];
+    s->tw[d] = g.tw_off[d]; s->ftw[d] = g.ftw_off[d];
+    s->lift[d] = (3 * 1024 + T.M[d] - 1) / T.M[d] * T.M[d];
+    s->PN[d] = T.P / T.N[d];
+    s->dH[d] = mul(T.H[d]); s->dA[d] = mul(s->A[d]); s->dB[d] = mul(s->B[d]); s->dM[d] = mul(T.M[d]); s->dN[d] = mul(T.N[d]);
+    s->hvol *= T.H[d];
+    s->mvol *= T.M[d];
+  }
+  s->dLx = mul(T.n_ch * T.H[1]);
+  s->dLy = mul(T.n_ch * T.H[0]);
+  s->inv_v = 1.0 / static_cast<double>(s->mvol);
+}
+
 // Fibers of the inverse gather (k_inv_fiber).  Orbits are taken in order; an orbit not
 // yet served opens a fiber whose taps are its own alias row, and the fiber also serves the
 // orbit of each image R_b^T q whose row, written out as a linear form in the spectrum
@@ -940,7 +1023,8 @@ static int build_fibers(const PlanTables& T, const std::vector<int2>& expand, st
       const long c = friedel[(w & 0x7FFFFFFFu) - 1];
       if (c >= 0) { w &= 0x7FFFFFFFu; j += c; }
     }
-    return (static_cast<uint64_t>(w) << 32) | static_cast<uint64_t>(floor_mod(j, P));
+    while (j >= P) j -= P;
+    return (static_cast<uint64_t>(w) << 32) | static_cast<uint64_t>(j);
   };
   for (size_t o = 0; o < no; ++o) {
     if (served[o]) continue;
@@ -956,7 +1040,9 @@ static int build_fibers(const PlanTables& T, const std::vector<int2>& expand, st
       for (int k = 0; k < 3; ++k) {
         long v = 0;
         for (int i = 0; i < 3; ++i) v += static_cast<long>(T.rep_ops[b].R[i][k]) * q[i];
-        idx[k] = floor_mod(v, T.M[k]);
+        while (v < 0) v += T.M[k];
+        while (v >= T.M[k]) v -= T.M[k];
+        idx[k] = v;
         jt += q[k] * T.rep_ops[b].t[k] * (P / T.N[k]);
       }
       long pos;
@@ -1087,41 +1173,52 @@ Status plan_device_init(Plan* p, std::string* err) {
   if (const char* f = std::getenv("CFFT_DISABLE_FAST")) {
     if (f[0] == '1') p->fast_h = 0;
   }
-  // distinct-image masks: op i contributes only if no earlier op maps the representative to the same point
-  std::vector<uint32_t> masks(static_cast<size_t>(g.n_orbits) * p->n_mask_words, 0u);
+  // General kernels: every axis length splits into two register radices, and the packed
+  // tables fit (the conditions of reps_quad below).
+  p->general = !p->fast_h && T.spec.size() < (1u << 20) - 1 && T.P <= 2048 && T.orbit_rep.size() < (1u << 21);
+  for (int d = 0; d < 3 && p->general; ++d) p->general = general_split(T.H[d], &p->gen.A[d], &p->gen.B[d]);
   const size_t hvol = static_cast<size_t>(T.H[0]) * T.H[1] * T.H[2];
+  const bool tables = p->fast_h || p->general;
+  // Expansion of the orbits over the channel points: the first operation that maps a
+  // representative to a point gives its phase.  The Stockham path (no packed tables) keeps
+  // that choice as one bit per operation instead.
+  std::vector<uint32_t> masks;
   std::vector<int2> expand;
-  if (p->fast_h) expand.assign(static_cast<size_t>(T.n_ch) * hvol, make_int2(-1, 0));
+  if (tables) expand.assign(static_cast<size_t>(T.n_ch) * hvol, make_int2(-1, 0));
+  else masks.assign(static_cast<size_t>(g.n_orbits) * p->n_mask_words, 0u);
+  std::vector<long> seen;
   for (int o = 0; o < g.n_orbits; ++o) {
     const int m = T.orbit_rep[o];
     const int q[3] = {m % T.M[0], (m / T.M[0]) % T.M[1], m / (T.M[0] * T.M[1])};
-    std::vector<long> seen;
+    seen.clear();
     for (int i = 0; i < g.n_rem; ++i) {
-      long li = 0, stride = 1;
       int qq[3];
       for (int dd = 0; dd < 3; ++dd) {
-        long v = 0;
-        for (int d2 = 0; d2 < 3; ++d2) v += static_cast<long>(T.rem_ops[i].R[d2][dd]) * q[d2];
-        qq[dd] = static_cast<int>(floor_mod(v, T.M[dd]));
-        li += qq[dd] * stride;
-        stride *= T.M[dd];
+        int v = 0;
+        for (int d2 = 0; d2 < 3; ++d2) v += T.rem_ops[i].R[d2][dd] * q[d2];
+        while (v < 0) v += T.M[dd];
+        while (v >= T.M[dd]) v -= T.M[dd];
+        qq[dd] = v;
       }
-      if (std::find(seen.begin(), seen.end(), li) != seen.end()) continue;
-      seen.push_back(li);
-      masks[static_cast<size_t>(o) * p->n_mask_words + (i >> 5)] |= 1u << (i & 31);
-      if (p->fast_h) {
-        long j = 0;
-        for (int dd = 0; dd < 3; ++dd) j += static_cast<long>(q[dd]) * T.rem_ops[i].t[dd] * (T.P / T.M[dd]);
-        size_t pos;
-        if (T.centered) {
-          const int c = T.chan_of_parity[(qq[0] & 1) + 2 * (qq[1] & 1) + 4 * (qq[2] & 1)];
-          if (c < 0) { *err = "orbit image outside the alive channels"; return Status::kInvalid; }
-          pos = static_cast<size_t>(c) * hvol + (static_cast<size_t>(qq[2] >> 1) * T.H[1] + (qq[1] >> 1)) * T.H[0] + (qq[0] >> 1);
-        } else {
-          pos = (static_cast<size_t>(qq[2]) * T.H[1] + qq[1]) * T.H[0] + qq[0];
-        }
-        expand[pos] = make_int2(o, static_cast<int>(floor_mod(j, T.P)));
+      if (!tables) {
+        const long li = qq[0] + static_cast<long>(T.M[0]) * (qq[1] + static_cast<long>(T.M[1]) * qq[2]);
+        if (std::find(seen.begin(), seen.end(), li) != seen.end()) continue;
+        seen.push_back(li);
+        masks[static_cast<size_t>(o) * p->n_mask_words + (i >> 5)] |= 1u << (i & 31);
+        continue;
       }
+      size_t pos;
+      if (T.centered) {
+        const int c = T.chan_of_parity[(qq[0] & 1) + 2 * (qq[1] & 1) + 4 * (qq[2] & 1)];
+        if (c < 0) { *err = "orbit image outside the alive channels"; return Status::kInvalid; }
+        pos = static_cast<size_t>(c) * hvol + (static_cast<size_t>(qq[2] >> 1) * T.H[1] + (qq[1] >> 1)) * T.H[0] + (qq[0] >> 1);
+      } else {
+        pos = (static_cast<size_t>(qq[2]) * T.H[1] + qq[1]) * T.H[0] + qq[0];
+      }
+      if (expand[pos].x >= 0) continue;
+      long j = 0;
+      for (int dd = 0; dd < 3; ++dd) j += static_cast<long>(q[dd]) * T.rem_ops[i].t[dd] * (T.P / T.M[dd]);
+      expand[pos] = make_int2(o, static_cast<int>(floor_mod(j, T.P)));
     }
   }
   for (const int2& e : expand)
@@ -1131,6 +1228,8 @@ Status plan_device_init(Plan* p, std::string* err) {
     hp[s] = static_cast<uint32_t>(T.spec[s].h[0]) | (static_cast<uint32_t>(T.spec[s].h[1]) << 10) |
             (static_cast<uint32_t>(T.spec[s].h[2]) << 20);
   std::vector<unsigned char> tab = p->precision == 8 ? make_table_bytes<double>(*p, &g) : make_table_bytes<float>(*p, &g);
+
+  if (p->general) fill_general(g, T, &p->gen);
 
   const size_t rs = p->precision;          // real size
   const size_t cs = 2 * rs;                // complex size
@@ -1142,15 +1241,15 @@ Status plan_device_init(Plan* p, std::string* err) {
   size_t budget = static_cast<size_t>(64) << 20;
   if (const char* cb = std::getenv("CFFT_CHUNK_BYTES")) budget = std::strtoull(cb, nullptr, 10);
   if (p->tune.chunk_bytes > 0) budget = static_cast<size_t>(p->tune.chunk_bytes);
-  const size_t per_field = T.n_ch * hvol * cs / (p->fast_h ? 2 : 1);
+  const size_t per_field = T.n_ch * hvol * cs / (tables ? 2 : 1);
   size_t ch = std::max<size_t>(1, std::min<size_t>(B, budget / std::max<size_t>(per_field, 1)));
   // Batches of at least 8 fields on the fast path run as two concurrent lanes.
   p->lanes = 1;
   if (p->tune.lanes > 0) p->lanes = std::min(Plan::kMaxLanes, p->tune.lanes);
   else if (const char* ln = std::getenv("CFFT_LANES")) p->lanes = std::max(1, std::min(Plan::kMaxLanes, std::atoi(ln)));
-  else if (p->fast_h && B >= 8) p->lanes = 2;
+  else if (tables && B >= 8) p->lanes = 2;
   if (p->lanes > 1) ch = std::min(ch, (B + p->lanes - 1) / p->lanes);
-  if (p->fast_h && ch < B && ch > 1) ch &= ~static_cast<size_t>(1);
+  if (tables && ch < B && ch > 1) ch &= ~static_cast<size_t>(1);
   p->chunk = static_cast<int>(ch);
   // launch geometry and shared memory (generic path)
   const long pe = static_cast<long>(T.n_ch) * T.H[0] * T.H[1];
@@ -1173,22 +1272,25 @@ Status plan_device_init(Plan* p, std::string* err) {
   if ((st = alloc(&p->d_tables, tab.size(), "tables")) != Status::kOk) return st;
   if ((st = alloc(&p->d_spec_h, hp.size() * 4, "spectral points")) != Status::kOk) return st;
   if ((st = alloc(&p->d_K, T.spec.size() * rs, "kernel")) != Status::kOk) return st;
-  if ((st = alloc(&p->d_orbit_rep, T.orbit_rep.size() * 4, "orbit reps")) != Status::kOk) return st;
-  if ((st = alloc(&p->d_inv_spec, T.inv_spec.size() * 4, "inverse spec")) != Status::kOk) return st;
-  if ((st = alloc(&p->d_inv_phase, T.inv_phase.size() * 4, "inverse phase")) != Status::kOk) return st;
-  if ((st = alloc(&p->d_img_mask, masks.size() * 4, "image masks")) != Status::kOk) return st;
-  p->w_lane_bytes = ((chunk * T.n_ch * hvol * cs + 255) / 256) * 256;
+  p->reps_quad = tables && T.spec.size() < (1u << 20) - 1 && T.P <= 2048 && T.orbit_rep.size() < (1u << 21);
+  if (!p->reps_quad) {  // the fibers replace these
+    if ((st = alloc(&p->d_orbit_rep, T.orbit_rep.size() * 4, "orbit reps")) != Status::kOk) return st;
+    if ((st = alloc(&p->d_inv_spec, T.inv_spec.size() * 4, "inverse spec")) != Status::kOk) return st;
+    if ((st = alloc(&p->d_inv_phase, T.inv_phase.size() * 4, "inverse phase")) != Status::kOk) return st;
+    if ((st = alloc(&p->d_img_mask, masks.size() * 4, "image masks")) != Status::kOk) return st;
+  }
+  const size_t slots = p->general ? (chunk + 1) / 2 : chunk;
+  p->w_lane_bytes = ((slots * T.n_ch * hvol * cs + 255) / 256) * 256;
   if ((st = alloc(&p->d_work_T, p->lanes * p->w_lane_bytes, "channel workspace")) != Status::kOk) return st;
   if ((st = alloc(&p->d_work_F, B * T.spec.size() * cs, "spectrum workspace")) != Status::kOk) return st;
   if ((st = alloc(&p->d_work_E, B * mvol * rs, "interaction workspace")) != Status::kOk) return st;
-  p->reps_quad = p->fast_h && T.spec.size() < (1u << 20) - 1 && T.P <= 2048 && T.orbit_rep.size() < (1u << 21);
   std::vector<uint2> fib_taps, fib_outs;
   if (p->reps_quad) {
     p->n_fib = build_fibers(T, expand, &fib_taps, &fib_outs);
     if ((st = alloc(&p->d_fib_taps, fib_taps.size() * sizeof(uint2), "fiber taps")) != Status::kOk) return st;
     if ((st = alloc(&p->d_fib_outs, fib_outs.size() * sizeof(uint2), "fiber outputs")) != Status::kOk) return st;
   }
-  if (p->fast_h) {
+  if (tables) {
     // Packed expansion entries (orbit | phase << 21) where they fit 32 bits.
     if ((st = alloc(&p->d_expand, expand.size() * (p->reps_quad ? 4 : sizeof(int2)), "expansion table")) != Status::kOk)
       return st;
@@ -1199,7 +1301,7 @@ Status plan_device_init(Plan* p, std::string* err) {
     const char* cl_env = std::getenv("CFFT_CLUSTER");
     const bool cluster_wanted = p->tune.cluster >= 0 ? p->tune.cluster > 0 : (cl_env && std::atoi(cl_env) > 0);
     const bool wide_wanted = p->tune.wide >= 0 ? p->tune.wide > 0 : !(wide_env && wide_env[0] == '0');
-    p->reps_wide = p->reps_quad && chunk >= gw && wide_wanted && !cluster_wanted;
+    p->reps_wide = p->fast_h && p->reps_quad && chunk >= gw && wide_wanted && !cluster_wanted;
     const size_t chunk4 = p->reps_wide ? (chunk + gw - 1) / gw * gw : (chunk + 3) / 4 * 4;  // whole rows of slots
     p->g0r_lane_bytes = (((p->reps_quad ? chunk4 : chunk + 1) * T.orbit_rep.size() * cs + 255) / 256) * 256;
     if ((st = alloc(&p->d_g0r, p->lanes * p->g0r_lane_bytes, "representative workspace")) != Status::kOk) return st;
@@ -1263,13 +1365,14 @@ Status plan_device_init(Plan* p, std::string* err) {
   CFFT_CUDA(cudaMemcpy(p->d_geom, &g, sizeof(g), cudaMemcpyHostToDevice), "upload geometry");
   CFFT_CUDA(cudaMemcpy(p->d_tables, tab.data(), tab.size(), cudaMemcpyHostToDevice), "upload tables");
   CFFT_CUDA(cudaMemcpy(p->d_spec_h, hp.data(), hp.size() * 4, cudaMemcpyHostToDevice), "upload spectral points");
-  if (!T.orbit_rep.empty()) {
+  if (!T.orbit_rep.empty() && !p->reps_quad) {
     CFFT_CUDA(cudaMemcpy(p->d_orbit_rep, T.orbit_rep.data(), T.orbit_rep.size() * 4, cudaMemcpyHostToDevice), "upload reps");
     CFFT_CUDA(cudaMemcpy(p->d_inv_spec, T.inv_spec.data(), T.inv_spec.size() * 4, cudaMemcpyHostToDevice), "upload inv spec");
     CFFT_CUDA(cudaMemcpy(p->d_inv_phase, T.inv_phase.data(), T.inv_phase.size() * 4, cudaMemcpyHostToDevice), "upload inv phase");
-    CFFT_CUDA(cudaMemcpy(p->d_img_mask, masks.data(), masks.size() * 4, cudaMemcpyHostToDevice), "upload masks");
+    if (!masks.empty())
+      CFFT_CUDA(cudaMemcpy(p->d_img_mask, masks.data(), masks.size() * 4, cudaMemcpyHostToDevice), "upload masks");
   }
-  if (p->fast_h && p->reps_quad) {
+  if (p->reps_quad) {
     std::vector<uint32_t> epk(expand.size());
     for (size_t i = 0; i < expand.size(); ++i)
       epk[i] = static_cast<uint32_t>(expand[i].x) | (static_cast<uint32_t>(expand[i].y) << 21);
@@ -1331,6 +1434,9 @@ Status plan_device_init(Plan* p, std::string* err) {
     CFFT_CUDA(cudaHostGetDevicePointer(&ds, hs, 0), "status word device address");
     p->d_status = static_cast<int*>(ds);
     if (const char* e = std::getenv("CFFT_WAIT_TIMEOUT_NS")) p->timeout_ns = std::strtoull(e, nullptr, 10);
+  }
+  if (p->general) {
+    if ((st = p->precision == 8 ? general_init_f64(err) : general_init_f32(err)) != Status::kOk) return st;
   }
   cudaStream_t s;
   CFFT_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "create stream");
@@ -1585,37 +1691,42 @@ Status exec_step_diffusion(Plan* p, void* q, const void* w, double dt, int n_ste
   return Status::kOk;
 }
 
-// _build_fill_map (src/q_fused_krfft.jl:733-783): for each grid point the first
-// operation that lands it on the stride-L subgrid.
 static Status ensure_fill_map(Plan* p, std::string* err) {
   if (p->d_fill_map) return Status::kOk;
   const PlanTables& T = p->T;
-  const long n1 = T.N[0], n2 = T.N[1], n3 = T.N[2];
-  p->fill_map.assign(n1 * n2 * n3, -1);
-  for (long z = 0; z < n3; ++z)
-    for (long y = 0; y < n2; ++y)
-      for (long x = 0; x < n1; ++x) {
-        const long X[3] = {x, y, z};
-        for (const auto& op : T.ops) {
-          long sub = 0, stride = 1;
-          bool on = true;
-          for (int d = 0; d < 3 && on; ++d) {
-            long v = op.t[d];
-            for (int j = 0; j < 3; ++j) v += static_cast<long>(op.R[d][j]) * X[j];
-            v = floor_mod(v, T.N[d]);
-            if (v % T.L[d] != 0) on = false;
-            sub += (v / T.L[d]) * stride;
-            stride *= T.M[d];
-          }
-          if (on) { p->fill_map[x + n1 * (y + n2 * z)] = static_cast<int32_t>(sub); break; }
-        }
-        if (p->fill_map[x + n1 * (y + n2 * z)] < 0) {
-          *err = "No symmetry operation maps a grid point to the subgrid";
-          return Status::kInvalid;
-        }
-      }
-  CFFT_CUDA(cudaMalloc(&p->d_fill_map, p->fill_map.size() * 4), "alloc fill map");
-  CFFT_CUDA(cudaMemcpy(p->d_fill_map, p->fill_map.data(), p->fill_map.size() * 4, cudaMemcpyHostToDevice), "upload fill map");
+  const long n = static_cast<long>(T.N[0]) * T.N[1] * T.N[2];
+  std::vector<int32_t> ops;
+  for (const auto& op : T.ops) {
+    for (int i = 0; i < 3; ++i)
+      for (int j = 0; j < 3; ++j) ops.push_back(op.R[i][j]);
+    for (int i = 0; i < 3; ++i) ops.push_back(op.t[i]);
+  }
+  void *map = nullptr, *tmp = nullptr;
+  const size_t ob = ops.size() * 4;
+  int missing = 0;
+  cudaError_t e = cudaMalloc(&map, static_cast<size_t>(n) * 4);
+  if (e == cudaSuccess) e = cudaMalloc(&tmp, ob + 4);
+  cudaStream_t s = static_cast<cudaStream_t>(p->own_stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(tmp, ops.data(), ob, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(static_cast<char*>(tmp) + ob, 0, 4, s);
+  if (e == cudaSuccess) {
+    int* count = reinterpret_cast<int*>(static_cast<char*>(tmp) + ob);
+    k_fill_map<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(static_cast<const int32_t*>(tmp), static_cast<int>(T.ops.size()),
+                                                                    T.N[0], T.N[1], T.N[2], T.L[0], T.L[1], T.L[2], T.M[0], T.M[1],
+                                                                    static_cast<int32_t*>(map), count);
+    ++g_launches;
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&missing, count, 4, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  }
+  if (tmp) cudaFree(tmp);
+  if (e != cudaSuccess || missing) {
+    if (map) cudaFree(map);
+    if (e != cudaSuccess) { *err = cuda_msg(e, "fill map"); return Status::kCuda; }
+    *err = "No symmetry operation maps a grid point to the subgrid";
+    return Status::kInvalid;
+  }
+  p->d_fill_map = map;
   return Status::kOk;
 }
 
@@ -1626,13 +1737,17 @@ Status exec_full_to_sub(Plan* p, const void* u, void* f0, int B, void* stream, s
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t mvol = static_cast<size_t>(T.M[0]) * T.M[1] * T.M[2];
   const size_t nvol = static_cast<size_t>(T.N[0]) * T.N[1] * T.N[2];
-  const int grid = static_cast<int>(std::min<size_t>((mvol * B + 255) / 256, 148 * 16));
-  if (p->precision == 8)
-    k_full_to_sub<double><<<grid, 256, 0, s>>>(static_cast<const double*>(u), static_cast<double*>(f0), T.N[0], T.N[1],
-                                               T.L[0], T.L[1], T.L[2], T.M[0], T.M[1], mvol, nvol, B);
-  else
-    k_full_to_sub<float><<<grid, 256, 0, s>>>(static_cast<const float*>(u), static_cast<float*>(f0), T.N[0], T.N[1],
-                                              T.L[0], T.L[1], T.L[2], T.M[0], T.M[1], mvol, nvol, B);
+  const int bx = T.M[0] <= 32 ? 32 : T.M[0] <= 64 ? 64 : 128;
+  const dim3 blk(bx, 256 / bx);
+  for (int b0 = 0; b0 < B; b0 += 65535) {
+    const dim3 grid((T.M[1] + blk.y - 1) / blk.y, T.M[2], std::min(B - b0, 65535));
+    if (p->precision == 8)
+      k_full_to_sub<double><<<grid, blk, 0, s>>>(static_cast<const double*>(u) + b0 * nvol, static_cast<double*>(f0) + b0 * mvol,
+                                                 T.N[0], T.N[1], T.L[0], T.L[1], T.L[2], T.M[0], T.M[1], T.M[2], mvol, nvol);
+    else
+      k_full_to_sub<float><<<grid, blk, 0, s>>>(static_cast<const float*>(u) + b0 * nvol, static_cast<float*>(f0) + b0 * mvol,
+                                                T.N[0], T.N[1], T.L[0], T.L[1], T.L[2], T.M[0], T.M[1], T.M[2], mvol, nvol);
+  }
   ++g_launches;
   CFFT_CUDA(cudaGetLastError(), "fullgrid_to_subgrid launch");
   return Status::kOk;
@@ -1776,13 +1891,17 @@ Status exec_sub_to_full(Plan* p, const void* f0, void* u, int B, void* stream, s
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t mvol = static_cast<size_t>(T.M[0]) * T.M[1] * T.M[2];
   const size_t nvol = static_cast<size_t>(T.N[0]) * T.N[1] * T.N[2];
-  const int grid = static_cast<int>(std::min<size_t>((nvol * B + 255) / 256, 148 * 16));
-  if (p->precision == 8)
-    k_sub_to_full<double><<<grid, 256, 0, s>>>(static_cast<const double*>(f0), static_cast<const int32_t*>(p->d_fill_map),
-                                               static_cast<double*>(u), mvol, nvol, B);
-  else
-    k_sub_to_full<float><<<grid, 256, 0, s>>>(static_cast<const float*>(f0), static_cast<const int32_t*>(p->d_fill_map),
-                                              static_cast<float*>(u), mvol, nvol, B);
+  const int32_t* map = static_cast<const int32_t*>(p->d_fill_map);
+  const bool vec = nvol % 4 == 0 && reinterpret_cast<uintptr_t>(u) % 16 == 0;
+  const size_t per = vec ? 1024 : 256;
+  const dim3 grid(static_cast<unsigned>((nvol + per - 1) / per), (B + kFillFields - 1) / kFillFields);
+  if (p->precision == 8) {
+    auto* k = vec ? k_sub_to_full<double, 4> : k_sub_to_full<double, 1>;
+    k<<<grid, 256, 0, s>>>(static_cast<const double*>(f0), map, static_cast<double*>(u), mvol, nvol, B);
+  } else {
+    auto* k = vec ? k_sub_to_full<float, 4> : k_sub_to_full<float, 1>;
+    k<<<grid, 256, 0, s>>>(static_cast<const float*>(f0), map, static_cast<float*>(u), mvol, nvol, B);
+  }
   ++g_launches;
   CFFT_CUDA(cudaGetLastError(), "subgrid_to_fullgrid launch");
   return Status::kOk;

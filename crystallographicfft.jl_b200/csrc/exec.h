@@ -4,6 +4,7 @@
 #include <string>
 
 #include "cfft_internal.h"
+#include "fast_api.h"
 
 namespace cfft {
 
@@ -26,7 +27,6 @@ struct Plan {
   double lattice[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
   double ds = 0.0;
   int n_mask_words = 1;
-  std::vector<int32_t> fill_map;  // N-grid -> M-grid linear index (built on first use)
   // device buffers (owned)
   void* d_geom = nullptr;       // DevGeom
   void* d_tables = nullptr;     // twiddles / phases (complex T)
@@ -68,6 +68,8 @@ struct Plan {
   // launch geometry
   int threads_xy = 0, threads_z = 0;
   int fast_h = 0;               // cubic channel edge of the compile-time sized kernels (0 = generic)
+  bool general = false;         // general kernels (any 2-3-5 grid; two fields per slot)
+  GenShape gen;                 // their geometry
   int chunk = 1;                // fields per workspace chunk
   int lanes = 1;                // concurrent chunk lanes
   int cent_type = 0;            // plane-kernel centring (0 plain, 1 I, 2 F, 3 C, 4 A)

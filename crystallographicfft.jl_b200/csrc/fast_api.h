@@ -59,6 +59,25 @@ struct FastArgs {
   int tma = -1;
 };
 
+// Geometry of the general kernels (any 2-3-5 channel grid), passed by value.  Each axis length
+// is A x B with both factors in general_radix; a "d" member is the multiplier of div_by.
+struct GenShape {
+  int H[3], A[3], B[3], M[3], N[3];
+  int nch, centered, d, P, n_spec, n_orbits;
+  int S;             // shared-memory row stride (odd)
+  int chan[8];       // channel of a parity class, or -1
+  int tw[3], ftw[3], ph;  // table offsets: line twiddles, fold twiddles, phases
+  int lift[3];       // multiple of M above any |R^T h|
+  int PN[3];         // P / N
+  uint32_t dH[3], dA[3], dB[3], dM[3], dN[3], dLx, dLy;
+  size_t hvol, mvol;
+  double inv_v;      // normalisation of the inverse
+};
+Status general_f32(const FastArgs& a, const GenShape& s, std::string* err);
+Status general_f64(const FastArgs& a, const GenShape& s, std::string* err);
+Status general_init_f32(std::string* err);
+Status general_init_f64(std::string* err);
+
 // Stages 0 and 5 (plane kernels) and stages 1-4 (z FFTs, gathers).
 Status fast_planes_f32(const FastArgs& a, std::string* err);
 Status fast_planes_f64(const FastArgs& a, std::string* err);

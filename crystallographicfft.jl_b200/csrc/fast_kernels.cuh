@@ -19,6 +19,7 @@
 
 #include "device_common.cuh"
 #include "fast_api.h"
+#include "launch.cuh"
 
 namespace cfft {
 namespace {
@@ -29,15 +30,6 @@ namespace {
 // twiddles in constant memory, so no runtime division or shared-memory pass remains
 // inside an FFT.  Shared-memory rows are padded to an odd stride (H + 1 complex) so
 // row and column accesses of a warp are bank-conflict free.
-
-// Programmatic dependent launch: wait until the previous kernel of the stream has
-// completed and its writes are visible (a no-op when the kernel was launched without
-// the attribute), then let the next kernel of the stream start launching.  Called first
-// in every kernel that launch_k starts, before any global memory access.
-__device__ __forceinline__ void pdl_enter() {
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-}
 
 // Drop one 128-byte L2 line without writing it back (its contents become undefined).
 // Used on channel-workspace lines that have been read for the last time, so the dirty
@@ -1964,42 +1956,6 @@ k_qsep_z(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__
 }
 
 constexpr int kMaxDynSmemFast = 227 * 1024;
-constexpr int kSMs = 148;  // B200: the unit of the launch-size rules
-
-// Programmatic dependent launch of the fast-path kernels (off with CFFT_PDL=0): each
-// kernel of a lane may launch while its predecessor in the stream is finishing, and
-// waits for it in hardware (griddepcontrol.wait, pdl_wait below) before touching memory.
-inline bool pdl_enabled() {
-  static const bool on = [] {
-    const char* e = std::getenv("CFFT_PDL");
-    return !(e && e[0] == '0');
-  }();
-  return on;
-}
-// First failure of a launch_k launch on this thread since fast_unit_launch last read it.
-inline cudaError_t& launch_error() {
-  static thread_local cudaError_t e = cudaSuccess;
-  return e;
-}
-template <typename... KArgs, typename... Args>
-inline void launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
-  if (pdl_enabled()) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
-    if (e != cudaSuccess && launch_error() == cudaSuccess) launch_error() = e;
-  } else {
-    k<<<grid, block, smem, st>>>(std::forward<Args>(args)...);
-  }
-}
 
 // Persistent bulk-copy plane kernels (tma_planes.cuh).  They serve centred plans with
 // H >= 16 whose per-group stage and buffer fit at least two groups into one CTA's
@@ -2102,12 +2058,6 @@ inline int zr_slots() {
     case 4: { constexpr int CTT = 4; __VA_ARGS__; } break;         \
     default: { constexpr int CTT = 0; __VA_ARGS__; } break;        \
   }
-
-inline Status fast_cuda(cudaError_t e, const char* what, std::string* err) {
-  if (e == cudaSuccess) return Status::kOk;
-  *err = std::string(what) + ": " + cudaGetErrorString(e);
-  return Status::kCuda;
-}
 
 // Cluster kernels: attributes, launch (cluster size at run time, through
 // cudaLaunchKernelEx) and occupancy, for the instantiations that fit.

@@ -75,3 +75,37 @@ def test_separable_step(cf, O, prep, sg, n, batch, precision):
     for b in range(batch):
         assert rel_err(q[b].cpu().numpy(), (b + 1) * want) < 2 * TOL[precision], b
     plan.close()
+
+
+@pytest.mark.parametrize("sg,N,batch,precision", [(47, (20, 24, 30), 3, 8), (47, (36, 50, 54), 2, 4), (47, (64, 32, 96), 1, 4),
+                                                  (191, (9, 9, 25), 5, 8), (191, (27, 27, 10), 2, 8), (191, (45, 45, 16), 2, 4),
+                                                  (229, (20, 20, 20), 9, 8), (229, (40, 40, 40), 4, 4), (225, (36, 36, 36), 17, 8),
+                                                  (230, (72, 72, 72), 1, 4), (227, (80, 80, 80), 3, 4), (166, (12, 12, 30), 2, 8),
+                                                  (123, (24, 24, 40), 2, 8), (221, (90, 90, 90), 1, 4), (62, (48, 20, 60), 33, 4)])
+def test_general_shapes(cf, O, prep, sg, N, batch, precision):
+    # radices 2 to 16 on every axis, one-factor and two-factor lengths, unequal axes, folds
+    check(cf, O, prep, sg, N, precision, batch)
+
+
+@pytest.mark.parametrize("sg,N,batch,precision", [(11, (30, 30), 1, 8), (11, (160, 160), 5, 8), (2, (18, 50), 3, 4), (17, (45, 45), 2, 8),
+                                                  (9, (64, 24), 7, 4)])
+def test_general_planes(cf, O, prep, sg, N, batch, precision):
+    check(cf, O, prep, sg, N, precision, batch)
+
+
+@pytest.mark.parametrize("sg,N,precision", [(229, (20, 20, 20), 8), (225, (30, 30, 30), 4), (47, (18, 10, 24), 8), (191, (9, 9, 5), 4)])
+def test_grid_conversion_shapes(cf, O, prep, sg, N, precision):
+    # whole grid -> subgrid -> whole grid of symmetric fields: copies, so equal to the bit
+    p, batch = prep(sg, N, seed=34), 6
+    plan = cf.KRFFTPlan(p["spec"], p["ops_s"], precision=precision, max_batch=batch)
+    u = torch.tensor(np.ascontiguousarray(np.stack([(b + 1) * p["u"].T for b in range(batch)])), device="cuda",
+                     dtype=torch.float32 if precision == 4 else torch.float64)
+    L = plan.L
+    f0 = plan.fullgrid_to_subgrid(u)
+    assert torch.equal(f0, u[:, ::L[2], ::L[1], ::L[0]])
+    back = plan.subgrid_to_fullgrid(f0)
+    assert torch.max(torch.abs(back - u)).item() <= 1e-5 * torch.max(torch.abs(u)).item()
+    assert torch.equal(back[:, ::L[2], ::L[1], ::L[0]], f0)
+    shifted = torch.empty(u.numel() + 1, dtype=u.dtype, device="cuda")[1:].view(u.shape)  # unaligned output
+    assert torch.equal(plan.subgrid_to_fullgrid(f0, out=shifted), back)
+    plan.close()
