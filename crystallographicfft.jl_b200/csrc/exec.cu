@@ -1243,11 +1243,15 @@ Status plan_device_init(Plan* p, std::string* err) {
   if (p->tune.chunk_bytes > 0) budget = static_cast<size_t>(p->tune.chunk_bytes);
   const size_t per_field = T.n_ch * hvol * cs / (tables ? 2 : 1);
   size_t ch = std::max<size_t>(1, std::min<size_t>(B, budget / std::max<size_t>(per_field, 1)));
-  // Batches of at least 8 fields on the fast path run as two concurrent lanes.
+  // Two concurrent lanes once the batch's channel workspace reaches 48 MiB: below, one lane
+  // fills the SMs and a second doubles the launches.  Measured with one / two lanes, us per
+  // round trip: Im-3m 128^3 FP32 32 fields (16 MiB) 59 / 61, 128 fields (64 MiB) 150 / 128;
+  // Pmmm 64^3 FP64 64 fields (16 MiB) 69 / 83, 256 fields (64 MiB) 246 / 218; P6/mmm 60 x 60 x 80
+  // FP64 16 fields (35 MiB) 122 / 123, 32 fields (70 MiB) 244 / 222.
   p->lanes = 1;
   if (p->tune.lanes > 0) p->lanes = std::min(Plan::kMaxLanes, p->tune.lanes);
   else if (const char* ln = std::getenv("CFFT_LANES")) p->lanes = std::max(1, std::min(Plan::kMaxLanes, std::atoi(ln)));
-  else if (tables && B >= 8) p->lanes = 2;
+  else if (tables && B >= 8 && B * per_field >= (static_cast<size_t>(48) << 20)) p->lanes = 2;
   if (p->lanes > 1) ch = std::min(ch, (B + p->lanes - 1) / p->lanes);
   if (tables && ch < B && ch > 1) ch &= ~static_cast<size_t>(1);
   p->chunk = static_cast<int>(ch);
