@@ -18,6 +18,7 @@ Array conventions
 from __future__ import annotations
 
 import ctypes
+import functools
 from dataclasses import dataclass
 
 import numpy as np
@@ -28,8 +29,10 @@ from ._lib import LIB, CFFTDesc, CFFTError, CFFTInfo, CFFTTuning, check
 PATH_AUTO, PATH_M2, PATH_CENTERED, PATH_M2Q, PATH_M7, PATH_FULLGRID = 0, 1, 2, 3, 4, 5
 _REAL = {4: np.float32, 8: np.float64}
 _CPLX = {4: np.complex64, 8: np.complex128}
+_TENSOR = {}  # (kind, precision) -> torch dtype, filled on first use
 
 
+@functools.lru_cache(maxsize=None)
 def _torch():
     import torch  # device buffers and streams only
 
@@ -95,6 +98,7 @@ class KRFFTPlan:
         self.M = tuple(info.M[i] for i in range(dim))
         self.H = tuple(info.H[i] for i in range(dim))
         self.n_spec = info.n_spec
+        self.mvol = int(np.prod(self.M))
         self.centered = bool(info.centered)
         self.centering = sym.CENTERING_NAMES[info.centering]
         self.n_channels = info.n_channels
@@ -116,10 +120,6 @@ class KRFFTPlan:
     @property
     def handle(self):
         return self._h
-
-    @property
-    def mvol(self) -> int:
-        return int(np.prod(self.M))
 
     # -- tables ---------------------------------------------------------------
     def q_tables(self):
@@ -196,8 +196,7 @@ class KRFFTPlan:
 
     @staticmethod
     def _stream():
-        torch = _torch()
-        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _torch().cuda.current_stream().cuda_stream
 
     def _new_field_tensor(self, B, like):
         torch = _torch()
@@ -211,11 +210,13 @@ class KRFFTPlan:
         return torch.empty((B, self.n_spec) if B > 1 else (self.n_spec,), dtype=dt, device=like.device)
 
     def _check_tensor(self, x, kind):
-        torch = _torch()
         if not x.is_cuda or not x.is_contiguous():
             raise CFFTError(1, "tensors must be contiguous CUDA tensors")
-        want = {("r", 4): torch.float32, ("r", 8): torch.float64, ("c", 4): torch.complex64, ("c", 8): torch.complex128}
-        if x.dtype != want[(kind, self.precision)]:
+        if not _TENSOR:
+            torch = _torch()
+            _TENSOR.update({("r", 4): torch.float32, ("r", 8): torch.float64, ("c", 4): torch.complex64,
+                            ("c", 8): torch.complex128})
+        if x.dtype != _TENSOR[kind, self.precision]:
             raise CFFTError(1, f"tensor dtype {x.dtype} does not match plan precision {self.precision}")
 
     # -- execution ------------------------------------------------------------
@@ -226,7 +227,7 @@ class KRFFTPlan:
             B = self._batch_of(f0, self.mvol)
             F = self._new_spec_tensor(B, f0) if out is None else out
             self._check_tensor(F, "c")
-            check(LIB.cfft_forward(self._h, ctypes.c_void_p(f0.data_ptr()), ctypes.c_void_p(F.data_ptr()), B, self._stream()))
+            check(LIB.cfft_forward(self._h, f0.data_ptr(), F.data_ptr(), B, self._stream()))
             return F
         flat, B, batched = self._field_host(f0)
         F = np.empty((B, self.n_spec), dtype=_CPLX[self.precision])
@@ -240,7 +241,7 @@ class KRFFTPlan:
             B = self._batch_of(F, self.n_spec)
             f0 = self._new_field_tensor(B, F) if out is None else out
             self._check_tensor(f0, "r")
-            check(LIB.cfft_backward(self._h, ctypes.c_void_p(F.data_ptr()), ctypes.c_void_p(f0.data_ptr()), B, self._stream()))
+            check(LIB.cfft_backward(self._h, F.data_ptr(), f0.data_ptr(), B, self._stream()))
             return f0
         Fa = np.ascontiguousarray(np.asarray(F, dtype=_CPLX[self.precision]))
         batched = Fa.ndim == 2
@@ -256,7 +257,7 @@ class KRFFTPlan:
         if _is_tensor(f0):
             self._check_tensor(f0, "r")
             B = self._batch_of(f0, self.mvol)
-            check(LIB.cfft_scft_step(self._h, ctypes.c_void_p(f0.data_ptr()), B, self._stream()))
+            check(LIB.cfft_scft_step(self._h, f0.data_ptr(), B, self._stream()))
             return f0
         flat, B, batched = self._field_host(f0)
         check(LIB.cfft_scft_step_host(self._h, flat.ctypes.data_as(ctypes.c_void_p), B))
@@ -271,7 +272,7 @@ class KRFFTPlan:
         B = self._batch_of(q, self.mvol)
         if w.numel() != q.numel():
             raise CFFTError(1, "w must have the layout of q")
-        check(LIB.cfft_step_diffusion(self._h, ctypes.c_void_p(q.data_ptr()), ctypes.c_void_p(w.data_ptr()),
+        check(LIB.cfft_step_diffusion(self._h, q.data_ptr(), w.data_ptr(),
                                       float(dt), int(n_steps), B, self._stream()))
         return q
 
@@ -281,7 +282,7 @@ class KRFFTPlan:
         nvol = int(np.prod(self.N))
         B = self._batch_of(u, nvol)
         f0 = self._new_field_tensor(B, u) if out is None else out
-        check(LIB.cfft_fullgrid_to_subgrid(self._h, ctypes.c_void_p(u.data_ptr()), ctypes.c_void_p(f0.data_ptr()), B, self._stream()))
+        check(LIB.cfft_fullgrid_to_subgrid(self._h, u.data_ptr(), f0.data_ptr(), B, self._stream()))
         return f0
 
     def subgrid_spectrum(self, f0, out=None):
@@ -294,7 +295,7 @@ class KRFFTPlan:
         shape = tuple(reversed(self.M))
         G0 = torch.empty(((B,) + shape) if B > 1 else shape, dtype=cdt, device=f0.device) if out is None else out
         self._check_tensor(G0, "c")
-        check(LIB.cfft_subgrid_spectrum(self._h, ctypes.c_void_p(f0.data_ptr()), ctypes.c_void_p(G0.data_ptr()), B,
+        check(LIB.cfft_subgrid_spectrum(self._h, f0.data_ptr(), G0.data_ptr(), B,
                                         self._stream()))
         return G0
 
@@ -305,7 +306,7 @@ class KRFFTPlan:
         B = self._batch_of(f0, self.mvol)
         shape = tuple(reversed(self.N))
         u = torch.empty(((B,) + shape) if B > 1 else shape, dtype=f0.dtype, device=f0.device) if out is None else out
-        check(LIB.cfft_subgrid_to_fullgrid(self._h, ctypes.c_void_p(f0.data_ptr()), ctypes.c_void_p(u.data_ptr()), B, self._stream()))
+        check(LIB.cfft_subgrid_to_fullgrid(self._h, f0.data_ptr(), u.data_ptr(), B, self._stream()))
         return u
 
 
