@@ -210,6 +210,17 @@ template <> __device__ __forceinline__ void vload<double>(double* out, const dou
   const double2 v = *reinterpret_cast<const double2*>(p);
   out[0] = v.x; out[1] = v.y;
 }
+// The same through the read-only path (data no thread of the kernel writes), so that the
+// compiler may issue the loads ahead of stores.
+template <typename T> __device__ __forceinline__ void vload_nc(T* out, const T* p);
+template <> __device__ __forceinline__ void vload_nc<float>(float* out, const float* p) {
+  const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+  out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
+}
+template <> __device__ __forceinline__ void vload_nc<double>(double* out, const double* p) {
+  const double2 v = __ldg(reinterpret_cast<const double2*>(p));
+  out[0] = v.x; out[1] = v.y;
+}
 template <typename T> __device__ __forceinline__ void vstore(T* p, const T* in);
 template <> __device__ __forceinline__ void vstore<float>(float* p, const float* in) {
   *reinterpret_cast<float4*>(p) = make_float4(in[0], in[1], in[2], in[3]);

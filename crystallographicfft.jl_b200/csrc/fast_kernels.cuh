@@ -238,26 +238,31 @@ __device__ __forceinline__ void fold_plane(const DevGeom* __restrict__ g, const 
       for (int e = tid; e < H * H / VW; e += nth) {
         int ix0, iy;
         fold_item<H, VW>(e, &ix0, &iy);
+        // All sixteen field loads first (field a stands in for a missing b), then the factors:
+        // interleaved, every octant's product waits for its own loads before the next
+        // octant's are issued.
         T va[8][VW], vb[8][VW];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const int idx = ((iz + ((k >> 2) & 1) * H) * M + iy + ((k >> 1) & 1) * H) * M + ix0 + (k & 1) * H;
           vload_stream<T>(va[k], srca + idx);
-          if (has_b) vload_stream<T>(vb[k], srcb + idx);
-          else {
+          vload_stream<T>(vb[k], (has_b ? srcb : srca) + idx);
+        }
+        if (!has_b) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
 #pragma unroll
             for (int l = 0; l < VW; ++l) vb[k][l] = zero;
-          }
-          if (USE_E) {
-            T ea[VW];
-            vload<T>(ea, Ea + idx);
+        }
+        if (USE_E) {
 #pragma unroll
-            for (int l = 0; l < VW; ++l) va[k][l] *= ea[l];
-            if (has_b) {
-              vload<T>(ea, Eb + idx);
+          for (int k = 0; k < 8; ++k) {
+            const int idx = ((iz + ((k >> 2) & 1) * H) * M + iy + ((k >> 1) & 1) * H) * M + ix0 + (k & 1) * H;
+            T ea[VW], eb[VW];
+            vload_nc<T>(ea, Ea + idx);
+            vload_nc<T>(eb, (has_b ? Eb : Ea) + idx);
 #pragma unroll
-              for (int l = 0; l < VW; ++l) vb[k][l] *= ea[l];
-            }
+            for (int l = 0; l < VW; ++l) { va[k][l] *= ea[l]; vb[k][l] *= eb[l]; }
           }
         }
         fold_emit<T, H, CT, VW, PV>(va, vb, ix0, iy, ftx, ftz, buf);
@@ -366,15 +371,11 @@ __device__ __forceinline__ void unfold_plane(const DevGeom* __restrict__ g, cons
         for (int k = 0; k < 8; ++k) {
           const int idx = ((iz + ((k >> 2) & 1) * H) * M + iy + ((k >> 1) & 1) * H) * M + ix0 + (k & 1) * H;
           if (USE_E) {
-            T ea[VW];
-            vload<T>(ea, Ea + idx);
+            T ea[VW], eb[VW];
+            vload_nc<T>(ea, Ea + idx);
+            vload_nc<T>(eb, (has_b ? Eb : Ea) + idx);
 #pragma unroll
-            for (int l = 0; l < VW; ++l) oa[k][l] *= ea[l];
-            if (has_b) {
-              vload<T>(ea, Eb + idx);
-#pragma unroll
-              for (int l = 0; l < VW; ++l) ob[k][l] *= ea[l];
-            }
+            for (int l = 0; l < VW; ++l) { oa[k][l] *= ea[l]; ob[k][l] *= eb[l]; }
           }
           vstore_stream<T>(dsta + idx, oa[k]);
           if (has_b) vstore_stream<T>(dstb + idx, ob[k]);
@@ -622,11 +623,11 @@ template <typename T, int VW> __device__ __forceinline__ void vw_load_stream(T (
 }
 template <typename T, int VW> __device__ __forceinline__ void vw_load(T (&o)[VW], const T* p) {
   if constexpr (VW == 2 && sizeof(T) == 4) {
-    const float2 v = *reinterpret_cast<const float2*>(p);
+    const float2 v = __ldg(reinterpret_cast<const float2*>(p));
     o[0] = v.x; o[1] = v.y;
   } else {
 #pragma unroll
-    for (int l = 0; l < VW; ++l) o[l] = p[l];
+    for (int l = 0; l < VW; ++l) o[l] = __ldg(p + l);
   }
 }
 template <typename T, int VW> __device__ __forceinline__ void vw_store_stream(T* p, const T (&o)[VW]) {
@@ -681,23 +682,23 @@ __device__ __forceinline__ void fold_rows(const DevGeom* __restrict__ g, const t
       for (int k = 0; k < 8; ++k) {
         const int idx = ((iz + ((k >> 2) & 1) * H) * M + iy + ((k >> 1) & 1) * H) * M + ix0 + (k & 1) * H;
         vw_load_stream<T, VW>(va[k], srca + idx);
+        vw_load_stream<T, VW>(vb[k], (has_b ? srcb : srca) + idx);
+      }
+      if (!has_b) {
 #pragma unroll
-        for (int l = 0; l < VW; ++l) vb[k][l] = zero;
-        if (has_b) vw_load_stream<T, VW>(vb[k], srcb + idx);
+        for (int k = 0; k < 8; ++k)
+#pragma unroll
+          for (int l = 0; l < VW; ++l) vb[k][l] = zero;
       }
       if (USE_E) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const int idx = ((iz + ((k >> 2) & 1) * H) * M + iy + ((k >> 1) & 1) * H) * M + ix0 + (k & 1) * H;
-          T ea[VW];
+          T ea[VW], eb[VW];
           vw_load<T, VW>(ea, Ea + idx);
+          vw_load<T, VW>(eb, (has_b ? Eb : Ea) + idx);
 #pragma unroll
-          for (int l = 0; l < VW; ++l) va[k][l] *= ea[l];
-          if (has_b) {
-            vw_load<T, VW>(ea, Eb + idx);
-#pragma unroll
-            for (int l = 0; l < VW; ++l) vb[k][l] *= ea[l];
-          }
+          for (int l = 0; l < VW; ++l) { va[k][l] *= ea[l]; vb[k][l] *= eb[l]; }
         }
       }
       fold_emit<T, H, CT, VW>(va, vb, ix0, iy, ftx, ftz, buf);
@@ -776,15 +777,11 @@ __device__ __forceinline__ void unfold_rows(const DevGeom* __restrict__ g, const
       for (int k = 0; k < 8; ++k) {
         const int idx = ((iz + ((k >> 2) & 1) * H) * M + iy + ((k >> 1) & 1) * H) * M + ix0 + (k & 1) * H;
         if (USE_E) {
-          T ea[VW];
+          T ea[VW], eb[VW];
           vw_load<T, VW>(ea, Ea + idx);
+          vw_load<T, VW>(eb, (has_b ? Eb : Ea) + idx);
 #pragma unroll
-          for (int l = 0; l < VW; ++l) oa[k][l] *= ea[l];
-          if (has_b) {
-            vw_load<T, VW>(ea, Eb + idx);
-#pragma unroll
-            for (int l = 0; l < VW; ++l) ob[k][l] *= ea[l];
-          }
+          for (int l = 0; l < VW; ++l) { oa[k][l] *= ea[l]; ob[k][l] *= eb[l]; }
         }
         vw_store_stream<T, VW>(dsta + idx, oa[k]);
         if (has_b) vw_store_stream<T, VW>(dstb + idx, ob[k]);

@@ -173,7 +173,7 @@ k_gplane_fwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
 #pragma unroll
         for (int k = 0; k < U; ++k) {
           const int e = e0 + k * blockDim.x, idx = iz * plane + e;
-          if (e < plane) v[k] = mk<C>(v[k].x * Ea[idx], has_b ? v[k].y * Eb[idx] : zero);
+          if (e < plane) v[k] = mk<C>(v[k].x * __ldg(Ea + idx), has_b ? v[k].y * __ldg(Eb + idx) : zero);
         }
       }
 #pragma unroll
@@ -197,7 +197,7 @@ k_gplane_fwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const int idx = ((iz + ((k >> 2) & 1) * H2) * M1 + iy + ((k >> 1) & 1) * H1) * M0 + ix + (k & 1) * H0;
-          p[k] = mk<C>(p[k].x * Ea[idx], has_b ? p[k].y * Eb[idx] : zero);
+          p[k] = mk<C>(p[k].x * __ldg(Ea + idx), has_b ? p[k].y * __ldg(Eb + idx) : zero);
         }
       }
       wht8c(p);
@@ -307,7 +307,7 @@ k_gplane_bwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
   const T hi = static_cast<T>(s.inv_v), lo = static_cast<T>(s.inv_v - static_cast<double>(hi));
   auto put = [&](int idx, C v) {
     T a = fma(v.x, hi, v.x * lo), b = fma(v.y, hi, v.y * lo);
-    if (E) { a *= Ea[idx]; if (has_b) b *= Eb[idx]; }
+    if (E) { a *= __ldg(Ea + idx); if (has_b) b *= __ldg(Eb + idx); }
     __stcs(dsta + idx, a);
     if (has_b) __stcs(dstb + idx, b);
   };
