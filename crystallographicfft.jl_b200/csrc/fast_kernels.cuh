@@ -810,7 +810,6 @@ template <typename T, int H, int CT>
 __global__ void __launch_bounds__(split_threads<H, CT>(), split_blocks<T, H, CT>())
 k_plane_fwd_s(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
               const T* __restrict__ f0, const T* __restrict__ E, typename Cx<T>::type* __restrict__ W, int nfields) {
-  pdl_enter();
   using C = typename Cx<T>::type;
   constexpr int nch = Cent<CT>::n, S = H + 1, PL = H * S, A = split_a<H>(), B = split_b<H>(), HV = H * H * H;
   constexpr int VW = H % fold_width<T>() == 0 ? fold_width<T>() : 1;
@@ -818,6 +817,7 @@ k_plane_fwd_s(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restr
   C* buf = reinterpret_cast<C*>(smem_raw);
   C* tw = buf + nch * PL;
   load_line_twiddles<C, H>(g, tables, tw);
+  pdl_enter();
   const int iz = blockIdx.x, slot = blockIdx.y;
   const int fa = 2 * slot;
   const bool has_b = fa + 1 < nfields;
@@ -867,7 +867,6 @@ template <typename T, int H, int CT>
 __global__ void __launch_bounds__(split_threads<H, CT>(), split_blocks<T, H, CT>())
 k_plane_bwd_s(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
               const typename Cx<T>::type* __restrict__ W, const T* __restrict__ E, T* __restrict__ f0, int nfields) {
-  pdl_enter();
   using C = typename Cx<T>::type;
   constexpr int nch = Cent<CT>::n, S = H + 1, PL = H * S, A = split_a<H>(), B = split_b<H>(), HV = H * H * H;
   constexpr int VW = H % fold_width<T>() == 0 ? fold_width<T>() : 1;
@@ -875,6 +874,7 @@ k_plane_bwd_s(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restr
   C* buf = reinterpret_cast<C*>(smem_raw);
   C* tw = buf + nch * PL;
   load_line_twiddles<C, H>(g, tables, tw);
+  pdl_enter();
   const int iz = blockIdx.x, slot = blockIdx.y;
   const int fa = 2 * slot;
   const bool has_b = fa + 1 < nfields;
@@ -1349,7 +1349,6 @@ k_fft_z_recon_diag8(const DevGeom* __restrict__ g, const typename Cx<T>::type* _
                     const T* __restrict__ K, const uint4* __restrict__ units, const uint2* __restrict__ pts,
                     const typename Cx<T>::type* __restrict__ pq, int npts,
                     const typename Cx<T>::type* __restrict__ W, typename Cx<T>::type* __restrict__ F, int nfields) {
-  pdl_enter();
   using C = typename Cx<T>::type;
   constexpr int S = H + 1, HV = H * H * H, NTH = zr_threads<H, SL, SPLIT>(), NL = SL * 2 * H;
   constexpr int RS = H * S;  // one row of (x, z) lines
@@ -1362,6 +1361,23 @@ k_fft_z_recon_diag8(const DevGeom* __restrict__ g, const typename Cx<T>::type* _
   const int slot0 = blockIdx.y * SL;
   const int nslots = (nfields + 1) / 2;
   const int nch = g->n_ch;
+  C* tw = buf + SL * 2 * RS;
+  if constexpr (SPLIT) load_line_twiddles<C, H>(g, tables, tw);
+  // The first round of points and weights does not depend on the previous kernel either.
+  auto load_point = [&](int i, uint2* pt, C (&Pw)[4], C (&Qw)[4]) {
+    *pt = __ldg(pts + un.y + i);
+#pragma unroll
+    for (int sg = 0; sg < 4; ++sg) {
+      const C* p = pq + static_cast<size_t>(2 * sg) * npts + un.y + i;
+      Pw[sg] = __ldg(p);
+      Qw[sg] = __ldg(p + npts);
+    }
+  };
+  constexpr bool EARLY = SL == 1;
+  uint2 pt0 = make_uint2(0u, 0u);
+  C P0[4], Q0[4];
+  if (EARLY && tid < static_cast<int>(un.z)) load_point(tid, &pt0, P0, Q0);
+  pdl_enter();
   if constexpr (!SPLIT) {
     if (tid < NL) {
       const int k = tid / (2 * H), r = (tid / H) & 1, x = tid % H;
@@ -1380,8 +1396,6 @@ k_fft_z_recon_diag8(const DevGeom* __restrict__ g, const typename Cx<T>::type* _
     }
   } else {
     constexpr int A = split_a<H>(), B = split_b<H>();
-    C* tw = buf + SL * 2 * RS;
-    load_line_twiddles<C, H>(g, tables, tw);
     if constexpr (B > 1) __syncthreads();
     for (int i = tid; i < NL * B; i += NTH) {
       const int l = i % NL, j = i / NL;
@@ -1444,13 +1458,14 @@ k_fft_z_recon_diag8(const DevGeom* __restrict__ g, const typename Cx<T>::type* _
   const int ns = g->n_spec;
   const int nvalid = min(SL, nslots - slot0);
   for (int i = tid; i < static_cast<int>(un.z); i += NTH) {
-    const uint2 pt = __ldg(pts + un.y + i);
+    uint2 pt;
     C Pw[4], Qw[4];
+    if (EARLY && i == tid) {
+      pt = pt0;
 #pragma unroll
-    for (int sg = 0; sg < 4; ++sg) {
-      const C* p = pq + static_cast<size_t>(2 * sg) * npts + un.y + i;
-      Pw[sg] = __ldg(p);
-      Qw[sg] = __ldg(p + npts);
+      for (int sg = 0; sg < 4; ++sg) { Pw[sg] = P0[sg]; Qw[sg] = Q0[sg]; }
+    } else {
+      load_point(i, &pt, Pw, Qw);
     }
     const uint32_t sidx = pt.x, hp = pt.y;
     const int h0 = static_cast<int>(hp & 1023u), h1 = static_cast<int>((hp >> 10) & 1023u), h2 = static_cast<int>((hp >> 20) & 1023u);
@@ -1567,12 +1582,23 @@ __global__ void __launch_bounds__(kFibers * L)
 k_inv_fiber(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
             const uint2* __restrict__ taps, const uint2* __restrict__ outs, int nf,
             const typename Cx<T>::type* __restrict__ F, typename Cx<T>::type* __restrict__ G0P, int nb) {
-  pdl_enter();
   using C = typename Cx<T>::type;
   constexpr int RS = L + 1;
   __shared__ C tile[D * kFibers * RS];
   const int lane = threadIdx.x % kFibers, j = threadIdx.x / kFibers;
   const int f0 = blockIdx.x * kFibers, f = f0 + lane;
+  // Rows of two slots are small launches that wait on the previous kernel: their table loads
+  // go before the wait.  Full rows would pay for the registers (Ia-3d 96^3 contour steps of 256
+  // fields: 3339 us with it, 3235 without).
+  constexpr bool EARLY = L == 2;
+  uint2 t[D], o[D];
+  if constexpr (!EARLY) pdl_enter();
+#pragma unroll
+  for (int m = 0; m < D; ++m) {
+    t[m] = f < nf ? __ldg(taps + static_cast<size_t>(m) * nf + f) : make_uint2(0u, 0u);
+    if (EARLY) o[m] = f < nf ? __ldg(outs + static_cast<size_t>(m) * nf + f) : make_uint2(0u, 0u);
+  }
+  if constexpr (EARLY) pdl_enter();
   const int gq = blockIdx.y;
   const int fa = 2 * (gq * L + j);
   const C* ph = tables + g->ph_off;
@@ -1582,10 +1608,7 @@ k_inv_fiber(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restric
   if (f < nf && fa < nb) {
     const C* Fa = F + static_cast<size_t>(fa) * ns;
     const bool has_b = fa + 1 < nb;
-    uint2 t[D];
     C va[D], vb[D];
-#pragma unroll
-    for (int m = 0; m < D; ++m) t[m] = __ldg(taps + static_cast<size_t>(m) * nf + f);
 #pragma unroll
     for (int m = 0; m < D; ++m) {
       const uint32_t sp = t[m].x & 0x7FFFFFFFu;
@@ -1607,8 +1630,8 @@ k_inv_fiber(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restric
     const T inv_d = static_cast<T>(1.0 / static_cast<double>(D));
 #pragma unroll
     for (int b = 0; b < D; ++b) {
-      const uint2 o = __ldg(outs + static_cast<size_t>(b) * nf + f);
-      if (o.x) tile[(b * kFibers + lane) * RS + j] = cscale(cmulc(x[b], ph[o.y]), inv_d);
+      if (!EARLY) o[b] = __ldg(outs + static_cast<size_t>(b) * nf + f);
+      if (o[b].x) tile[(b * kFibers + lane) * RS + j] = cscale(cmulc(x[b], ph[o[b].y]), inv_d);
     }
   }
   __syncthreads();
@@ -1619,8 +1642,8 @@ k_inv_fiber(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restric
   for (int e = threadIdx.x; e < D * kFibers * L; e += kFibers * L) {
     const int k = e % L, fb = (e / L) % kFibers, b = e / (L * kFibers);
     if (fb < cnt) {
-      const uint32_t o = __ldg(outs + static_cast<size_t>(b) * nf + f0 + fb).x;
-      if (o) dst[static_cast<size_t>(o - 1) * L + k] = tile[(b * kFibers + fb) * RS + k];
+      const uint32_t at = __ldg(outs + static_cast<size_t>(b) * nf + f0 + fb).x;
+      if (at) dst[static_cast<size_t>(at - 1) * L + k] = tile[(b * kFibers + fb) * RS + k];
     }
   }
 }
@@ -1701,26 +1724,36 @@ __global__ void __launch_bounds__(expand_threads<typename Cx<T>::type, H, LS>())
 k_expand_ifft_z(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
                 const uint32_t* __restrict__ ETP, const typename Cx<T>::type* __restrict__ G0P,
                 typename Cx<T>::type* __restrict__ W, int nfields) {
-  pdl_enter();
   using C = typename Cx<T>::type;
   constexpr int HV = H * H * H, PS = expand_plane<H>(), NTH = expand_threads<C, H, LS>();
   constexpr int SPV = 16 / static_cast<int>(sizeof(C)), NP = LS / SPV;  // slots per 16 bytes, pieces per row
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);  // [slot][z][x]
   C* tw = buf + LS * PS;
-  if constexpr (SPLIT) load_line_twiddles<C, H>(g, tables, tw);
   const int y = blockIdx.x, c = blockIdx.y, gq = blockIdx.z / (L / LS), part = blockIdx.z % (L / LS);
   const int slot0 = gq * L + part * LS;
-  if (2 * slot0 >= nfields) return;
+  if (2 * slot0 >= nfields) {
+    pdl_enter();
+    return;
+  }
   const uint32_t* et = ETP + static_cast<size_t>(c) * HV + y * H;
   const C* rp = G0P + static_cast<size_t>(gq) * g->n_orbits * L + part * LS;
   const C* ph = tables + g->ph_off;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < H * H * NP; i += NTH) {
+  // Entries and phases of a short loop are fetched before the previous kernel has finished.
+  constexpr int ITEMS = H * H * NP, ROUNDS = (ITEMS + NTH - 1) / NTH, AHEAD = ROUNDS <= 6 ? ROUNDS : 0;
+  if constexpr (SPLIT) load_line_twiddles<C, H>(g, tables, tw);
+  uint32_t te[AHEAD > 0 ? AHEAD : 1];
+  C we[AHEAD > 0 ? AHEAD : 1];
+#pragma unroll
+  for (int k = 0; k < AHEAD; ++k) {
+    const int i = min(static_cast<int>(threadIdx.x) + k * NTH, ITEMS - 1);
+    te[k] = __ldg(et + i / (NP * H) * H * H + (i / NP) % H);
+    we[k] = __ldg(ph + (te[k] >> 21));
+  }
+  pdl_enter();
+  auto put = [&](int i, uint32_t t, C w) {
     const int p = i % NP, x = (i / NP) % H, z = i / (NP * H);
-    const uint32_t t = __ldg(et + z * H * H + x);
     const C* src = rp + static_cast<size_t>(L) * (t & 0x1FFFFFu) + p * SPV;
-    const C w = ph[t >> 21];
     C* d = buf + (p * SPV) * PS + z * H + x;
     if constexpr (SPV == 2) {
       const float4 u = __ldg(reinterpret_cast<const float4*>(src));
@@ -1728,6 +1761,19 @@ k_expand_ifft_z(const DevGeom* __restrict__ g, const typename Cx<T>::type* __res
       d[PS] = cmulc(mk<C>(u.z, u.w), w);
     } else {
       d[0] = cmulc(__ldg(src), w);
+    }
+  };
+  if constexpr (AHEAD > 0) {
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) {
+      const int i = threadIdx.x + k * NTH;
+      if (ITEMS % NTH == 0 || i < ITEMS) put(i, te[k], we[k]);
+    }
+  } else {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < ITEMS; i += NTH) {
+      const uint32_t t = __ldg(et + i / (NP * H) * H * H + (i / NP) % H);
+      put(i, t, ph[t >> 21]);
     }
   }
   __syncthreads();
@@ -1779,13 +1825,13 @@ __global__ void __launch_bounds__(expand_threads<typename Cx<T>::type, H, 2>())
 k_qmul_ifft_z_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
                 const typename Cx<T>::type* __restrict__ QT, const int32_t* __restrict__ GT,
                 const typename Cx<T>::type* __restrict__ WT, typename Cx<T>::type* __restrict__ W2) {
-  pdl_enter();
   using C = typename Cx<T>::type;
   constexpr int HV = H * H * H;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);  // [z][x]
   C* tw = buf + expand_plane<H>();
   load_line_twiddles<C, H>(g, tables, tw);
+  pdl_enter();
   const int y = blockIdx.x, c = blockIdx.y, slot = blockIdx.z;
   const int d = g->d;
   const size_t np = static_cast<size_t>(g->n_ch) * HV;
@@ -1829,13 +1875,13 @@ template <typename T, int H>
 __global__ void __launch_bounds__(kSepThreads)
 k_qsep_z(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
          const typename Cx<T>::type* __restrict__ QS, typename Cx<T>::type* __restrict__ W, int PP) {
-  pdl_enter();
   using C = typename Cx<T>::type;
   constexpr int HV = H * H * H, S = H + 1, A = split_a<H>(), B = split_b<H>(), HP = H / 2 + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);  // [row][side][pair][z]
   C* tw = buf + 4 * PP * S;
   load_line_twiddles<C, H>(g, tables, tw);
+  pdl_enter();
   const int y = blockIdx.x, ym = y ? H - y : 0, rows = ym == y ? 1 : 2;
   const int p0 = blockIdx.y * PP, np = min(PP, HP - p0), slot = blockIdx.z;
   const int lines = rows * 2 * np;

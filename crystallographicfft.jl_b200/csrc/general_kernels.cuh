@@ -138,7 +138,6 @@ template <typename T>
 __global__ void __launch_bounds__(kGenThreads, sizeof(T) == 4 ? 2 : 1)
 k_gplane_fwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, const T* __restrict__ f0,
              const T* __restrict__ E, typename Cx<T>::type* __restrict__ W, int nfields) {
-  pdl_enter();
   using C = typename Cx<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
@@ -147,6 +146,7 @@ k_gplane_fwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
   C* tw1 = tw0 + H0;
   copy_twiddles(tw0, tables + s.tw[0], H0);
   copy_twiddles(tw1, tables + s.tw[1], H1);
+  pdl_enter();
   const int iz = blockIdx.x, slot = blockIdx.y, fa = 2 * slot;
   const bool has_b = fa + 1 < nfields;
   const T zero = static_cast<T>(0);
@@ -260,7 +260,6 @@ __global__ void __launch_bounds__(kGenThreads, sizeof(T) == 4 ? 2 : 1)
 k_gplane_bwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, const typename Cx<T>::type* __restrict__ W,
              const uint32_t* __restrict__ ETP, const typename Cx<T>::type* __restrict__ G0P, const T* __restrict__ E,
              T* __restrict__ f0, int nfields) {
-  pdl_enter();
   using C = typename Cx<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
@@ -269,6 +268,7 @@ k_gplane_bwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
   C* tw1 = tw0 + H0;
   copy_twiddles(tw0, tables + s.tw[0], H0);
   copy_twiddles(tw1, tables + s.tw[1], H1);
+  pdl_enter();
   const int iz = blockIdx.x, slot = blockIdx.y, fa = 2 * slot;
   const bool has_b = fa + 1 < nfields;
   const int A0 = s.A[0], B0 = s.B[0], A1 = s.A[1], B1 = s.B[1];
@@ -349,13 +349,13 @@ template <typename T, bool INV>
 __global__ void __launch_bounds__(kGenThreads, sizeof(T) == 4 ? 2 : 1)
 k_gline_z(const GenShape s, const typename Cx<T>::type* __restrict__ tables, const uint32_t* __restrict__ ETP,
           const typename Cx<T>::type* __restrict__ G0P, typename Cx<T>::type* __restrict__ W) {
-  pdl_enter();
   using C = typename Cx<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);  // [z position][x]
   const int H0 = s.H[0], A = s.A[2], B = s.B[2];
   C* tw = buf + H0 * s.H[2];
   copy_twiddles(tw, tables + s.tw[2], s.H[2]);
+  pdl_enter();
   const int y = blockIdx.x, c = blockIdx.y, slot = blockIdx.z;
   const size_t plane = static_cast<size_t>(H0) * s.H[1];
   const size_t at = static_cast<size_t>(c) * s.hvol + static_cast<size_t>(y) * H0;
@@ -386,7 +386,6 @@ __global__ void __launch_bounds__(128)
 k_grecon(const GenShape s, const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
          const uint32_t* __restrict__ spec_h, const T* __restrict__ K, const typename Cx<T>::type* __restrict__ W,
          typename Cx<T>::type* __restrict__ F, int nfields) {
-  pdl_enter();
   using C = typename Cx<T>::type;
   __shared__ int sR[8][9], sT[8][3];
   const int D = s.d;
@@ -397,8 +396,9 @@ k_grecon(const GenShape s, const DevGeom* __restrict__ g, const typename Cx<T>::
   }
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x, slot = blockIdx.y, fa = 2 * slot;
+  const uint32_t hp = __ldg(spec_h + min(i, s.n_spec - 1));
+  pdl_enter();
   if (i >= s.n_spec) return;
-  const uint32_t hp = spec_h[i];
   const int h[3] = {static_cast<int>(hp & 1023u), static_cast<int>((hp >> 10) & 1023u), static_cast<int>((hp >> 20) & 1023u)};
   const C* Wb = W + static_cast<size_t>(slot) * s.nch * s.hvol;
   const int sh = s.centered ? 1 : 0;

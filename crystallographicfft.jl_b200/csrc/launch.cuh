@@ -15,8 +15,10 @@ namespace {
 
 // Programmatic dependent launch: wait until the previous kernel of the stream has
 // completed and its writes are visible (a no-op when the kernel was launched without
-// the attribute), then let the next kernel of the stream start launching.  Called first
-// in every kernel that launch_k starts, before any global memory access.
+// the attribute), then let the next kernel of the stream start launching.  Called in
+// every kernel that launch_k starts, before any access to memory that a kernel writes.
+// Loads of the plan's constant tables may come before it: they are then in flight while the
+// previous kernel finishes.
 __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
