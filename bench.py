@@ -62,7 +62,7 @@ def load_package():
 # warm-start network, the space-group table and the C ABI wrappers do not change it.
 TRANSFORM_SOURCES = ("cfft_internal.h", "device_common.cuh", "exec.cu", "exec.h", "fast_api.h", "fast_kernels.cuh",
                      "fast_other_f32.cu", "fast_other_f64.cu", "fast_planes_f32.cu", "fast_planes_f64.cu",
-                     "tma_planes.cuh")
+                     "general_f32.cu", "general_f64.cu", "general_kernels.cuh", "launch.cuh", "tma_planes.cuh")
 
 
 def kernel_source_sha():
@@ -491,7 +491,7 @@ def run_ours(args):
     alg = algorithmic_bytes_per_field(M, plan.n_spec) * B
     achieved = alg / (ms_step * 1e-3) / 1e9
     names = ["plane_fwd (fold+xy FFT)", "z FFT fwd (+ spectral gather when fused)", "spectral gather (separate kernel)",
-             "regroup + inverse gather", "expansion + inverse z FFT", "plane_bwd (xy IFFT+unfold)"]
+             "inverse gather by fibers", "expansion + inverse z FFT", "plane_bwd (xy IFFT+unfold)"]
     top = int(np.argmax(stage))
     # The largest stage as a kernel roofline.  The plane kernels move the path's f0 bytes
     # (4 M^3 per field, read by the forward fold, written by the backward unfold); the
@@ -516,7 +516,7 @@ def run_ours(args):
                    "forward_rel_err_vs_fp64": fwd_err},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "peak_source": peak_src, "traffic": None,
-                     "scope": "whole forward+backward per batch (6 launches per 64-field chunk); algorithmic bytes 2*(4*M^3 + 8*n_spec) per field",
+                     "scope": "whole forward+backward per batch (5 launches per 64-field chunk); algorithmic bytes 2*(4*M^3 + 8*n_spec) per field",
                      "stage_ms": {n: float(v) for n, v in zip(names, stage)}, "dominant_stage": names[top],
                      "dominant_kernel": kern, "flops_per_field": flops_field,
                      "achieved_tflops": flops_field / (us_field * 1e-6) / 1e12},

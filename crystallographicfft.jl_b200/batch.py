@@ -5,7 +5,7 @@ Neither has a reference counterpart: CrystallographicFFT.jl transforms one field
 time on the CPU.  They serve batches of fields of uneven space group and grid size.
 
 * autotune_plan times candidate execution choices (cfft_tuning: chunk size, lanes,
-  fused-z slots per CTA, the wide backward gather, the bulk-copy plane kernels, the
+  fused-z slots per CTA, the rows of the backward gather, the bulk-copy plane kernels, the
   fused cluster kernels) on the device with CUDA events, by coordinate descent from the
   defaults, and caches the winner in a JSON file keyed by device, operations, grid,
   precision, batch, operation and path; autotune_path also chooses the decomposition

@@ -1,19 +1,20 @@
 // Device execution layer of libcfft_b200 (sm_100a).
 //
-// Forward KRFFT per batch of fields (centred fold path; the plain M2 path is the
-// same pipeline with one channel and no fold):
-//   k_plane_fwd   f0 (HBM) -> [fold (WHT8) + twiddle] -> x/y FFT in shared memory
-//                 -> channel workspace   (one CTA per z-plane pair per field)
-//   k_fft_z       z FFT of the channel workspace in place (one CTA per xz-plane)
-//   k_recon       spectral-ASU gather: F(h) = sum_b e^{-2 pi i h.t_b/N} G0(R_b^T h mod M)
-//                 (indices and phases computed on the fly from the representative ops)
-// Backward:
-//   k_inv_recon   G0 at orbit representatives from the aliasing identity
-//                 G0(q) = (1/d) sum_a F(q + M.alpha_a), expanded to the whole orbit
-//                 with G0(R^T q) = e^{2 pi i q.s/M} G0(q)
-//   k_fft_z (inverse), k_plane_bwd (inverse x/y FFT + unfold (inverse WHT / 8) -> f0)
+// Three families of transform kernels, chosen per plan:
+//  - cubic channel grids of certain edges: compile-time sized kernels (fast_kernels.cuh);
+//  - other channel grids of 2-3-5 lengths: general kernels (general_kernels.cuh);
+//  - lengths that do not split into two register radices, tables past the packed limits,
+//    and the allocation-free forward: the Stockham kernels below, one field per transform:
+//      k_plane_fwd   f0 (HBM) -> [fold (WHT8) + twiddle] -> x/y FFT in shared memory
+//                    -> channel workspace   (one CTA per z-plane per field)
+//      k_fft_z       z FFT of the channel workspace in place (one CTA per xz-plane)
+//      k_recon       spectral-ASU gather: F(h) = sum_b e^{-2 pi i h.t_b/N} G0(R_b^T h mod M)
+//      k_inv_recon   G0 at orbit representatives from the aliasing identity
+//                    G0(q) = (1/d) sum_a F(q + M.alpha_a), expanded to the whole orbit
+//                    with G0(R^T q) = e^{2 pi i q.s/M} G0(q)
+//      k_fft_z (inverse), k_plane_bwd (inverse x/y FFT + unfold (inverse WHT / 8) -> f0)
 // The diffusion kernel K multiplies inside k_recon, and e^{-w dt/2} inside the
-// plane kernels, so one SCFT contour step is six launches with no extra passes.
+// plane kernels, so one SCFT contour step is five launches with no extra passes.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -596,7 +597,7 @@ std::vector<unsigned char> make_table_bytes(const Plan& p, DevGeom* g) {
 // point lie in that unit's two rows.  Units are ordered by point count, largest first.
 // Leaves the fusion off (plan unchanged) when a point falls in a parity class without
 // a channel or CFFT_ZRECON=0.
-Status build_zrecon_units(Plan* p, const DevGeom& g, std::string* err) {
+Status build_zrecon_units(Plan* p, std::string* err) {
   if (const char* e = std::getenv("CFFT_ZRECON")) if (e[0] == '0') return Status::kOk;
   const PlanTables& T = p->T;
   const int H = p->fast_h, nch = T.n_ch;
@@ -652,39 +653,12 @@ Status build_zrecon_units(Plan* p, const DevGeom& g, std::string* err) {
     pts.insert(pts.end(), u.pts.begin(), u.pts.end());
   }
   if (ut.empty()) return Status::kOk;
-  // Points with their packed h, and the weights of the Hermitian tap pairs (sg, 7 - sg): with
-  // u = w[sg], v = w[7 - sg] the phases e^{-2 pi i h.t / N} of the two sign images,
-  // Pw = (u + v) / 2 and Qw = ((v.y - u.y) / 2, (u.x - v.x) / 2).
-  std::vector<uint2> pt(pts.size());
-  std::vector<double> pq(pts.size() * 16), phase(2 * static_cast<size_t>(T.P));
-  for (int j = 0; j < T.P; ++j) {
-    phase[2 * j] = std::cos(2.0 * M_PI * j / T.P);
-    phase[2 * j + 1] = -std::sin(2.0 * M_PI * j / T.P);
-  }
+  std::vector<uint2> pt(pts.size());  // with the packed h
   for (size_t i = 0; i < pts.size(); ++i) {
     const auto& h = T.spec[pts[i]].h;
     pt[i] = make_uint2(pts[i], static_cast<uint32_t>(h[0]) | (static_cast<uint32_t>(h[1]) << 10) | (static_cast<uint32_t>(h[2]) << 20));
-    const double* w[8];
-    for (int sg = 0; sg < 8; ++sg) {
-      long j = 0;
-      for (int d = 0; d < 3; ++d) j += static_cast<long>(h[d]) * g.rep_tp[g.sign_op[sg]][d];
-      w[sg] = &phase[2 * floor_mod(j, T.P)];
-    }
-    for (int sg = 0; sg < 4; ++sg) {
-      const double* u = w[sg];
-      const double* v = w[7 - sg];
-      double* op = &pq[(static_cast<size_t>(2 * sg) * pts.size() + i) * 2];
-      double* oq = op + pts.size() * 2;
-      op[0] = 0.5 * (u[0] + v[0]);
-      op[1] = 0.5 * (u[1] + v[1]);
-      oq[0] = 0.5 * (v[1] - u[1]);
-      oq[1] = 0.5 * (u[0] - v[0]);
-    }
   }
-  std::vector<float> pqf;
-  if (p->precision == 4) pqf.assign(pq.begin(), pq.end());
-  const void* pq_src = p->precision == 4 ? static_cast<const void*>(pqf.data()) : pq.data();
-  const size_t pq_bytes = pq.size() * p->precision;
+  const size_t pq_bytes = pts.size() * 16 * p->precision;
   // Plan-owned device tables: counted in the plan's device bytes, allocation failures
   // reported as such (like the other plan buffers).
   for (auto [ptr, bytes, what] : {std::tuple<void**, size_t, const char*>{&p->d_zr_units, ut.size() * sizeof(uint4), "fused gather units"},
@@ -696,8 +670,13 @@ Status build_zrecon_units(Plan* p, const DevGeom& g, std::string* err) {
   }
   CFFT_CUDA(cudaMemcpy(p->d_zr_units, ut.data(), ut.size() * sizeof(uint4), cudaMemcpyHostToDevice), "upload units");
   CFFT_CUDA(cudaMemcpy(p->d_zr_pts, pt.data(), pt.size() * sizeof(uint2), cudaMemcpyHostToDevice), "upload unit points");
-  CFFT_CUDA(cudaMemcpy(p->d_zr_pq, pq_src, pq_bytes, cudaMemcpyHostToDevice), "upload unit weights");
   p->zr_npts = static_cast<int>(pts.size());
+  // The weights, on the default stream: the kernel upload that ends the plan's set-up waits for it.
+  FastArgs a;
+  a.geom = p->d_geom; a.tables = p->d_tables; a.zr_pts = p->d_zr_pts; a.zr_pq = p->d_zr_pq; a.n_spec_pts = p->zr_npts;
+  a.stage = 8;
+  const Status ws = p->precision == 8 ? fast_other_f64(a, err) : fast_other_f32(a, err);
+  if (ws != Status::kOk) return ws;
   p->zr_units = static_cast<int>(ut.size());
   p->zrecon = true;
   return Status::kOk;
@@ -1389,7 +1368,7 @@ Status plan_device_init(Plan* p, std::string* err) {
     CFFT_CUDA(cudaMemcpy(p->d_fib_outs, fib_outs.data(), fib_outs.size() * sizeof(uint2), cudaMemcpyHostToDevice), "upload fiber outputs");
   }
   if (p->fast_h && p->rep_diag8 && !p->qmode) {
-    Status zs = build_zrecon_units(p, g, err);
+    Status zs = build_zrecon_units(p, err);
     if (zs != Status::kOk) return zs;
   }
   // Orbit expansion writes only alive positions; channel positions never written stay zero.
@@ -1898,13 +1877,16 @@ Status exec_sub_to_full(Plan* p, const void* f0, void* u, int B, void* stream, s
   const int32_t* map = static_cast<const int32_t*>(p->d_fill_map);
   const bool vec = nvol % 4 == 0 && reinterpret_cast<uintptr_t>(u) % 16 == 0;
   const size_t per = vec ? 1024 : 256;
-  const dim3 grid(static_cast<unsigned>((nvol + per - 1) / per), (B + kFillFields - 1) / kFillFields);
-  if (p->precision == 8) {
-    auto* k = vec ? k_sub_to_full<double, 4> : k_sub_to_full<double, 1>;
-    k<<<grid, 256, 0, s>>>(static_cast<const double*>(f0), map, static_cast<double*>(u), mvol, nvol, B);
-  } else {
-    auto* k = vec ? k_sub_to_full<float, 4> : k_sub_to_full<float, 1>;
-    k<<<grid, 256, 0, s>>>(static_cast<const float*>(f0), map, static_cast<float*>(u), mvol, nvol, B);
+  for (int b0 = 0; b0 < B; b0 += 65535 * kFillFields) {
+    const int nb = std::min(B - b0, 65535 * kFillFields);
+    const dim3 grid(static_cast<unsigned>((nvol + per - 1) / per), (nb + kFillFields - 1) / kFillFields);
+    if (p->precision == 8) {
+      auto* k = vec ? k_sub_to_full<double, 4> : k_sub_to_full<double, 1>;
+      k<<<grid, 256, 0, s>>>(static_cast<const double*>(f0) + b0 * mvol, map, static_cast<double*>(u) + b0 * nvol, mvol, nvol, nb);
+    } else {
+      auto* k = vec ? k_sub_to_full<float, 4> : k_sub_to_full<float, 1>;
+      k<<<grid, 256, 0, s>>>(static_cast<const float*>(f0) + b0 * mvol, map, static_cast<float*>(u) + b0 * nvol, mvol, nvol, nb);
+    }
   }
   ++g_launches;
   CFFT_CUDA(cudaGetLastError(), "subgrid_to_fullgrid launch");

@@ -14,7 +14,7 @@ struct Tuning {
   int64_t chunk_bytes = 0;  // channel workspace per chunk
   int lanes = 0;            // concurrent chunk lanes
   int zr_slots = 0;         // slots per CTA of the fused z FFT + gather (2 or 4)
-  int wide = -1;            // backward gather in 128-byte field groups
+  int wide = -1;            // representatives in rows of 64 bytes
   int tma = -1;             // bulk-copy plane kernels: bit 0 forward, bit 1 backward
   int cluster = -1;         // fused cluster kernels: 0, 8 or 16 CTAs
 };

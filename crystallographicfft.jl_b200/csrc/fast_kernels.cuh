@@ -482,10 +482,15 @@ template <typename T> inline int plane_line_threads(int H, int nch, bool folded)
   return folded && rounds(base + 64) < rounds(base) && rounds(base + 64) <= 2 ? base + 64 : base;
 }
 
+// Registers of the forward plane kernel: its sixteen loads in flight take up to 130; below
+// H = 32 a cap of 112 keeps a block more on an SM (Ia-3d 96^3 contour steps, 256 fields x 20:
+// 3244 us without, 3115 with 112, 3151 with 96; Im-3m 128^3: 125.7 / 126.2 / 129.3).
+template <typename T, int H> constexpr int fold_registers() { return sizeof(T) == 4 && H < 32 ? 112 : 255; }
+
 // Forward plane kernel, cubic H: fold (or plain load) of two fields + x FFT + y FFT
 // -> W[slot][c][z][y][x].
 template <typename T, int H, int CT>
-__global__ void k_plane_fwd_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+__global__ void __maxnreg__((fold_registers<T, H>())) k_plane_fwd_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
                               const T* __restrict__ f0, const T* __restrict__ E, typename Cx<T>::type* __restrict__ W,
                               int nfields) {
   pdl_enter();
@@ -1319,6 +1324,32 @@ __global__ void k_recon_diag8(const DevGeom* __restrict__ g, const typename Cx<T
     if (USE_K) { acca = cscale(acca, kk); accb = cscale(accb, kk); }
     F[static_cast<size_t>(fa) * ns + s] = acca;
     if (fa + 1 < nfields) F[static_cast<size_t>(fa + 1) * ns + s] = accb;
+  }
+}
+
+// Weights of the Hermitian tap pairs (sg, 7 - sg) of the fused gather's points, once per plan:
+// with u = w[sg], v = w[7 - sg] the phases e^{-2 pi i h.t / N} of the two sign images,
+// Pw = (u + v) / 2 and Qw = ((v.y - u.y) / 2, (u.x - v.x) / 2).
+template <typename T>
+__global__ void __launch_bounds__(256) k_zr_weights(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
+                                                    const uint2* __restrict__ pts, int npts, typename Cx<T>::type* __restrict__ pq) {
+  using C = typename Cx<T>::type;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= npts) return;
+  const uint32_t hp = pts[i].y;
+  const int h[3] = {static_cast<int>(hp & 1023u), static_cast<int>((hp >> 10) & 1023u), static_cast<int>((hp >> 20) & 1023u)};
+  const int P = g->P;
+  C w[8];
+  for (int sg = 0; sg < 8; ++sg) {
+    const int* tp = g->rep_tp[g->sign_op[sg]];
+    const int j = (h[0] * tp[0] + h[1] * tp[1] + h[2] * tp[2]) % P;
+    w[sg] = tables[g->ph_off + (j < 0 ? j + P : j)];
+  }
+  const T half = static_cast<T>(0.5);
+  for (int sg = 0; sg < 4; ++sg) {
+    const C u = w[sg], v = w[7 - sg];
+    pq[static_cast<size_t>(2 * sg) * npts + i] = mk<C>(half * (u.x + v.x), half * (u.y + v.y));
+    pq[static_cast<size_t>(2 * sg + 1) * npts + i] = mk<C>(half * (v.y - u.y), half * (u.x - v.x));
   }
 }
 
@@ -2455,6 +2486,10 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
         });
         break;
       }
+      case 8:  // plan set-up: weights of the fused gather
+        k_zr_weights<T><<<(a.n_spec_pts + 255) / 256, 256, 0, st>>>(g, tab, static_cast<const uint2*>(a.zr_pts), a.n_spec_pts,
+                                                                   static_cast<C*>(const_cast<void*>(a.zr_pq)));
+        break;
       case 7:  // forward z FFT + separable Q-multiply + inverse z FFT, in place on W
         CFFT_FOR_H(H, {
           constexpr int HP = HH / 2 + 1;

@@ -93,7 +93,7 @@ typedef struct cfft_info {
   int max_batch;
   int P;                 /* lcm(N): phase denominator */
   int64_t workspace_bytes;
-  int exec_path;         /* bit 0: compile-time sized kernels; bit 1: packed quad backward gather;
+  int exec_path;         /* bit 0: compile-time sized kernels; bit 1: packed backward gather by fibers;
                             bit 2: fused 8-CTA cluster kernels; bit 3 / bit 4: persistent bulk-copy
                             (TMA) forward / backward plane kernels; bit 5: backward gather in
                             groups of 16 (FP32) / 8 (FP64) fields; bit 6: separable Q-multiply
@@ -186,7 +186,7 @@ typedef struct cfft_tuning {
   int64_t chunk_bytes;   /* channel workspace per chunk (CFFT_CHUNK_BYTES; 64 MiB) */
   int lanes;             /* concurrent chunk lanes 1..4 (CFFT_LANES; 2 for batches >= 8) */
   int zr_slots;          /* workspace slots per CTA of the fused z FFT + gather, 2 or 4 (CFFT_ZR_SLOTS; 4) */
-  int wide;              /* backward gather in 128-byte field groups: 0, 1 (CFFT_WIDE; 1) */
+  int wide;              /* backward representatives in 64-byte rows: 0, 1 (CFFT_WIDE; 1) */
   int tma;               /* bulk-copy plane kernels: 0, 1 forward, 2 backward, 3 both (CFFT_TMA; 0) */
   int cluster;           /* fused cluster kernels: 0, 8 or 16 CTAs (CFFT_CLUSTER; 0) */
 } cfft_tuning;
