@@ -704,6 +704,7 @@ Status launch_stage(Plan* p, int stage, const T* f0, typename Cx<T>::type* F, co
     a.W = W;
     a.G0R = p->d_g0r ? static_cast<char*>(p->d_g0r) + lane * p->g0r_lane_bytes : nullptr;
     a.f0 = f0; a.F = F; a.Fin = Fin; a.f0_out = f0_out; a.E = E;
+    a.slot_fields = p->general ? 1 : 2;
     a.stage = stage; a.nb = nb; a.H = p->fast_h; a.n_ch = T_.n_ch; a.centered = T_.centered ? 1 : 0;
     a.cent_type = p->cent_type; a.d = T_.d;
     a.n_spec = static_cast<int>(T_.spec.size()); a.n_orbits = static_cast<int>(T_.orbit_rep.size());
@@ -1220,7 +1221,7 @@ Status plan_device_init(Plan* p, std::string* err) {
   size_t budget = static_cast<size_t>(64) << 20;
   if (const char* cb = std::getenv("CFFT_CHUNK_BYTES")) budget = std::strtoull(cb, nullptr, 10);
   if (p->tune.chunk_bytes > 0) budget = static_cast<size_t>(p->tune.chunk_bytes);
-  const size_t per_field = T.n_ch * hvol * cs / (tables ? 2 : 1);
+  const size_t per_field = T.n_ch * hvol * cs / (p->fast_h ? 2 : 1);
   size_t ch = std::max<size_t>(1, std::min<size_t>(B, budget / std::max<size_t>(per_field, 1)));
   // Two concurrent lanes once the batch's channel workspace reaches 48 MiB: below, one lane
   // fills the SMs and a second doubles the launches.  Measured with one / two lanes, us per
@@ -1232,7 +1233,7 @@ Status plan_device_init(Plan* p, std::string* err) {
   else if (const char* ln = std::getenv("CFFT_LANES")) p->lanes = std::max(1, std::min(Plan::kMaxLanes, std::atoi(ln)));
   else if (tables && B >= 8 && B * per_field >= (static_cast<size_t>(48) << 20)) p->lanes = 2;
   if (p->lanes > 1) ch = std::min(ch, (B + p->lanes - 1) / p->lanes);
-  if (tables && ch < B && ch > 1) ch &= ~static_cast<size_t>(1);
+  if (p->fast_h && ch < B && ch > 1) ch &= ~static_cast<size_t>(1);
   p->chunk = static_cast<int>(ch);
   // launch geometry and shared memory (generic path)
   const long pe = static_cast<long>(T.n_ch) * T.H[0] * T.H[1];
@@ -1262,8 +1263,7 @@ Status plan_device_init(Plan* p, std::string* err) {
     if ((st = alloc(&p->d_inv_phase, T.inv_phase.size() * 4, "inverse phase")) != Status::kOk) return st;
     if ((st = alloc(&p->d_img_mask, masks.size() * 4, "image masks")) != Status::kOk) return st;
   }
-  const size_t slots = p->general ? (chunk + 1) / 2 : chunk;
-  p->w_lane_bytes = ((slots * T.n_ch * hvol * cs + 255) / 256) * 256;
+  p->w_lane_bytes = ((chunk * T.n_ch * hvol * cs + 255) / 256) * 256;
   if ((st = alloc(&p->d_work_T, p->lanes * p->w_lane_bytes, "channel workspace")) != Status::kOk) return st;
   if ((st = alloc(&p->d_work_F, B * T.spec.size() * cs, "spectrum workspace")) != Status::kOk) return st;
   if ((st = alloc(&p->d_work_E, B * mvol * rs, "interaction workspace")) != Status::kOk) return st;

@@ -68,7 +68,7 @@ struct Plan {
   // launch geometry
   int threads_xy = 0, threads_z = 0;
   int fast_h = 0;               // cubic channel edge of the compile-time sized kernels (0 = generic)
-  bool general = false;         // general kernels (any 2-3-5 grid; two fields per slot)
+  bool general = false;         // general kernels (any 2-3-5 grid; one field per slot)
   GenShape gen;                 // their geometry
   int chunk = 1;                // fields per workspace chunk
   int lanes = 1;                // concurrent chunk lanes

@@ -1607,8 +1607,9 @@ template <typename C, int D> __device__ __forceinline__ void wht_d(C (&v)[D]) {
 // group are exchanged through shared memory and leave as whole rows G0P[group][orbit][L]
 // for the expansion.  Im-3m 128^3 FP32, 64 fields: 7.5 + 15.0 us (regroup of the spectra
 // and one gather per orbit, 8 x the loads) before.
+// NF: fields per slot, 2 or, for the general kernels, 1.
 constexpr int kFibers = 32;
-template <typename T, int D, int L>
+template <typename T, int D, int L, int NF>
 __global__ void __launch_bounds__(kFibers * L)
 k_inv_fiber(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
             const uint2* __restrict__ taps, const uint2* __restrict__ outs, int nf,
@@ -1631,14 +1632,14 @@ k_inv_fiber(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restric
   }
   if constexpr (EARLY) pdl_enter();
   const int gq = blockIdx.y;
-  const int fa = 2 * (gq * L + j);
+  const int fa = NF * (gq * L + j);
   const C* ph = tables + g->ph_off;
   const int ns = g->n_spec;
   const C zero = mk<C>(static_cast<T>(0), static_cast<T>(0));
   C x[D];
   if (f < nf && fa < nb) {
     const C* Fa = F + static_cast<size_t>(fa) * ns;
-    const bool has_b = fa + 1 < nb;
+    const bool has_b = NF == 2 && fa + 1 < nb;
     C va[D], vb[D];
 #pragma unroll
     for (int m = 0; m < D; ++m) {
@@ -2505,18 +2506,20 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
           const uint2* tp = static_cast<const uint2*>(a.fib_taps);
           const uint2* fo = static_cast<const uint2*>(a.fib_outs);
           const int fb = (a.n_fib + kFibers - 1) / kFibers;
-#define CFFT_INV_FIBER(LL)                                                                                          \
-  {                                                                                                                 \
-    const dim3 gf(fb, (nslots + (LL) - 1) / (LL));                                                                  \
-    switch (a.d) {                                                                                                  \
-      case 1: launch_k(k_inv_fiber<T, 1, LL>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
-      case 2: launch_k(k_inv_fiber<T, 2, LL>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
-      case 4: launch_k(k_inv_fiber<T, 4, LL>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
-      default: launch_k(k_inv_fiber<T, 8, LL>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
-    }                                                                                                               \
+#define CFFT_INV_FIBER(LL, NF)                                                                                          \
+  {                                                                                                                     \
+    const int ns = (nb + (NF) - 1) / (NF);                                                                              \
+    const dim3 gf(fb, (ns + (LL) - 1) / (LL));                                                                          \
+    switch (a.d) {                                                                                                      \
+      case 1: launch_k(k_inv_fiber<T, 1, LL, NF>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
+      case 2: launch_k(k_inv_fiber<T, 2, LL, NF>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
+      case 4: launch_k(k_inv_fiber<T, 4, LL, NF>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
+      default: launch_k(k_inv_fiber<T, 8, LL, NF>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
+    }                                                                                                                   \
   }
-          if (a.reps_wide) CFFT_INV_FIBER(wide_slots<C>())
-          else CFFT_INV_FIBER(2)
+          if (a.slot_fields == 1) CFFT_INV_FIBER(2, 1)
+          else if (a.reps_wide) CFFT_INV_FIBER(wide_slots<C>(), 2)
+          else CFFT_INV_FIBER(2, 2)
 #undef CFFT_INV_FIBER
           break;
         }

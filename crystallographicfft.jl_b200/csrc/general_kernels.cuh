@@ -1,11 +1,14 @@
 // Kernels of libcfft_b200 for channel grids of any 2-3-5 shape (sm_100a): unequal axes,
 // plane groups, and cubic edges without a compile-time sized kernel.
 //
-// As on the compile-time sized path two real fields share a complex transform, the inverse
-// gather works by fibers (k_inv_fiber) and the orbit expansion feeds the inverse z lines.  A
-// line of n = A x B points is two in-place register passes through one shared-memory buffer,
-// the radices 2 to 16 chosen at run time; lengths that do not split that way keep the
-// Stockham kernels of exec.cu (out of place, one field per transform, a pass per factor up
+// As on the compile-time sized path the inverse gather works by fibers (k_inv_fiber) and the
+// orbit expansion feeds the inverse z lines.  Each field has its own workspace slot and
+// complex transform: two fields as a + i b would halve the line transforms (GPU us of a round
+// trip, paired / alone: P6/mmm 60 x 60 x 80 FP64 x4 43 / 63, Im-3m 160^3 FP64 x8 91 / 119, p4mm
+// 160^2 FP64 x64 34 / 35), but the rounding error of one would then scale with the other, and a
+// NaN or the imaginary part of an inverse would cross over.  A line of n = A x B points is two in-place register passes
+// through one shared-memory buffer, the radices 2 to 16 chosen at run time; lengths that do
+// not split that way keep the Stockham kernels of exec.cu (out of place, a pass per factor up
 // to 8), which these replace: P6/mmm 60 x 60 x 80 FP64, 4 fields, plane kernels 45 / 47 us,
 // z 25 / 25, inverse gather 33 before.
 #pragma once
@@ -130,14 +133,14 @@ template <typename C> __device__ __forceinline__ void copy_twiddles(C* dst, cons
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = __ldg(src + i);
 }
 
-// Forward plane kernel: fold (or plain load) of two fields, x and y lines, -> W[slot][c][z][y][x].
+// Forward plane kernel: fold (or plain load) of a field, x and y lines, -> W[field][c][z][y][x].
 // The fold puts x at position x / B + A (x mod B) (y likewise), so the first pass works on
 // contiguous blocks of A and both passes leave frequencies in natural order: the last one
 // stores straight to the workspace along x.
 template <typename T>
 __global__ void __launch_bounds__(kGenThreads, sizeof(T) == 4 ? 2 : 1)
 k_gplane_fwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, const T* __restrict__ f0,
-             const T* __restrict__ E, typename Cx<T>::type* __restrict__ W, int nfields) {
+             const T* __restrict__ E, typename Cx<T>::type* __restrict__ W) {
   using C = typename Cx<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
@@ -147,13 +150,10 @@ k_gplane_fwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
   copy_twiddles(tw0, tables + s.tw[0], H0);
   copy_twiddles(tw1, tables + s.tw[1], H1);
   pdl_enter();
-  const int iz = blockIdx.x, slot = blockIdx.y, fa = 2 * slot;
-  const bool has_b = fa + 1 < nfields;
+  const int iz = blockIdx.x, f = blockIdx.y;
   const T zero = static_cast<T>(0);
-  const T* srca = f0 + static_cast<size_t>(fa) * s.mvol;
-  const T* srcb = srca + s.mvol;
-  const T* Ea = E ? E + static_cast<size_t>(fa) * s.mvol : nullptr;
-  const T* Eb = E ? Ea + s.mvol : nullptr;
+  const T* src = f0 + static_cast<size_t>(f) * s.mvol;
+  const T* Ef = E ? E + static_cast<size_t>(f) * s.mvol : nullptr;
   const int A0 = s.A[0], B0 = s.B[0], A1 = s.A[1], B1 = s.B[1];
   const int plane = H0 * H1;
   auto place = [&](int iy, int ix) {
@@ -161,25 +161,25 @@ k_gplane_fwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
     return buf + (qy + A1 * (iy - qy * B1)) * S + qx + A0 * (ix - qx * B0);
   };
   if (!s.centered) {
-    constexpr int U = 4;  // values in flight per field and thread
+    constexpr int U = 8;  // values in flight per thread
     for (int e0 = threadIdx.x; e0 < plane; e0 += U * blockDim.x) {
-      C v[U];
+      T v[U];
 #pragma unroll
       for (int k = 0; k < U; ++k) {
-        const int e = e0 + k * blockDim.x, idx = iz * plane + e;
-        v[k] = mk<C>(e < plane ? __ldcs(srca + idx) : zero, e < plane && has_b ? __ldcs(srcb + idx) : zero);
+        const int e = e0 + k * blockDim.x;
+        v[k] = e < plane ? __ldcs(src + iz * plane + e) : zero;
       }
-      if (E) {
+      if (Ef) {
 #pragma unroll
         for (int k = 0; k < U; ++k) {
-          const int e = e0 + k * blockDim.x, idx = iz * plane + e;
-          if (e < plane) v[k] = mk<C>(v[k].x * __ldg(Ea + idx), has_b ? v[k].y * __ldg(Eb + idx) : zero);
+          const int e = e0 + k * blockDim.x;
+          if (e < plane) v[k] *= __ldg(Ef + iz * plane + e);
         }
       }
 #pragma unroll
       for (int k = 0; k < U; ++k) {
         const int e = e0 + k * blockDim.x, iy = div_by(e, s.dH[0]);
-        if (e < plane) *place(iy, e - iy * H0) = v[k];
+        if (e < plane) *place(iy, e - iy * H0) = mk<C>(v[k], zero);
       }
     }
   } else {
@@ -187,31 +187,28 @@ k_gplane_fwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
     for (int e = threadIdx.x; e < plane; e += blockDim.x) {
       const int iy = div_by(e, s.dH[0]), ix = e - iy * H0;
       C* d = place(iy, ix);
-      C p[8];
+      T p[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int idx = ((iz + ((k >> 2) & 1) * H2) * M1 + iy + ((k >> 1) & 1) * H1) * M0 + ix + (k & 1) * H0;
-        p[k] = mk<C>(__ldcs(srca + idx), has_b ? __ldcs(srcb + idx) : zero);
-      }
-      if (E) {
+      for (int k = 0; k < 8; ++k)
+        p[k] = __ldcs(src + ((iz + ((k >> 2) & 1) * H2) * M1 + iy + ((k >> 1) & 1) * H1) * M0 + ix + (k & 1) * H0);
+      if (Ef) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int idx = ((iz + ((k >> 2) & 1) * H2) * M1 + iy + ((k >> 1) & 1) * H1) * M0 + ix + (k & 1) * H0;
-          p[k] = mk<C>(p[k].x * __ldg(Ea + idx), has_b ? p[k].y * __ldg(Eb + idx) : zero);
-        }
+        for (int k = 0; k < 8; ++k)
+          p[k] *= __ldg(Ef + ((iz + ((k >> 2) & 1) * H2) * M1 + iy + ((k >> 1) & 1) * H1) * M0 + ix + (k & 1) * H0);
       }
-      wht8c(p);
+      wht8(p);
       const C tx = tables[s.ftw[0] + ix], ty = tables[s.ftw[1] + iy], tz = tables[s.ftw[2] + iz];
       const C txy = cmul(tx, ty);
 #pragma unroll
       for (int o = 0; o < 8; ++o) {
         const int c = s.chan[o];
         if (c < 0) continue;
-        C w = p[o];
-        if ((o & 3) == 3) w = cmul(w, txy);
-        else if (o & 1) w = cmul(w, tx);
-        else if (o & 2) w = cmul(w, ty);
-        if (o & 4) w = cmul(w, tz);
+        C w = mk<C>(p[o], zero);
+        if ((o & 3) == 3) w = cscale(txy, p[o]);
+        else if (o & 1) w = cscale(tx, p[o]);
+        else if (o & 2) w = cscale(ty, p[o]);
+        if (o == 4) w = cscale(tz, p[o]);
+        else if (o & 4) w = cmul(w, tz);
         d[c * PL] = w;
       }
     }
@@ -230,7 +227,7 @@ k_gplane_fwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
   }
   // y lines: line l = (c, x)
   auto col = [&](int l) { const int c = div_by(l, s.dH[0]); return c * PL + l - c * H0; };
-  C* dst = W + static_cast<size_t>(slot) * nch * s.hvol + static_cast<size_t>(iz) * plane;
+  C* dst = W + static_cast<size_t>(f) * nch * s.hvol + static_cast<size_t>(iz) * plane;
   auto out = [&](int l, int ky) { const int c = div_by(l, s.dH[0]); return dst + static_cast<size_t>(c) * s.hvol + ky * H0 + l - c * H0; };
   if (B1 > 1) {
     line_pass<C, false, true>(A1, B1, Ly, s.dLy, tw1, [&](int l, int j, int r) { return buf[col(l) + (j * A1 + r) * S]; },
@@ -245,21 +242,21 @@ k_gplane_fwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
 }
 
 // X at a channel point from the packed expansion entry (orbit | phase << 21) and the
-// representatives' rows G0P[slot / 2][orbit][slot & 1].
+// representatives' rows G0P[field / 2][orbit][field & 1].
 template <typename C>
 __device__ __forceinline__ C expand_point(const uint32_t* __restrict__ et, const C* __restrict__ rp, const C* __restrict__ ph) {
   const uint32_t t = __ldg(et);
   return cmulc(__ldg(rp + 2 * static_cast<size_t>(t & 0x1FFFFFu)), __ldg(ph + (t >> 21)));
 }
 
-// Backward plane kernel: inverse y and x lines of W[slot][c][iz] (or, for a single z plane,
-// of the orbit expansion itself) and the unfold.  Natural order in, so x comes out at
+// Backward plane kernel: inverse y and x lines of W[field][c][iz] (or, for a single z plane,
+// of the orbit expansion itself) and the unfold's real part.  Natural order in, so x comes out at
 // (x mod A) B + x / A, where the unfold reads it.
 template <typename T, bool EXPAND>
 __global__ void __launch_bounds__(kGenThreads, sizeof(T) == 4 ? 2 : 1)
 k_gplane_bwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, const typename Cx<T>::type* __restrict__ W,
              const uint32_t* __restrict__ ETP, const typename Cx<T>::type* __restrict__ G0P, const T* __restrict__ E,
-             T* __restrict__ f0, int nfields) {
+             T* __restrict__ f0) {
   using C = typename Cx<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
@@ -269,13 +266,12 @@ k_gplane_bwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
   copy_twiddles(tw0, tables + s.tw[0], H0);
   copy_twiddles(tw1, tables + s.tw[1], H1);
   pdl_enter();
-  const int iz = blockIdx.x, slot = blockIdx.y, fa = 2 * slot;
-  const bool has_b = fa + 1 < nfields;
+  const int iz = blockIdx.x, f = blockIdx.y;
   const int A0 = s.A[0], B0 = s.B[0], A1 = s.A[1], B1 = s.B[1];
   const int plane = H0 * H1, Lx = nch * H1, Ly = nch * H0;
   __syncthreads();
-  const C* src = EXPAND ? nullptr : W + static_cast<size_t>(slot) * nch * s.hvol + static_cast<size_t>(iz) * plane;
-  const C* rp = EXPAND ? G0P + static_cast<size_t>(slot >> 1) * s.n_orbits * 2 + (slot & 1) : nullptr;
+  const C* src = EXPAND ? nullptr : W + static_cast<size_t>(f) * nch * s.hvol + static_cast<size_t>(iz) * plane;
+  const C* rp = EXPAND ? G0P + static_cast<size_t>(f >> 1) * s.n_orbits * 2 + (f & 1) : nullptr;
   auto in = [&](int l, int ky) {
     const int c = div_by(l, s.dH[0]);
     const size_t at = static_cast<size_t>(c) * s.hvol + ky * H0 + l - c * H0;
@@ -299,29 +295,26 @@ k_gplane_bwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
                               [&](int l, int j, int k, C v) { buf[l * S + j * B0 + k] = v; });
     __syncthreads();
   }
-  T* dsta = f0 + static_cast<size_t>(fa) * s.mvol;
-  T* dstb = dsta + s.mvol;
-  const T* Ea = E ? E + static_cast<size_t>(fa) * s.mvol : nullptr;
-  const T* Eb = E ? Ea + s.mvol : nullptr;
+  T* dst = f0 + static_cast<size_t>(f) * s.mvol;
+  const T* Ef = E ? E + static_cast<size_t>(f) * s.mvol : nullptr;
   // v / V as two terms: the rounding error of 1 / V alone accumulates over a contour loop.
   const T hi = static_cast<T>(s.inv_v), lo = static_cast<T>(s.inv_v - static_cast<double>(hi));
-  auto put = [&](int idx, C v) {
-    T a = fma(v.x, hi, v.x * lo), b = fma(v.y, hi, v.y * lo);
-    if (E) { a *= __ldg(Ea + idx); if (has_b) b *= __ldg(Eb + idx); }
-    __stcs(dsta + idx, a);
-    if (has_b) __stcs(dstb + idx, b);
+  auto put = [&](int idx, T v) {
+    T a = fma(v, hi, v * lo);
+    if (Ef) a *= __ldg(Ef + idx);
+    __stcs(dst + idx, a);
   };
   for (int e = threadIdx.x; e < plane; e += blockDim.x) {
     const int iy = div_by(e, s.dH[0]), ix = e - iy * H0;
     const int qx = div_by(ix, s.dA[0]), qy = div_by(iy, s.dA[1]);
     const C* d = buf + ((iy - qy * A1) * B1 + qy) * S + (ix - qx * A0) * B0 + qx;
     if (!s.centered) {
-      put(iz * plane + e, *d);
+      put(iz * plane + e, d->x);
     } else {
       const int M0 = 2 * H0, M1 = 2 * H1;
       const C tx = tables[s.ftw[0] + ix], ty = tables[s.ftw[1] + iy], tz = tables[s.ftw[2] + iz];
       const C txy = cmul(tx, ty);
-      C p[8];
+      T p[8];
 #pragma unroll
       for (int o = 0; o < 8; ++o) {
         const int c = s.chan[o];
@@ -333,9 +326,9 @@ k_gplane_bwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
           else if (o & 2) w = cmulc(w, ty);
           if (o & 4) w = cmulc(w, tz);
         }
-        p[o] = w;
+        p[o] = w.x;
       }
-      wht8c(p);
+      wht8(p);
 #pragma unroll
       for (int k = 0; k < 8; ++k)
         put(((iz + ((k >> 2) & 1) * H2) * M1 + iy + ((k >> 1) & 1) * H1) * M0 + ix + (k & 1) * H0, p[k]);
@@ -343,7 +336,7 @@ k_gplane_bwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
   }
 }
 
-// z lines of one (y, c, slot): forward in place on W, or inverse from the orbit expansion
+// z lines of one (y, c, field): forward in place on W, or inverse from the orbit expansion
 // into W.  Both ends in natural order: the first pass loads, the second stores, along x.
 template <typename T, bool INV>
 __global__ void __launch_bounds__(kGenThreads, sizeof(T) == 4 ? 2 : 1)
@@ -356,11 +349,11 @@ k_gline_z(const GenShape s, const typename Cx<T>::type* __restrict__ tables, con
   C* tw = buf + H0 * s.H[2];
   copy_twiddles(tw, tables + s.tw[2], s.H[2]);
   pdl_enter();
-  const int y = blockIdx.x, c = blockIdx.y, slot = blockIdx.z;
+  const int y = blockIdx.x, c = blockIdx.y, f = blockIdx.z;
   const size_t plane = static_cast<size_t>(H0) * s.H[1];
   const size_t at = static_cast<size_t>(c) * s.hvol + static_cast<size_t>(y) * H0;
-  C* w = W + static_cast<size_t>(slot) * s.nch * s.hvol + at;
-  const C* rp = INV ? G0P + static_cast<size_t>(slot >> 1) * s.n_orbits * 2 + (slot & 1) : nullptr;
+  C* w = W + static_cast<size_t>(f) * s.nch * s.hvol + at;
+  const C* rp = INV ? G0P + static_cast<size_t>(f >> 1) * s.n_orbits * 2 + (f & 1) : nullptr;
   auto in = [&](int x, int z) {
     if constexpr (INV) return expand_point(ETP + at + z * plane + x, rp, tables + s.ph);
     else return w[z * plane + x];
@@ -378,14 +371,13 @@ k_gline_z(const GenShape s, const typename Cx<T>::type* __restrict__ tables, con
                            [&](int x, int j, int k, C v) { w[(j + A * k) * plane + x] = v; });
 }
 
-// Spectral-ASU gather from W: F(h) = sum_r e^{-2 pi i h.t_r / N} G0(R_r^T h mod M), the two
-// fields of the slot separated by X(q) and X(-q).  Indices are computed on the fly (h and R
-// are small, the moduli multiplications).
+// Spectral-ASU gather from W: F(h) = sum_r e^{-2 pi i h.t_r / N} G0(R_r^T h mod M).  Indices
+// are computed on the fly (h and R are small, the moduli multiplications).
 template <typename T>
 __global__ void __launch_bounds__(128)
 k_grecon(const GenShape s, const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
          const uint32_t* __restrict__ spec_h, const T* __restrict__ K, const typename Cx<T>::type* __restrict__ W,
-         typename Cx<T>::type* __restrict__ F, int nfields) {
+         typename Cx<T>::type* __restrict__ F) {
   using C = typename Cx<T>::type;
   __shared__ int sR[8][9], sT[8][3];
   const int D = s.d;
@@ -395,24 +387,22 @@ k_grecon(const GenShape s, const DevGeom* __restrict__ g, const typename Cx<T>::
     sT[i / 3][i % 3] = t < 0 ? t + s.N[i % 3] : t;
   }
   __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, slot = blockIdx.y, fa = 2 * slot;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, f = blockIdx.y;
   const uint32_t hp = __ldg(spec_h + min(i, s.n_spec - 1));
   pdl_enter();
   if (i >= s.n_spec) return;
   const int h[3] = {static_cast<int>(hp & 1023u), static_cast<int>((hp >> 10) & 1023u), static_cast<int>((hp >> 20) & 1023u)};
-  const C* Wb = W + static_cast<size_t>(slot) * s.nch * s.hvol;
+  const C* Wb = W + static_cast<size_t>(f) * s.nch * s.hvol;
   const int sh = s.centered ? 1 : 0;
-  const T half = static_cast<T>(0.5);
-  C acca = mk<C>(static_cast<T>(0), static_cast<T>(0)), accb = acca;
+  C acc = mk<C>(static_cast<T>(0), static_cast<T>(0));
 #pragma unroll 4
   for (int r = 0; r < D; ++r) {
-    int q[3], n[3], j = 0;
+    int q[3], j = 0;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       // |v| <= 3 x 1023; a multiple of M above that makes it positive
       const int v = sR[r][d] * h[0] + sR[r][3 + d] * h[1] + sR[r][6 + d] * h[2] + s.lift[d];
       q[d] = v - div_by(v, s.dM[d]) * s.M[d];
-      n[d] = q[d] ? s.M[d] - q[d] : 0;
       const int a = h[d] * sT[r][d];
       j += (a - div_by(a, s.dN[d]) * s.N[d]) * s.PN[d];
     }
@@ -425,14 +415,10 @@ k_grecon(const GenShape s, const DevGeom* __restrict__ g, const typename Cx<T>::
     }
     const C* Wc = Wb + static_cast<size_t>(c) * s.hvol;
     const C X = __ldg(Wc + (static_cast<size_t>(q[2] >> sh) * s.H[1] + (q[1] >> sh)) * s.H[0] + (q[0] >> sh));
-    const C Xn = __ldg(Wc + (static_cast<size_t>(n[2] >> sh) * s.H[1] + (n[1] >> sh)) * s.H[0] + (n[0] >> sh));
-    const C w = __ldg(tables + s.ph + j);
-    acca = cadd(acca, cmul(mk<C>(half * (X.x + Xn.x), half * (X.y - Xn.y)), w));
-    accb = cadd(accb, cmul(mk<C>(half * (X.y + Xn.y), half * (Xn.x - X.x)), w));
+    acc = cadd(acc, cmul(X, __ldg(tables + s.ph + j)));
   }
-  if (K) { const T k = K[i]; acca = cscale(acca, k); accb = cscale(accb, k); }
-  F[static_cast<size_t>(fa) * s.n_spec + i] = acca;
-  if (fa + 1 < nfields) F[static_cast<size_t>(fa + 1) * s.n_spec + i] = accb;
+  if (K) acc = cscale(acc, K[i]);
+  F[static_cast<size_t>(f) * s.n_spec + i] = acc;
 }
 
 inline int gen_threads(long items) {  // one butterfly or value per thread, in warps
@@ -458,33 +444,32 @@ Status gen_unit_launch(const FastArgs& a, const GenShape& s, std::string* err) {
   const uint32_t* et = static_cast<const uint32_t*>(a.expand);
   const C* rep = static_cast<const C*>(a.G0R);
   cudaStream_t st = static_cast<cudaStream_t>(a.stream);
-  const int nslots = (a.nb + 1) / 2;
   const size_t cs = sizeof(C);
   const size_t smem_p = (static_cast<size_t>(s.nch) * s.H[1] * s.S + s.H[0] + s.H[1]) * cs;
   const size_t smem_z = (static_cast<size_t>(s.H[0]) * s.H[2] + s.H[2]) * cs;
   const int thr_p = gen_threads(static_cast<long>(s.nch) * s.H[1] * s.B[0]);
   const int thr_z = gen_threads(static_cast<long>(s.H[0]) * s.B[2]);
-  const dim3 gp(s.H[2], nslots), gz(s.H[1], s.nch, nslots);
+  const dim3 gp(s.H[2], a.nb), gz(s.H[1], s.nch, a.nb);
   switch (a.stage) {
     case 0:
-      launch_k(k_gplane_fwd<T>, gp, thr_p, smem_p, st, s, tab, static_cast<const T*>(a.f0), static_cast<const T*>(a.E), W, a.nb);
+      launch_k(k_gplane_fwd<T>, gp, thr_p, smem_p, st, s, tab, static_cast<const T*>(a.f0), static_cast<const T*>(a.E), W);
       break;
     case 1:
       launch_k(k_gline_z<T, false>, gz, thr_z, smem_z, st, s, tab, nullptr, nullptr, W);
       break;
     case 2:
-      launch_k(k_grecon<T>, dim3((s.n_spec + 127) / 128, nslots), 128, 0, st, s, static_cast<const DevGeom*>(a.geom), tab,
-               static_cast<const uint32_t*>(a.spec_h), a.use_K ? static_cast<const T*>(a.K) : nullptr, W, static_cast<C*>(a.F), a.nb);
+      launch_k(k_grecon<T>, dim3((s.n_spec + 127) / 128, a.nb), 128, 0, st, s, static_cast<const DevGeom*>(a.geom), tab,
+               static_cast<const uint32_t*>(a.spec_h), a.use_K ? static_cast<const T*>(a.K) : nullptr, W, static_cast<C*>(a.F));
       break;
     case 4:
       launch_k(k_gline_z<T, true>, gz, thr_z, smem_z, st, s, tab, et, rep, W);
       break;
     default:
       if (s.H[2] == 1)
-        launch_k(k_gplane_bwd<T, true>, gp, thr_p, smem_p, st, s, tab, W, et, rep, static_cast<const T*>(a.E), static_cast<T*>(a.f0_out), a.nb);
+        launch_k(k_gplane_bwd<T, true>, gp, thr_p, smem_p, st, s, tab, W, et, rep, static_cast<const T*>(a.E), static_cast<T*>(a.f0_out));
       else
         launch_k(k_gplane_bwd<T, false>, gp, thr_p, smem_p, st, s, tab, W, nullptr, nullptr, static_cast<const T*>(a.E),
-                 static_cast<T*>(a.f0_out), a.nb);
+                 static_cast<T*>(a.f0_out));
       break;
   }
   const cudaError_t le = launch_error();
