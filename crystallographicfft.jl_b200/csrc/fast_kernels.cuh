@@ -1601,9 +1601,10 @@ template <typename C, int D> __device__ __forceinline__ void wht_d(C (&v)[D]) {
 // y = phase numerator j, F(q + M m) = e^{2 pi i j / P} F[x] (conjugated first where
 // flagged).  Outputs ([b][fiber]): x = orbit + 1 (0: none), y = phase numerator.
 //
-// Each spectrum value is read about once, so the gather reads F field by field as the
-// caller stores it: a warp takes 32 fibers of one workspace slot, whose taps are near
-// neighbours in the spectral order.  The slot inputs X = G_a + i G_b of the L slots of a
+// Each spectrum value is read once or twice (plain and conjugated taps make different fibers,
+// which neighbour one another), so the gather reads F field by field as the caller stores
+// it: a warp takes 32 fibers of one workspace slot, whose taps are near neighbours in the
+// spectral order.  The slot inputs X = G_a + i G_b of the L slots of a
 // group are exchanged through shared memory and leave as whole rows G0P[group][orbit][L]
 // for the expansion.  Im-3m 128^3 FP32, 64 fields: 7.5 + 15.0 us (regroup of the spectra
 // and one gather per orbit, 8 x the loads) before.

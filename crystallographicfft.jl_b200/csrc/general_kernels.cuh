@@ -6,10 +6,10 @@
 // complex transform: two fields as a + i b would halve the line transforms (GPU us of a round
 // trip, paired / alone: P6/mmm 60 x 60 x 80 FP64 x4 43 / 63, Im-3m 160^3 FP64 x8 91 / 119, p4mm
 // 160^2 FP64 x64 34 / 35), but the rounding error of one would then scale with the other, and a
-// NaN or the imaginary part of an inverse would cross over.  A line of n = A x B points is two in-place register passes
-// through one shared-memory buffer, the radices 2 to 16 chosen at run time; lengths that do
-// not split that way keep the Stockham kernels of exec.cu (out of place, a pass per factor up
-// to 8), which these replace: P6/mmm 60 x 60 x 80 FP64, 4 fields, plane kernels 45 / 47 us,
+// NaN or the imaginary part of an inverse would cross over.  A line of n = A x B points is two
+// in-place register passes through one shared-memory buffer, the radices 2 to 16 chosen at
+// run time; lengths that do not split that way keep the Stockham kernels of exec.cu (out of
+// place, a pass per factor up to 8), which these replace: P6/mmm 60 x 60 x 80 FP64, 4 fields, plane kernels 45 / 47 us,
 // z 25 / 25, inverse gather 33 before.
 #pragma once
 
