@@ -482,14 +482,19 @@ template <typename T> inline int plane_line_threads(int H, int nch, bool folded)
   return folded && rounds(base + 64) < rounds(base) && rounds(base + 64) <= 2 ? base + 64 : base;
 }
 
-// Registers of the forward plane kernel: its sixteen loads in flight take up to 130; below
-// H = 32 a cap of 112 keeps a block more on an SM (Ia-3d 96^3 contour steps, 256 fields x 20:
-// 3244 us without, 3115 with 112, 3151 with 96; Im-3m 128^3: 125.7 / 126.2 / 129.3).
-template <typename T, int H> constexpr int fold_registers() { return sizeof(T) == 4 && H < 32 ? 112 : 255; }
+// Registers of the forward plane kernel: with its sixteen loads in flight it takes 138 (FP32,
+// H = 32) without factors and 168 with them, three blocks of 128 threads on an SM; the factors are
+// a template parameter so that a plain transform does not carry them (as a run-time choice: 162
+// for both; FP64, H = 16, 166 instead of 114; forward us of Im-3m 128^3 FP32 x64 36.4 / 35.2,
+// 96^3 FP64 x135 66 / 60).  FP32 at H = 24 is capped at 112, one more block (forward us of Im-3m
+// 96^3 x135: 30.0 / 32.5 without, Ia-3d 96^3 x256: 50.1 / 54.4).  Not elsewhere: H = 8 then spills
+// (Im-3m 32^3 x256 8.3 / 7.3 without), H = 12 and 16 are even, and 128 at H = 32 is slower (Im-3m
+// 128^3 x128, three contour steps 674 / 659).
+template <typename T, int H> constexpr int fold_registers() { return sizeof(T) == 4 && H == 24 ? 112 : 255; }
 
 // Forward plane kernel, cubic H: fold (or plain load) of two fields + x FFT + y FFT
 // -> W[slot][c][z][y][x].
-template <typename T, int H, int CT>
+template <typename T, int H, int CT, bool UE>
 __global__ void __maxnreg__((fold_registers<T, H>())) k_plane_fwd_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
                               const T* __restrict__ f0, const T* __restrict__ E, typename Cx<T>::type* __restrict__ W,
                               int nfields) {
@@ -501,7 +506,7 @@ __global__ void __maxnreg__((fold_registers<T, H>())) k_plane_fwd_h(const DevGeo
   const int iz = blockIdx.x, slot = blockIdx.y;
   const int fa = 2 * slot;
   const bool has_b = fa + 1 < nfields;
-  const bool USE_E = E != nullptr;  // warp-uniform
+  constexpr bool USE_E = UE;
   const int tid = threadIdx.x, nth = blockDim.x;
   const size_t mvol = static_cast<size_t>(g->M[0]) * g->M[1] * g->M[2];
   const T* srca = f0 + static_cast<size_t>(fa) * mvol;
@@ -2224,7 +2229,8 @@ Status fast_unit_init(std::string* err) {
       if constexpr (GROUP == 0) {
         for (int ct = 0; ct < 5; ++ct) {
           CFFT_FOR_CT(ct, {
-            cudaFuncSetAttribute(k_plane_fwd_h<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
+            cudaFuncSetAttribute(k_plane_fwd_h<T, HH, CTT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
+            cudaFuncSetAttribute(k_plane_fwd_h<T, HH, CTT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
             cudaFuncSetAttribute(k_plane_bwd_h<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
             cudaFuncSetAttribute(k_plane_fwd_s<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
             cudaFuncSetAttribute(k_plane_bwd_s<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
@@ -2396,7 +2402,7 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
           if (!done && split)
             launch_k(k_plane_fwd_s<T, HH, CTT>, dim3(H, nslots), split_threads<HH, CTT>(), smem_plane + HH * cs, st, g, tab, f0, E, W, nb);
           else if (!done)
-            launch_k(k_plane_fwd_h<T, HH, CTT>, dim3(H, nslots), thr_plane, smem_plane, st, g, tab, f0, E, W, nb);
+            launch_k(E ? k_plane_fwd_h<T, HH, CTT, true> : k_plane_fwd_h<T, HH, CTT, false>, dim3(H, nslots), thr_plane, smem_plane, st, g, tab, f0, E, W, nb);
         });
       });
     } else {
