@@ -473,13 +473,17 @@ template <typename T, int H, int CT> constexpr int row_vec() {
 // two warps more where that saves the fold a round (H = 24: 144 items on 160 threads instead
 // of 96 or 128).  Measured, Ia-3d 96^3 FP32 contour steps of 256 fields, us for three: 637 /
 // 680 / 620 / 693 with 96 / 128 / 160 / 192 threads; Im-3m 64^3 FP32 round trips of 256
-// fields: 40.7 / 43.9 with 64 / 128; Pmmm 64^3 FP64, 256 fields: 217 / 229 with 64 / 128.
-template <typename T> inline int plane_line_threads(int H, int nch, bool folded) {
+// fields: 40.7 / 43.9 with 64 / 128; Pmmm 64^3 FP64, 256 fields: 217 / 229 with 64 / 128.  FP64,
+// forward + backward with / without the two warps: Im-3m 64^3 x64 27.7 / 31.9, 64^3 x256 69.2 /
+// 69.8, 48^3 x64 19.2 / 20.3, 96^3 x32 (384 blocks) 42.1 / 46.5, but 96^3 x135 (816 per lane)
+// 126.3 / 122.8 and three contour steps there 599 / 551: at H = 24 only up to four blocks per SM.
+template <typename T> inline int plane_line_threads(int H, int nch, bool folded, int ntasks) {
   constexpr int v = 16 / static_cast<int>(sizeof(T));
   const int base = std::max(64, ((nch * H + 31) / 32) * 32);
   const int items = H * H / (H % v == 0 ? v : 1);
   const auto rounds = [&](int t) { return (items + t - 1) / t; };
-  return folded && rounds(base + 64) < rounds(base) && rounds(base + 64) <= 2 ? base + 64 : base;
+  const bool fits = sizeof(T) == 4 || H < 24 || ntasks <= 4 * kSMs;
+  return folded && fits && rounds(base + 64) < rounds(base) && rounds(base + 64) <= 2 ? base + 64 : base;
 }
 
 // Registers of the forward plane kernel: with its sixteen loads in flight it takes 138 (FP32,
@@ -1372,9 +1376,9 @@ __global__ void __launch_bounds__(256) k_zr_weights(const DevGeom* __restrict__ 
 // Points: pts[i] = (spectral index, packed h); weights pq[2 sg][i] = Pw, pq[2 sg + 1][i] = Qw
 // of the four Hermitian tap pairs (sg, 7 - sg): looking the eight phases up per point instead costs
 // eight divergent table reads for values that every slot and both fields share.
-// SPLIT: lines of two passes (see split_pass1) instead of one line per thread, for FP64 and
-// H = 48, where a line per thread leaves 8 to 11 warps on an SM, and for small launches.
-template <typename T, int H> constexpr bool zr_split() { return sizeof(T) == 8 || H > 32; }
+// SPLIT: lines of two passes (see split_pass1) instead of one line per thread, for H = 48, where
+// a line per thread leaves 8 to 11 warps on an SM, and for small launches.
+template <int H> constexpr bool zr_split() { return H > 32; }
 template <int H, int SL, bool SPLIT> constexpr int zr_threads() {
   constexpr int n = SL * 2 * H * (SPLIT ? split_b<H>() : 1);
   return n <= 64 ? 64 : SPLIT && n > 256 ? 256 : ((n + 31) / 32) * 32;
@@ -2268,7 +2272,7 @@ Status fast_unit_init(std::string* err) {
         // share above 48 KB (FP64, 4 slots) needs the attribute, so failures are reported.
         {
           constexpr int kZr = kMaxDynSmemFast - 1024;
-          constexpr bool SP = zr_split<T, HH>();
+          constexpr bool SP = zr_split<HH>();
           cudaError_t ze = cudaFuncSetAttribute(k_fft_z_recon_diag8<T, HH, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kZr);
           if (ze == cudaSuccess) ze = cudaFuncSetAttribute(k_fft_z_recon_diag8<T, HH, 2, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kZr);
           if (ze == cudaSuccess) ze = cudaFuncSetAttribute(k_fft_z_recon_diag8<T, HH, 4, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kZr);
@@ -2362,9 +2366,9 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
       if (ce != cudaSuccess) return fast_cuda(ce, "fused cluster launch", err);
       return fast_cuda(cudaGetLastError(), "fused cluster launch", err);
     }
-    const int thr_plane = plane_line_threads<T>(H, nch, a.cent_type != 0);
-    const size_t smem_plane = static_cast<size_t>(nch) * H * (H + 1) * cs;
     const int ntasks = nslots * H;
+    const int thr_plane = plane_line_threads<T>(H, nch, a.cent_type != 0, ntasks);
+    const size_t smem_plane = static_cast<size_t>(nch) * H * (H + 1) * cs;
     // Split lines while the launch has at most one CTA per SM: then the length of a thread's
     // chain counts, beyond that the extra shared-memory passes do.  Ia-3d 96^3 FP32, three
     // contour steps of 2 / 32 fields: 69 / 140 us against 84 / 140 with a line per thread; of
@@ -2470,19 +2474,24 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
       }
       case 6: {
         // Fused z FFT + diagonal-sign gather.  One slot per CTA (split lines) while that
-        // gives at most two CTAs per SM; else 4 slots per CTA in FP32 (2 on request).  FP64 and
-        // H = 48 split their lines: 2 slots where the units hold many points, whose weights the
-        // slots share (Pmmm 64^3 FP64, 256 fields, round trip: 211 / 212 / 218 us with 2 / 1 / 4), 1
-        // else (Im-3m 96^3 FP64, 64 fields: 64.3 / 66.9 / 67.5 with 1 / 2 / 4).
+        // gives at most two CTAs per SM, else four (two on request), one line per thread.  FP64 below
+        // H = 24, whose blocks of four slots are 64 to 128 threads, changes over at 2048 CTAs of one
+        // slot (forward us with 1 / 4 slots: Im-3m 48^3 x64, 896 CTAs, 7.8 / 10.6; 64^3 x64, 1152, 10.6 /
+        // 13.3; Fm-3m 64^3 x256, 2304, 22.8 / 21.8; Im-3m 48^3 x256, 3584, 18.6 / 16.4; from H = 24 on
+        // 4 slots are ahead at every size: Im-3m 96^3 x135 61.6 / 45.3, Pm-3m 48^3 x256 29.3 / 24.3).
+        // H = 48: 2 split slots where the units hold many points, whose weights the slots share,
+        // else 1.
         const T* K = a.use_K ? static_cast<const T*>(a.K) : nullptr;
         const uint4* un = static_cast<const uint4*>(a.zr_units);
         const uint2* pt = static_cast<const uint2*>(a.zr_pts);
         const C* pq = static_cast<const C*>(a.zr_pq);
         const C* Wc = W;
         CFFT_FOR_H(H, {
-          constexpr bool SP = zr_split<T, HH>();
+          constexpr bool SP = zr_split<HH>();
+          const int one = a.zr_n_units * nslots;  // CTAs of one slot
           const int sl = a.zr_slots == 2 || a.zr_slots == 4 ? a.zr_slots
-                         : a.zr_n_units * nslots <= 2 * kSMs ? 1 : SP ? (a.n_spec_pts > 512 * a.zr_n_units ? 2 : 1) : zr_slots();
+                         : one <= 2 * kSMs || (sizeof(T) == 8 && HH < 24 && one < 2048) ? 1
+                         : SP ? (a.n_spec_pts > 512 * a.zr_n_units ? 2 : 1) : zr_slots();
           const size_t sm = (static_cast<size_t>(sl) * 2 * HH * (HH + 1) + HH) * cs;
           const dim3 gzr(a.zr_n_units, (nslots + sl - 1) / sl);
           if (sl == 1)
