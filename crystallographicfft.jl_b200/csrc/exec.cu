@@ -1196,16 +1196,25 @@ Status plan_device_init(Plan* p, std::string* err) {
   if (p->tune.chunk_bytes > 0) budget = static_cast<size_t>(p->tune.chunk_bytes);
   const size_t per_field = T.n_ch * hvol * cs / (p->fast_h ? 2 : 1);
   size_t ch = std::max<size_t>(1, std::min<size_t>(B, budget / std::max<size_t>(per_field, 1)));
-  // Two concurrent lanes once the batch's channel workspace reaches 48 MiB: below, one lane
-  // fills the SMs and a second doubles the launches.  Measured with one / two lanes, us per
-  // round trip: Im-3m 128^3 FP32 32 fields (16 MiB) 59 / 61, 128 fields (64 MiB) 150 / 128;
-  // Pmmm 64^3 FP64 64 fields (16 MiB) 69 / 83, 256 fields (64 MiB) 246 / 218; P6/mmm 60 x 60 x 80
-  // FP64 16 fields (35 MiB) 122 / 123, 32 fields (70 MiB) 244 / 222.
+  // Two concurrent lanes from 24 MiB of channel workspace on the compile-time sizes: below, a
+  // second lane doubles the launches of a batch that one fills the SMs with.  us of a plain round
+  // trip / of one step of a contour loop with one and two lanes: Im-3m FP32 128^3 x64 (32 MiB)
+  // 92 / 125 and 78 / 101, x32 (16) 57 / 63 and 58 / 63, 192^3 x16 (27) 87 / 108 and 85 / 96, 64^3
+  // x256 (16) 43 / 48 and 50 / 46; FP64 128^3 x32 (32) 93 / 124 and 85 / 108, Pm-3m 64^3 x128 (32) 77 /
+  // 88 and 72 / 74, 64^3 x64 (16) 41 / 44 and 47 / 46.  The general kernels' launches are longer
+  // for their workspace and change over at 8 MiB (GPU us of a round trip with one and two): P6/mmm
+  // 60 x 60 x 80 FP64 x4 (18 MiB) 63 and 59, Im-3m 160^3 FP64 x8 (32) 119 and 114, P2_13 40^3 FP32
+  // x128 (8) 79 and 75, Im-3m 40^3 FP32 x128 (4) 35 and 36, Pm-3m 20^3 FP32 x128 (1) 21 and 24.
   p->lanes = 1;
   if (p->tune.lanes > 0) p->lanes = std::min(Plan::kMaxLanes, p->tune.lanes);
   else if (const char* ln = std::getenv("CFFT_LANES")) p->lanes = std::max(1, std::min(Plan::kMaxLanes, std::atoi(ln)));
-  else if (tables && B >= 8 && B * per_field >= (static_cast<size_t>(48) << 20)) p->lanes = 2;
-  if (p->lanes > 1) ch = std::min(ch, (B + p->lanes - 1) / p->lanes);
+  else if (p->fast_h ? B >= 8 && B * per_field >= (static_cast<size_t>(24) << 20)
+                     : p->general && B >= 4 && B * per_field >= (static_cast<size_t>(8) << 20)) p->lanes = 2;
+  if (p->lanes > 1) {  // whole pairs of fields, no lane left with a remainder
+    size_t per = (B + p->lanes - 1) / p->lanes;
+    if (p->fast_h) per += per & 1;
+    ch = std::min(ch, per);
+  }
   if (p->fast_h && ch < B && ch > 1) ch &= ~static_cast<size_t>(1);
   p->chunk = static_cast<int>(ch);
   // launch geometry and shared memory (generic path)
