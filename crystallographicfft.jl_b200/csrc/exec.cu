@@ -1260,13 +1260,21 @@ Status plan_device_init(Plan* p, std::string* err) {
     if ((st = alloc(&p->d_expand, expand.size() * (p->reps_quad ? 4 : sizeof(int2)), "expansion table")) != Status::kOk)
       return st;
     // Rows of 64 bytes (8 FP32 / 4 FP64 slots) once a chunk fills one; the fused cluster
-    // kernels read rows of 2 slots, so CFFT_CLUSTER keeps those.
+    // kernels read rows of 2 slots, so CFFT_CLUSTER keeps those.  So do launches of the
+    // expansion with few blocks from H = 32 on, where a block of full rows takes 64 KB of
+    // shared memory: up to half an SM count of blocks (backward GPU us, rows of 2 / full rows: Pm-3m
+    // 64^3 FP32 x16, 32 blocks, 10.4 / 13.2; Im-3m 128^3 x16, 128 blocks, 25.9 / 23.7; P1 32^3 FP64 x16,
+    // 64 blocks, 14.5 / 19.5, x64, 256 blocks, 34.9 / 27.2), in FP64 with several aliases per
+    // fiber two blocks per SM (Pm-3m 64^3 x64, 256 blocks, 23.7 / 26.7; Im-3m 128^3 x8, 128 blocks, 21.0 / 22.7,
+    // x32 in two lanes 39.5 / 41.7).
     const size_t gw = 128 / cs;
     const char* wide_env = std::getenv("CFFT_WIDE");
     const char* cl_env = std::getenv("CFFT_CLUSTER");
     const bool cluster_wanted = p->tune.cluster >= 0 ? p->tune.cluster > 0 : (cl_env && std::atoi(cl_env) > 0);
     const bool wide_wanted = p->tune.wide >= 0 ? p->tune.wide > 0 : !(wide_env && wide_env[0] == '0');
-    p->reps_wide = p->fast_h && p->reps_quad && chunk >= gw && wide_wanted && !cluster_wanted;
+    const size_t groups = (chunk + gw - 1) / gw;
+    const bool few = p->fast_h >= 32 && 2 * T.n_ch * p->fast_h * groups <= (p->precision == 8 && T.d > 1 ? 4u : 1u) * 148u;
+    p->reps_wide = p->fast_h && p->reps_quad && chunk >= gw && !few && wide_wanted && !cluster_wanted;
     const size_t chunk4 = p->reps_wide ? (chunk + gw - 1) / gw * gw : (chunk + 3) / 4 * 4;  // whole rows of slots
     p->g0r_lane_bytes = (((p->reps_quad ? chunk4 : chunk + 1) * T.orbit_rep.size() * cs + 255) / 256) * 256;
     if ((st = alloc(&p->d_g0r, p->lanes * p->g0r_lane_bytes, "representative workspace")) != Status::kOk) return st;
