@@ -688,7 +688,7 @@ Status build_zrecon_units(Plan* p, std::string* err) {
 template <typename T>
 Status launch_stage(Plan* p, int stage, const T* f0, typename Cx<T>::type* F, const typename Cx<T>::type* Fin,
                     T* f0_out, const T* E, bool use_K, int nb, cudaStream_t st, std::string* err, int lane = 0,
-                    bool q_step = false) {
+                    bool q_step = false, int lanes = 1) {
   using C = typename Cx<T>::type;
   const DevGeom* g = static_cast<const DevGeom*>(p->d_geom);
   const C* tab = static_cast<const C*>(p->d_tables);
@@ -705,6 +705,7 @@ Status launch_stage(Plan* p, int stage, const T* f0, typename Cx<T>::type* F, co
     a.G0R = p->d_g0r ? static_cast<char*>(p->d_g0r) + lane * p->g0r_lane_bytes : nullptr;
     a.f0 = f0; a.F = F; a.Fin = Fin; a.f0_out = f0_out; a.E = E;
     a.slot_fields = p->general ? 1 : 2;
+    a.lanes = lanes;
     a.stage = stage; a.nb = nb; a.H = p->fast_h; a.n_ch = T_.n_ch; a.centered = T_.centered ? 1 : 0;
     a.cent_type = p->cent_type; a.d = T_.d;
     a.n_spec = static_cast<int>(T_.spec.size()); a.n_orbits = static_cast<int>(T_.orbit_rep.size());
@@ -806,7 +807,7 @@ Status run_chunks(Plan* p, bool fwd, bool bwd, const T* f0, typename Cx<T>::type
       for (int s : {0, 1, 4, 5}) {
         if (p->qsep && s == 1) continue;
         if (p->qsep && s == 4) s = 7;
-        Status r = launch_stage<T>(p, s, fin, Fc, Fc, fout, Ec, false, nb, ls, err, lane, true);
+        Status r = launch_stage<T>(p, s, fin, Fc, Fc, fout, Ec, false, nb, ls, err, lane, true, lanes);
         if (r != Status::kOk) return r;
       }
       continue;
@@ -814,12 +815,12 @@ Status run_chunks(Plan* p, bool fwd, bool bwd, const T* f0, typename Cx<T>::type
     if (fwd)
       for (int s : {0, 1, 2}) {
         if (p->zrecon && s == 1) continue;  // stage 6 = z FFT + gather
-        Status r = launch_stage<T>(p, p->zrecon && s == 2 ? 6 : s, fin, Fc, nullptr, nullptr, Ec, use_K, nb, ls, err, lane);
+        Status r = launch_stage<T>(p, p->zrecon && s == 2 ? 6 : s, fin, Fc, nullptr, nullptr, Ec, use_K, nb, ls, err, lane, false, lanes);
         if (r != Status::kOk) return r;
       }
     if (bwd)
       for (int s = 3; s < 6; ++s) {
-        Status r = launch_stage<T>(p, s, nullptr, nullptr, Fc, fout, Ec, false, nb, ls, err, lane);
+        Status r = launch_stage<T>(p, s, nullptr, nullptr, Fc, fout, Ec, false, nb, ls, err, lane, false, lanes);
         if (r != Status::kOk) return r;
       }
   }

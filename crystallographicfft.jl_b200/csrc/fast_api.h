@@ -31,6 +31,7 @@ struct FastArgs {
   const void* E = nullptr;
   // geometry / dispatch
   int slot_fields = 2;    // fields per workspace slot (1: general kernels)
+  int lanes = 1;          // chunks that run concurrently with this one, itself included
   int stage = 0, nb = 0, H = 0, n_ch = 1, centered = 0, cent_type = 0, d = 1;
   int n_spec = 0, n_orbits = 0;
   bool use_K = false, rep_diag8 = false, rep_perm = false, reps_quad = false;

@@ -2369,12 +2369,18 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
     const int ntasks = nslots * H;
     const int thr_plane = plane_line_threads<T>(H, nch, a.cent_type != 0, ntasks);
     const size_t smem_plane = static_cast<size_t>(nch) * H * (H + 1) * cs;
-    // Split lines while the launch has at most one CTA per SM: then the length of a thread's
-    // chain counts, beyond that the extra shared-memory passes do.  Ia-3d 96^3 FP32, three
-    // contour steps of 2 / 32 fields: 69 / 140 us against 84 / 140 with a line per thread; of
-    // Im-3m 128^3, 32 fields (256 CTAs): 58.9 against 56.5.  Above H = 32 the plane takes a
-    // whole SM either way and the split loses at every size.
-    const bool split = ntasks <= kSMs && H <= 32;
+    // Split lines while the launch has at most one CTA per SM, or as few lines as half the
+    // SMs' blocks of 128: then the length of a thread's chain counts, beyond that the extra
+    // shared-memory passes do.  GPU us of three contour steps, split / a line per thread: Ia-3d
+    // 96^3 FP32 x2 / x32, 69 / 84 and 140 / 140; Pm-3m 48^3 FP32 x16 (192 CTAs, 4608 lines) 47 / 55, Fm-3m
+    // 96^3 FP64 x16 (192, 9216) 89 / 100, but 96^3 FP32 x32 (384, 18432) 109 / 106, Im-3m 96^3 FP64 x16 (192,
+    // 18432) 114 / 105.  FP64 folds at H = 32, whose lines take 150 registers, gain from it for twice the
+    // lines of one CTA per SM, in all lanes: Im-3m 128^3 x16 (256, 32768) 188 / 226, Fm-3m 128^3 x32 (512,
+    // 32768) 271 / 359, Im-3m 128^3 x32 (two lanes) forward + backward 90 / 76.  Above H = 32 the plane
+    // takes a whole SM either way and the split loses at every size.
+    const int lines = ntasks * nch * H;
+    const bool split = H <= 32 && (ntasks <= kSMs || lines <= kSMs * 64 ||
+                                   (sizeof(T) == 8 && H == 32 && a.cent_type != 0 && a.lanes * lines <= kSMs * 256));
     auto al16 = [](const void* p) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     const int tmode = a.tma >= 0 ? a.tma : tma_mode();
     const bool tma = al16(f0) && al16(E) && al16(f0_out) && al16(W) && (tmode & (a.stage == 0 ? 1 : 2));
