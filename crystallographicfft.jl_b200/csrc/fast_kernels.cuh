@@ -298,9 +298,14 @@ __device__ __forceinline__ void fold_plane(const DevGeom* __restrict__ g, const 
 // v / V for the inverse transform's normalisation.  1/V rounded to FP32 is off by 7.5e-9
 // for edges with a factor 3, the same way in every step of a contour loop (7.5e-7 after a
 // hundred); its remainder as a second term makes the product correct to a rounding, which
-// does not accumulate.  Powers of two have no remainder.
+// does not accumulate.  Powers of two have no remainder.  The first term is rounded down, so
+// that the remainder is positive and an overflowed sum stays infinite (inf - inf would be NaN).
+template <typename T> constexpr T round_down(double x) {  // x in the normal range
+  const T r = static_cast<T>(x);
+  return static_cast<double>(r) > x ? static_cast<T>(x * (1.0 - 0x1p-24)) : r;
+}
 template <typename T, int V> __device__ __forceinline__ T div_const(T v) {
-  constexpr T hi = static_cast<T>(1.0 / V);
+  constexpr T hi = round_down<T>(1.0 / V);
   constexpr T lo = sizeof(T) == 4 ? static_cast<T>(1.0 / V - static_cast<double>(hi)) : static_cast<T>(0);
   if constexpr (lo == static_cast<T>(0)) return v * hi;
   else return fma(v, hi, v * lo);

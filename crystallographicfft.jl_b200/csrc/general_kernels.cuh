@@ -297,10 +297,11 @@ k_gplane_bwd(const GenShape s, const typename Cx<T>::type* __restrict__ tables, 
   }
   T* dst = f0 + static_cast<size_t>(f) * s.mvol;
   const T* Ef = E ? E + static_cast<size_t>(f) * s.mvol : nullptr;
-  // v / V as two terms: the rounding error of 1 / V alone accumulates over a contour loop.
-  const T hi = static_cast<T>(s.inv_v), lo = static_cast<T>(s.inv_v - static_cast<double>(hi));
+  // v / V as two terms, the first rounded down: see div_const.
+  const T hi = sizeof(T) == 4 ? static_cast<T>(__double2float_rd(s.inv_v)) : static_cast<T>(s.inv_v);
+  const T lo = static_cast<T>(s.inv_v - static_cast<double>(hi));
   auto put = [&](int idx, T v) {
-    T a = fma(v, hi, v * lo);
+    T a = lo == static_cast<T>(0) ? v * hi : fma(v, hi, v * lo);
     if (Ef) a *= __ldg(Ef + idx);
     __stcs(dst + idx, a);
   };
