@@ -7,7 +7,7 @@ time on the CPU.  They serve batches of fields of uneven space group and grid si
 * autotune_plan times candidate execution choices (cfft_tuning: chunk size, lanes,
   fused-z slots per CTA, the rows of the backward gather, the bulk-copy plane kernels, the
   fused cluster kernels) on the device with CUDA events, by coordinate descent from the
-  defaults, and caches the winner in a JSON file keyed by device, operations, grid,
+  defaults, and caches the winner in a JSON file keyed by device, library, operations, grid,
   precision, batch, operation and path; autotune_path also chooses the decomposition
   (centring fold, plain stride-L, Q-matrix steps).
 * MultiPlanStep runs one callable per plan, each on its own stream forked from and
@@ -17,13 +17,14 @@ time on the CPU.  They serve batches of fields of uneven space group and grid si
 """
 from __future__ import annotations
 
+import functools
 import hashlib
 import json
 import os
 
 import numpy as np
 
-from ._lib import CFFTError
+from ._lib import LIB_PATH, CFFTError
 from .plans import KRFFTPlan, _torch
 
 KNOBS = (
@@ -47,6 +48,19 @@ def _ops_signature(ops):
         h.update(np.asarray(op.R, dtype=np.int64).tobytes())
         h.update(np.asarray(op.t, dtype=np.int64).tobytes())
     return h.hexdigest()[:12]
+
+
+@functools.lru_cache(maxsize=None)
+def _library_signature(path):
+    """Digest of the library file: choices tuned on other kernels are not this library's."""
+    with open(path, "rb") as fh:
+        return hashlib.file_digest(fh, "sha1").hexdigest()[:12]
+
+
+def _cache_key(device, library, ops, N, precision, batch, op, n_steps, path, knobs):
+    return "|".join([device, library, _ops_signature(ops), "x".join(map(str, N)), str(precision), str(batch), op,
+                     str(n_steps), str(path),
+                     hashlib.sha1(repr(tuple((k, tuple(v)) for k, v in knobs)).encode()).hexdigest()[:8]])
 
 
 def _time_op(plan, op, batch, n_steps, reps):
@@ -89,9 +103,8 @@ def autotune_plan(spec, ops_shifted, *, N=None, precision=4, batch=1, op="fwdbwd
     torch = _torch()
     N = tuple(spec.N if N is None else N)
     cache_path = cache_path or _default_cache()
-    key = "|".join([torch.cuda.get_device_name(), _ops_signature(ops_shifted), "x".join(map(str, N)), str(precision),
-                    str(batch), op, str(n_steps), str(path),
-                    hashlib.sha1(repr(tuple((k, tuple(v)) for k, v in knobs)).encode()).hexdigest()[:8]])
+    key = _cache_key(torch.cuda.get_device_name(), _library_signature(LIB_PATH), ops_shifted, N, precision, batch, op,
+                     n_steps, path, knobs)
     cache = {}
     if os.path.exists(cache_path):
         try:
