@@ -456,7 +456,7 @@ __global__ void k_block_scale(const int32_t* __restrict__ dims, const long long*
 // along x.
 template <typename T>
 __global__ void __launch_bounds__(256) k_full_to_sub(const T* __restrict__ u, T* __restrict__ f0, int N1, int N2, int L1, int L2,
-                                                     int L3, int M1, int M2, int M3, size_t mvol, size_t nvol) {
+                                                     int L3, int M1, int M2, size_t mvol, size_t nvol) {
   const int y = blockIdx.x * blockDim.y + threadIdx.y, z = blockIdx.y, b = blockIdx.z;
   if (y >= M2) return;
   const T* src = u + b * nvol + (static_cast<size_t>(z) * L3 * N2 + static_cast<size_t>(y) * L2) * N1;
@@ -699,7 +699,7 @@ Status launch_stage(Plan* p, int stage, const T* f0, typename Cx<T>::type* F, co
     if (p->cluster && (stage == 1 || stage == 4)) return Status::kOk;  // fused into stages 0 and 5
     FastArgs a;
     a.geom = p->d_geom; a.tables = p->d_tables; a.spec_h = p->d_spec_h; a.K = p->d_K;
-    a.inv_spec = p->d_inv_spec; a.inv_phase = p->d_inv_phase; a.expand = p->d_expand;
+    a.expand = p->d_expand;
     a.fib_taps = p->d_fib_taps; a.fib_outs = p->d_fib_outs; a.n_fib = p->n_fib;
     a.W = W;
     a.G0R = p->d_g0r ? static_cast<char*>(p->d_g0r) + lane * p->g0r_lane_bytes : nullptr;
@@ -709,7 +709,7 @@ Status launch_stage(Plan* p, int stage, const T* f0, typename Cx<T>::type* F, co
     a.stage = stage; a.nb = nb; a.H = p->fast_h; a.n_ch = T_.n_ch; a.centered = T_.centered ? 1 : 0;
     a.cent_type = p->cent_type; a.d = T_.d;
     a.n_spec = static_cast<int>(T_.spec.size()); a.n_orbits = static_cast<int>(T_.orbit_rep.size());
-    a.use_K = use_K; a.rep_diag8 = p->rep_diag8; a.rep_perm = p->rep_perm; a.reps_quad = p->reps_quad;
+    a.use_K = use_K; a.rep_diag8 = p->rep_diag8; a.rep_perm = p->rep_perm;
     a.reps_wide = p->reps_wide && !p->cluster;
     a.zr_units = p->d_zr_units; a.zr_pts = p->d_zr_pts; a.zr_pq = p->d_zr_pq; a.n_spec_pts = p->zr_npts; a.zr_n_units = p->zr_units;
     a.cluster = p->cluster;
@@ -1127,9 +1127,12 @@ Status plan_device_init(Plan* p, std::string* err) {
   if (const char* f = std::getenv("CFFT_DISABLE_FAST")) {
     if (f[0] == '1') p->fast_h = 0;
   }
-  // General kernels: every axis length splits into two register radices, and the packed
-  // tables fit (the conditions of reps_quad below).
-  p->general = !p->fast_h && T.spec.size() < (1u << 20) - 1 && T.P <= 2048 && T.orbit_rep.size() < (1u << 21);
+  // Packed tables: spectral index + 1 in 21 bits, orbit | phase << 21.  The compile-time sizes
+  // (at most 192 points an axis, 96^3 channel points) are far inside the limits.
+  const bool packed = T.spec.size() < (1u << 20) - 1 && T.P <= 2048 && T.orbit_rep.size() < (1u << 21);
+  if (!packed) p->fast_h = 0;
+  // General kernels: every axis length splits into two register radices, and the tables fit.
+  p->general = !p->fast_h && packed;
   for (int d = 0; d < 3 && p->general; ++d) p->general = general_split(T.H[d], &p->gen.A[d], &p->gen.B[d]);
   const size_t hvol = static_cast<size_t>(T.H[0]) * T.H[1] * T.H[2];
   const bool tables = p->fast_h || p->general;
@@ -1239,8 +1242,8 @@ Status plan_device_init(Plan* p, std::string* err) {
   if ((st = alloc(&p->d_tables, tab.size(), "tables")) != Status::kOk) return st;
   if ((st = alloc(&p->d_spec_h, hp.size() * 4, "spectral points")) != Status::kOk) return st;
   if ((st = alloc(&p->d_K, T.spec.size() * rs, "kernel")) != Status::kOk) return st;
-  p->reps_quad = tables && T.spec.size() < (1u << 20) - 1 && T.P <= 2048 && T.orbit_rep.size() < (1u << 21);
-  if (!p->reps_quad) {  // the fibers replace these
+  p->reps_quad = tables;
+  if (!tables) {  // the fibers replace these
     if ((st = alloc(&p->d_orbit_rep, T.orbit_rep.size() * 4, "orbit reps")) != Status::kOk) return st;
     if ((st = alloc(&p->d_inv_spec, T.inv_spec.size() * 4, "inverse spec")) != Status::kOk) return st;
     if ((st = alloc(&p->d_inv_phase, T.inv_phase.size() * 4, "inverse phase")) != Status::kOk) return st;
@@ -1251,15 +1254,13 @@ Status plan_device_init(Plan* p, std::string* err) {
   if ((st = alloc(&p->d_work_F, B * T.spec.size() * cs, "spectrum workspace")) != Status::kOk) return st;
   if ((st = alloc(&p->d_work_E, B * mvol * rs, "interaction workspace")) != Status::kOk) return st;
   std::vector<uint2> fib_taps, fib_outs;
-  if (p->reps_quad) {
+  if (tables) {
     p->n_fib = build_fibers(T, expand, &fib_taps, &fib_outs);
     if ((st = alloc(&p->d_fib_taps, fib_taps.size() * sizeof(uint2), "fiber taps")) != Status::kOk) return st;
     if ((st = alloc(&p->d_fib_outs, fib_outs.size() * sizeof(uint2), "fiber outputs")) != Status::kOk) return st;
   }
   if (tables) {
-    // Packed expansion entries (orbit | phase << 21) where they fit 32 bits.
-    if ((st = alloc(&p->d_expand, expand.size() * (p->reps_quad ? 4 : sizeof(int2)), "expansion table")) != Status::kOk)
-      return st;
+    if ((st = alloc(&p->d_expand, expand.size() * 4, "expansion table")) != Status::kOk) return st;
     // Rows of 64 bytes (8 FP32 / 4 FP64 slots) once a chunk fills one; the fused cluster
     // kernels read rows of 2 slots, so CFFT_CLUSTER keeps those.  So do launches of the
     // expansion with few blocks from H = 32 on, where a block of full rows takes 64 KB of
@@ -1275,9 +1276,9 @@ Status plan_device_init(Plan* p, std::string* err) {
     const bool wide_wanted = p->tune.wide >= 0 ? p->tune.wide > 0 : !(wide_env && wide_env[0] == '0');
     const size_t groups = (chunk + gw - 1) / gw;
     const bool few = p->fast_h >= 32 && 2 * T.n_ch * p->fast_h * groups <= (p->precision == 8 && T.d > 1 ? 4u : 1u) * 148u;
-    p->reps_wide = p->fast_h && p->reps_quad && chunk >= gw && !few && wide_wanted && !cluster_wanted;
+    p->reps_wide = p->fast_h && chunk >= gw && !few && wide_wanted && !cluster_wanted;
     const size_t chunk4 = p->reps_wide ? (chunk + gw - 1) / gw * gw : (chunk + 3) / 4 * 4;  // whole rows of slots
-    p->g0r_lane_bytes = (((p->reps_quad ? chunk4 : chunk + 1) * T.orbit_rep.size() * cs + 255) / 256) * 256;
+    p->g0r_lane_bytes = ((chunk4 * T.orbit_rep.size() * cs + 255) / 256) * 256;
     if ((st = alloc(&p->d_g0r, p->lanes * p->g0r_lane_bytes, "representative workspace")) != Status::kOk) return st;
   }
   // Q-matrix step (M2Q / M7): runs on the compile-time sized kernels only.
@@ -1339,20 +1340,18 @@ Status plan_device_init(Plan* p, std::string* err) {
   CFFT_CUDA(cudaMemcpy(p->d_geom, &g, sizeof(g), cudaMemcpyHostToDevice), "upload geometry");
   CFFT_CUDA(cudaMemcpy(p->d_tables, tab.data(), tab.size(), cudaMemcpyHostToDevice), "upload tables");
   CFFT_CUDA(cudaMemcpy(p->d_spec_h, hp.data(), hp.size() * 4, cudaMemcpyHostToDevice), "upload spectral points");
-  if (!T.orbit_rep.empty() && !p->reps_quad) {
+  if (!T.orbit_rep.empty() && !tables) {
     CFFT_CUDA(cudaMemcpy(p->d_orbit_rep, T.orbit_rep.data(), T.orbit_rep.size() * 4, cudaMemcpyHostToDevice), "upload reps");
     CFFT_CUDA(cudaMemcpy(p->d_inv_spec, T.inv_spec.data(), T.inv_spec.size() * 4, cudaMemcpyHostToDevice), "upload inv spec");
     CFFT_CUDA(cudaMemcpy(p->d_inv_phase, T.inv_phase.data(), T.inv_phase.size() * 4, cudaMemcpyHostToDevice), "upload inv phase");
     if (!masks.empty())
       CFFT_CUDA(cudaMemcpy(p->d_img_mask, masks.data(), masks.size() * 4, cudaMemcpyHostToDevice), "upload masks");
   }
-  if (p->reps_quad) {
+  if (tables) {
     std::vector<uint32_t> epk(expand.size());
     for (size_t i = 0; i < expand.size(); ++i)
       epk[i] = static_cast<uint32_t>(expand[i].x) | (static_cast<uint32_t>(expand[i].y) << 21);
     CFFT_CUDA(cudaMemcpy(p->d_expand, epk.data(), epk.size() * 4, cudaMemcpyHostToDevice), "upload expansion");
-  } else if (p->fast_h) {
-    CFFT_CUDA(cudaMemcpy(p->d_expand, expand.data(), expand.size() * sizeof(int2), cudaMemcpyHostToDevice), "upload expansion");
   }
   if (p->n_fib) {
     CFFT_CUDA(cudaMemcpy(p->d_fib_taps, fib_taps.data(), fib_taps.size() * sizeof(uint2), cudaMemcpyHostToDevice), "upload fiber taps");
@@ -1383,7 +1382,7 @@ Status plan_device_init(Plan* p, std::string* err) {
     const char* ce = std::getenv("CFFT_CLUSTER");
     const int want = p->tune.cluster >= 0 ? p->tune.cluster : (ce ? std::atoi(ce) : 0);
     p->cluster_ctas = want == 16 ? 16 : 8;
-    p->cluster = want != 0 && !p->qmode && p->reps_quad && fast_cluster_fits(p->fast_h, T.n_ch, p->precision);
+    p->cluster = want != 0 && !p->qmode && fast_cluster_fits(p->fast_h, T.n_ch, p->precision);
     if (p->cluster) {
       int mc = 0;
       st = p->precision == 8 ? fast_cluster_probe_f64(p->fast_h, p->cent_type, p->cluster_ctas, &mc, err)
@@ -1717,10 +1716,10 @@ Status exec_full_to_sub(Plan* p, const void* u, void* f0, int B, void* stream, s
     const dim3 grid((T.M[1] + blk.y - 1) / blk.y, T.M[2], std::min(B - b0, 65535));
     if (p->precision == 8)
       k_full_to_sub<double><<<grid, blk, 0, s>>>(static_cast<const double*>(u) + b0 * nvol, static_cast<double*>(f0) + b0 * mvol,
-                                                 T.N[0], T.N[1], T.L[0], T.L[1], T.L[2], T.M[0], T.M[1], T.M[2], mvol, nvol);
+                                                 T.N[0], T.N[1], T.L[0], T.L[1], T.L[2], T.M[0], T.M[1], mvol, nvol);
     else
       k_full_to_sub<float><<<grid, blk, 0, s>>>(static_cast<const float*>(u) + b0 * nvol, static_cast<float*>(f0) + b0 * mvol,
-                                                T.N[0], T.N[1], T.L[0], T.L[1], T.L[2], T.M[0], T.M[1], T.M[2], mvol, nvol);
+                                                T.N[0], T.N[1], T.L[0], T.L[1], T.L[2], T.M[0], T.M[1], mvol, nvol);
   }
   ++g_launches;
   CFFT_CUDA(cudaGetLastError(), "fullgrid_to_subgrid launch");

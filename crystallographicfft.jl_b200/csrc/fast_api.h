@@ -15,8 +15,6 @@ struct FastArgs {
   const void* tables = nullptr;
   const void* spec_h = nullptr;
   const void* K = nullptr;
-  const void* inv_spec = nullptr;
-  const void* inv_phase = nullptr;
   const void* fib_taps = nullptr;  // inverse gather by fibers: taps and outputs (uint2)
   const void* fib_outs = nullptr;
   int n_fib = 0;
@@ -34,7 +32,7 @@ struct FastArgs {
   int lanes = 1;          // chunks that run concurrently with this one, itself included
   int stage = 0, nb = 0, H = 0, n_ch = 1, centered = 0, cent_type = 0, d = 1;
   int n_spec = 0, n_orbits = 0;
-  bool use_K = false, rep_diag8 = false, rep_perm = false, reps_quad = false;
+  bool use_K = false, rep_diag8 = false, rep_perm = false;
   bool reps_wide = false;  // representatives in rows of 64 bytes (8 FP32 / 4 FP64 slots), else 2 slots
   // Stage 6 (fused z FFT + diagonal-sign gather): unit table and spectral points.
   const void* zr_units = nullptr;

@@ -89,21 +89,6 @@ struct RegFFT<C, INV, N, Ns, 1> {
 };
 template <typename C, bool INV, int N> __device__ __forceinline__ void reg_fft(C* v) { RegFFT<C, INV, N, 1, N>::run(v); }
 
-// FFT of `count` lines of length H in padded shared memory, one thread per line.
-// Line l starts at line_base(l) and has element stride es.
-template <typename C, bool INV, int H>
-__device__ __forceinline__ void smem_lines(C* buf, int count, int group, int gstride, int lstride, int es) {
-  for (int l = threadIdx.x; l < count; l += blockDim.x) {
-    C* p = buf + (l / group) * gstride + (l % group) * lstride;
-    C v[H];
-#pragma unroll
-    for (int i = 0; i < H; ++i) v[i] = p[i * es];
-    reg_fft<C, INV, H>(v);
-#pragma unroll
-    for (int i = 0; i < H; ++i) p[i * es] = v[i];
-  }
-}
-
 // Alive parity channels per centring (WHT index o = o0 + 2 o1 + 4 o2 of each channel),
 // as compile-time data so channel loops unroll with constant register indices.
 // CT: 0 plain (no fold), 1 I, 2 F, 3 C, 4 A (same order as the plan's offsets).
@@ -1136,41 +1121,6 @@ __global__ void k_fft_z_fwd_h(const DevGeom* __restrict__ g, const typename Cx<T
   }
 }
 
-// Backward: expand G0 from orbit representatives (ET table) + inverse z FFT, cubic H:
-// G0R[slot][o] -> W[slot][c][z][y][x].
-template <typename T, int H>
-__global__ void k_expand_ifft_z_h(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
-                                  const int2* __restrict__ ET, const typename Cx<T>::type* __restrict__ G0R,
-                                  typename Cx<T>::type* __restrict__ W) {
-  pdl_enter();
-  using C = typename Cx<T>::type;
-  constexpr int S = H + 1;
-  constexpr int PL = H * S;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* buf = reinterpret_cast<C*>(smem_raw);
-  const int y0 = blockIdx.x * kZB, c = blockIdx.y, slot = blockIdx.z;
-  const int ny = min(kZB, H - y0);
-  const int tid = threadIdx.x, nth = blockDim.x;
-  const size_t hvol = static_cast<size_t>(H) * H * H;
-  const int2* et = ET + static_cast<size_t>(c) * hvol;
-  const C* rep = G0R + static_cast<size_t>(slot) * g->n_orbits;
-  const C* ph = tables + g->ph_off;
-  for (int e = tid; e < ny * H * H; e += nth) {
-    const int x = e % H, z = (e / H) % H, yy = e / (H * H);
-    const int2 t = et[(static_cast<size_t>(z) * H + y0 + yy) * H + x];
-    buf[yy * PL + z * S + x] = cmulc(rep[t.x], ph[t.y]);  // G0R * e^{+2 pi i j/P}
-  }
-  __syncthreads();
-  smem_lines<C, true, H>(buf, ny * H, H, PL, 1, S);
-  __syncthreads();
-  C* dst = W + (static_cast<size_t>(slot) * g->n_ch + c) * hvol;
-  for (int e = tid; e < ny * H * H; e += nth) {
-    const int x = e % H, z = (e / H) % H, yy = e / (H * H);
-    dst[(static_cast<size_t>(z) * H + y0 + yy) * H + x] = buf[yy * PL + z * S + x];
-  }
-}
-
-
 // Spectral-ASU gather from the z-fastest packed workspace, cubic M (= 2H centred,
 // = H plain), D representative operations; separates the two fields of the slot on
 // the fly.  The geometry is staged in shared memory once per CTA.
@@ -1544,53 +1494,6 @@ k_fft_z_recon_diag8(const DevGeom* __restrict__ g, const typename Cx<T>::type* _
       const int fa = 2 * (slot0 + k);
       F[static_cast<size_t>(fa) * ns + sidx] = acca;
       if (fa + 1 < nfields) F[static_cast<size_t>(fa + 1) * ns + sidx] = accb;
-    }
-  }
-}
-
-// G0 at orbit representatives of the two fields of a slot, packed as G_a + i G_b.
-// Each thread serves SPT consecutive slots, reusing the table entries and keeping
-// several independent spectrum gathers in flight.
-constexpr int kRepSlots = 4;
-template <typename T>
-__global__ void k_inv_recon_reps(const DevGeom* __restrict__ g, const typename Cx<T>::type* __restrict__ tables,
-                                 const int32_t* __restrict__ inv_spec, const int32_t* __restrict__ inv_phase,
-                                 const typename Cx<T>::type* __restrict__ F, typename Cx<T>::type* __restrict__ G0R,
-                                 int nfields) {
-  pdl_enter();
-  using C = typename Cx<T>::type;
-  const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= g->n_orbits) return;
-  const int slot0 = blockIdx.y * kRepSlots;
-  const int nslots = (nfields + 1) / 2;
-  const int d = g->d;
-  const int ns = g->n_spec;
-  const C* ph = tables + g->ph_off;
-  C acc[2 * kRepSlots];
-#pragma unroll
-  for (int k = 0; k < 2 * kRepSlots; ++k) acc[k] = mk<C>(static_cast<T>(0), static_cast<T>(0));
-  for (int a = 0; a < d; ++a) {
-    const int s = inv_spec[static_cast<size_t>(o) * d + a];
-    if (s == 0) continue;
-    const int si = (s > 0 ? s : -s) - 1;
-    const C w = ph[inv_phase[static_cast<size_t>(o) * d + a]];
-#pragma unroll
-    for (int k = 0; k < 2 * kRepSlots; ++k) {
-      const int f = 2 * slot0 + k;
-      if (f < nfields) {
-        C v = F[static_cast<size_t>(f) * ns + si];
-        if (s < 0) v = cconj(v);
-        acc[k] = cadd(acc[k], cmulc(v, w));
-      }
-    }
-  }
-  const T inv_d = static_cast<T>(1.0 / static_cast<double>(d));
-#pragma unroll
-  for (int k = 0; k < kRepSlots; ++k) {
-    const int slot = slot0 + k;
-    if (slot < nslots) {
-      const C a = acc[2 * k], b = acc[2 * k + 1];
-      G0R[static_cast<size_t>(slot) * g->n_orbits + o] = mk<C>(inv_d * (a.x - b.y), inv_d * (a.y + b.x));
     }
   }
 }
@@ -2241,8 +2144,10 @@ Status fast_unit_init(std::string* err) {
             cudaFuncSetAttribute(k_plane_fwd_h<T, HH, CTT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
             cudaFuncSetAttribute(k_plane_fwd_h<T, HH, CTT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
             cudaFuncSetAttribute(k_plane_bwd_h<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
-            cudaFuncSetAttribute(k_plane_fwd_s<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
-            cudaFuncSetAttribute(k_plane_bwd_s<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
+            if constexpr (HH <= 32) {
+              cudaFuncSetAttribute(k_plane_fwd_s<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
+              cudaFuncSetAttribute(k_plane_bwd_s<T, HH, CTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
+            }
             // The bulk-copy kernels also hold a little static shared memory, so their
             // dynamic limit is their exact need; a refusal is reported.
             cudaError_t te = cudaSuccess;
@@ -2286,9 +2191,9 @@ Status fast_unit_init(std::string* err) {
         using CC = typename Cx<T>::type;
         cudaFuncSetAttribute(k_expand_ifft_z<T, HH, wide_slots<CC>(), expand_slots<CC, HH, wide_slots<CC>()>(), sizeof(T) == 8>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
-        cudaFuncSetAttribute(k_expand_ifft_z<T, HH, 2, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
+        if constexpr (HH <= 32)
+          cudaFuncSetAttribute(k_expand_ifft_z<T, HH, 2, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
         cudaFuncSetAttribute(k_qsep_z<T, HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
-        cudaFuncSetAttribute(k_expand_ifft_z_h<T, HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmemFast);
       }
     });
   }
@@ -2414,9 +2319,12 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
               done = true;
             }
           }
-          if (!done && split)
-            launch_k(k_plane_fwd_s<T, HH, CTT>, dim3(H, nslots), split_threads<HH, CTT>(), smem_plane + HH * cs, st, g, tab, f0, E, W, nb);
-          else if (!done)
+          if constexpr (HH <= 32)
+            if (!done && split) {
+              launch_k(k_plane_fwd_s<T, HH, CTT>, dim3(H, nslots), split_threads<HH, CTT>(), smem_plane + HH * cs, st, g, tab, f0, E, W, nb);
+              done = true;
+            }
+          if (!done)
             launch_k(E ? k_plane_fwd_h<T, HH, CTT, true> : k_plane_fwd_h<T, HH, CTT, false>, dim3(H, nslots), thr_plane, smem_plane, st, g, tab, f0, E, W, nb);
         });
       });
@@ -2435,15 +2343,17 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
               done = true;
             }
           }
-          if (!done && split)
-            launch_k(k_plane_bwd_s<T, HH, CTT>, dim3(H, nslots), split_threads<HH, CTT>(), smem_plane + HH * cs, st, g, tab, W, E, f0_out, nb);
-          else if (!done)
+          if constexpr (HH <= 32)
+            if (!done && split) {
+              launch_k(k_plane_bwd_s<T, HH, CTT>, dim3(H, nslots), split_threads<HH, CTT>(), smem_plane + HH * cs, st, g, tab, W, E, f0_out, nb);
+              done = true;
+            }
+          if (!done)
             launch_k(k_plane_bwd_h<T, HH, CTT>, dim3(H, nslots), thr_plane, smem_plane, st, g, tab, W, E, f0_out, nb);
         });
       });
     }
   } else {
-    const int thr_z = std::max(64, ((kZB * H + 31) / 32) * 32);
     const size_t smem_z = static_cast<size_t>(kZB) * H * (H + 1) * cs;
     const dim3 gz((H + kZB - 1) / kZB, nch, nslots);
     switch (a.stage) {
@@ -2528,11 +2438,9 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
         });
         break;
       case 3: {
-        const int no = a.n_orbits;
-        if (a.reps_quad) {
-          const uint2* tp = static_cast<const uint2*>(a.fib_taps);
-          const uint2* fo = static_cast<const uint2*>(a.fib_outs);
-          const int fb = (a.n_fib + kFibers - 1) / kFibers;
+        const uint2* tp = static_cast<const uint2*>(a.fib_taps);
+        const uint2* fo = static_cast<const uint2*>(a.fib_outs);
+        const int fb = (a.n_fib + kFibers - 1) / kFibers;
 #define CFFT_INV_FIBER(LL, NF)                                                                                          \
   {                                                                                                                     \
     const int ns = (nb + (NF) - 1) / (NF);                                                                              \
@@ -2544,14 +2452,10 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
       default: launch_k(k_inv_fiber<T, 8, LL, NF>, gf, kFibers * (LL), 0, st, g, tab, tp, fo, a.n_fib, Fin, G0R, nb); break; \
     }                                                                                                                   \
   }
-          if (a.slot_fields == 1) CFFT_INV_FIBER(2, 1)
-          else if (a.reps_wide) CFFT_INV_FIBER(wide_slots<C>(), 2)
-          else CFFT_INV_FIBER(2, 2)
+        if (a.slot_fields == 1) CFFT_INV_FIBER(2, 1)
+        else if (a.reps_wide) CFFT_INV_FIBER(wide_slots<C>(), 2)
+        else CFFT_INV_FIBER(2, 2)
 #undef CFFT_INV_FIBER
-          break;
-        }
-        launch_k(k_inv_recon_reps<T>, dim3((no + 127) / 128, (nslots + kRepSlots - 1) / kRepSlots), 128, 0, st, 
-            g, tab, static_cast<const int32_t*>(a.inv_spec), static_cast<const int32_t*>(a.inv_phase), Fin, G0R, nb);
         break;
       }
       default:
@@ -2572,14 +2476,13 @@ Status fast_unit_launch(const FastArgs& a, std::string* err) {
             constexpr int L = wide_slots<C>(), LS = expand_slots<C, HH, L>();
             launch_k(k_expand_ifft_z<T, HH, L, LS, sizeof(T) == 8>, dim3(HH, nch, (nslots + L - 1) / L * (L / LS)),
                      expand_threads<C, HH, LS>(), (expand_plane<HH>() * LS + HH) * sizeof(C), st, g, tab, et, G0R, W, nb);
-          } else if (a.reps_quad && (HH > 32 || HH * nch * ((nslots + 1) / 2) > kSMs)) {
+          } else if (HH > 32 || HH * nch * ((nslots + 1) / 2) > kSMs) {
             constexpr int half = ((2 * HH + 31) / 32) * 32;
             launch_k(k_expand2_ifft_z<T, HH, 2>, dim3((HH + 1) / 2, nch, (nslots + 1) / 2), 2 * half, 0, st, g, tab, et, G0R, W, nb);
-          } else if (a.reps_quad) {
+          } else if constexpr (HH <= 32) {
             launch_k(k_expand_ifft_z<T, HH, 2, 2, true>, dim3(HH, nch, (nslots + 1) / 2), expand_threads<C, HH, 2>(),
                      (expand_plane<HH>() * 2 + HH) * sizeof(C), st, g, tab, et, G0R, W, nb);
-          } else
-            launch_k(k_expand_ifft_z_h<T, HH>, gz, thr_z, smem_z, st, g, tab, static_cast<const int2*>(a.expand), G0R, W);
+          }
         });
         break;
     }
