@@ -1200,20 +1200,18 @@ Status plan_device_init(Plan* p, std::string* err) {
   if (p->tune.chunk_bytes > 0) budget = static_cast<size_t>(p->tune.chunk_bytes);
   const size_t per_field = T.n_ch * hvol * cs / (p->fast_h ? 2 : 1);
   size_t ch = std::max<size_t>(1, std::min<size_t>(B, budget / std::max<size_t>(per_field, 1)));
-  // Two concurrent lanes from 24 MiB of channel workspace on the compile-time sizes: below, a
-  // second lane doubles the launches of a batch that one fills the SMs with.  us of a plain round
-  // trip / of one step of a contour loop with one and two lanes: Im-3m FP32 128^3 x64 (32 MiB)
-  // 92 / 125 and 78 / 101, x32 (16) 57 / 63 and 58 / 63, 192^3 x16 (27) 87 / 108 and 85 / 96, 64^3
-  // x256 (16) 43 / 48 and 50 / 46; FP64 128^3 x32 (32) 93 / 124 and 85 / 108, Pm-3m 64^3 x128 (32) 77 /
-  // 88 and 72 / 74, 64^3 x64 (16) 41 / 44 and 47 / 46.  The general kernels' launches are longer
-  // for their workspace and change over at 8 MiB (GPU us of a round trip with one and two): P6/mmm
-  // 60 x 60 x 80 FP64 x4 (18 MiB) 63 and 59, Im-3m 160^3 FP64 x8 (32) 119 and 114, P2_13 40^3 FP32
-  // x128 (8) 79 and 75, Im-3m 40^3 FP32 x128 (4) 35 and 36, Pm-3m 20^3 FP32 x128 (1) 21 and 24.
+  // Two concurrent lanes from 32 MiB of channel workspace: below, a second lane doubles the
+  // launches of a batch that one fills the SMs with.  us of a plain round trip / of one step of
+  // a contour loop with one and two lanes: Im-3m FP32 128^3 x64 (32 MiB) 92 / 125 and 78 / 101, x32
+  // (16) 57 / 63 and 59 / 63, 64^3 x256 (16) 43 / 48 and 52 / 46, 192^3 x16 (27) 86 / 108 and 85 / 96, on
+  // new fields each call 89 and 92; FP64 128^3 x32 (32) 93 / 124 and 84 / 108, Pm-3m 64^3 x128 (32)
+  // 77 / 88 and 70 / 71, x64 (16) 41 / 44 and 46 / 44.  General kernels: P6/mmm 60 x 60 x 80 FP32 x32 (70)
+  // 224 / 266 and 209 / 242, Pm-3m 90^3 FP32 x32 (22) 89 / 90 and 88 / 83, Im-3m 160^3 FP64 x4 (16) 80 / 80
+  // and 81 / 74, 40^3 FP32 x128 (4) 39 / 38 and 48 / 35.
   p->lanes = 1;
   if (p->tune.lanes > 0) p->lanes = std::min(Plan::kMaxLanes, p->tune.lanes);
   else if (const char* ln = std::getenv("CFFT_LANES")) p->lanes = std::max(1, std::min(Plan::kMaxLanes, std::atoi(ln)));
-  else if (p->fast_h ? B >= 8 && B * per_field >= (static_cast<size_t>(24) << 20)
-                     : p->general && B >= 4 && B * per_field >= (static_cast<size_t>(8) << 20)) p->lanes = 2;
+  else if (tables && B >= 4 && B * per_field >= (static_cast<size_t>(32) << 20)) p->lanes = 2;
   if (p->lanes > 1) {  // whole pairs of fields, no lane left with a remainder
     size_t per = (B + p->lanes - 1) / p->lanes;
     if (p->fast_h) per += per & 1;
