@@ -708,7 +708,7 @@ Status launch_stage(Plan* p, int stage, const T* f0, typename Cx<T>::type* F, co
     a.lanes = lanes;
     a.stage = stage; a.nb = nb; a.H = p->fast_h; a.n_ch = T_.n_ch; a.centered = T_.centered ? 1 : 0;
     a.cent_type = p->cent_type; a.d = T_.d;
-    a.n_spec = static_cast<int>(T_.spec.size()); a.n_orbits = static_cast<int>(T_.orbit_rep.size());
+    a.n_spec = static_cast<int>(T_.spec.size());
     a.use_K = use_K; a.rep_diag8 = p->rep_diag8; a.rep_perm = p->rep_perm;
     a.reps_wide = p->reps_wide && !p->cluster;
     a.zr_units = p->d_zr_units; a.zr_pts = p->d_zr_pts; a.zr_pq = p->d_zr_pq; a.n_spec_pts = p->zr_npts; a.zr_n_units = p->zr_units;

@@ -31,7 +31,7 @@ struct FastArgs {
   int slot_fields = 2;    // fields per workspace slot (1: general kernels)
   int lanes = 1;          // chunks that run concurrently with this one, itself included
   int stage = 0, nb = 0, H = 0, n_ch = 1, centered = 0, cent_type = 0, d = 1;
-  int n_spec = 0, n_orbits = 0;
+  int n_spec = 0;
   bool use_K = false, rep_diag8 = false, rep_perm = false;
   bool reps_wide = false;  // representatives in rows of 64 bytes (8 FP32 / 4 FP64 slots), else 2 slots
   // Stage 6 (fused z FFT + diagonal-sign gather): unit table and spectral points.

@@ -28,7 +28,8 @@ constexpr int kSMs = 148;  // B200: the unit of the launch-size rules
 
 // Programmatic dependent launch of the fast-path kernels (off with CFFT_PDL=0): each
 // kernel of a lane may launch while its predecessor in the stream is finishing, and
-// waits for it in hardware (griddepcontrol.wait, pdl_enter) before touching memory.
+// waits for it in hardware (griddepcontrol.wait, pdl_enter) before touching memory that
+// another kernel writes.
 inline bool pdl_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("CFFT_PDL");

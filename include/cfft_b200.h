@@ -184,9 +184,11 @@ cfft_status cfft_plan_create(const cfft_desc* desc, cfft_plan* plan);
  * built-in default measured best on Im-3m 128^3). */
 typedef struct cfft_tuning {
   int64_t chunk_bytes;   /* channel workspace per chunk (CFFT_CHUNK_BYTES; 64 MiB) */
-  int lanes;             /* concurrent chunk lanes 1..4 (CFFT_LANES; 2 for batches >= 8) */
-  int zr_slots;          /* workspace slots per CTA of the fused z FFT + gather, 2 or 4 (CFFT_ZR_SLOTS; 4) */
-  int wide;              /* backward representatives in 64-byte rows: 0, 1 (CFFT_WIDE; 1) */
+  int lanes;             /* concurrent chunk lanes 1..4 (CFFT_LANES; 2 from 32 MiB of channel workspace) */
+  int zr_slots;          /* workspace slots per CTA of the fused z FFT + gather, 2 or 4 (CFFT_ZR_SLOTS;
+                            by default 1, 2 or 4 by launch size, edge and precision) */
+  int wide;              /* backward representatives in 64-byte rows: 0, 1 (CFFT_WIDE; 1 where a chunk
+                            fills a row and the expansion's launch is not small) */
   int tma;               /* bulk-copy plane kernels: 0, 1 forward, 2 backward, 3 both (CFFT_TMA; 0) */
   int cluster;           /* fused cluster kernels: 0, 8 or 16 CTAs (CFFT_CLUSTER; 0) */
 } cfft_tuning;
@@ -219,7 +221,10 @@ cfft_status cfft_update_kernel(cfft_plan plan, double ds, const double* lattice)
 cfft_status cfft_forward(cfft_plan plan, const void* f0, void* F, int batch, void* stream);
 
 /* ifft_unrecon_centered! / execute_m2_backward! (src/centering_fold.jl:745-775,
- * src/krfft.jl:1269-1277): F -> f0 (real part). */
+ * src/krfft.jl:1269-1277): F -> f0 (real part).  On compile-time sized channel grids
+ * (exec_path bit 0) fields 2i and 2i + 1 of a forward or backward call share a complex
+ * transform: their rounding errors scale with the larger of the two, a NaN or infinity in
+ * one reaches the other, and so does the imaginary part of an inverse that is not real. */
 cfft_status cfft_backward(cfft_plan plan, const void* F, void* f0, int batch, void* stream);
 
 /* Batched forms over an array of plans (no reference counterpart: a caller of the
