@@ -467,12 +467,15 @@ template <typename T, int H, int CT> constexpr int row_vec() {
 // forward + backward with / without the two warps: Im-3m 64^3 x64 27.7 / 31.9, 64^3 x256 69.2 /
 // 69.8, 48^3 x64 19.2 / 20.3, 96^3 x32 (384 blocks) 42.1 / 46.5, but 96^3 x135 (816 per lane)
 // 126.3 / 122.8 and three contour steps there 599 / 551: at H = 24 only up to four blocks per SM.
+// F centring (two channels), FP32: Fm-3m 96^3 x32 (384 blocks) 29.1 / 30.0, x135 (1632) 55.0 / 53.1, x256
+// (1536 per lane) 83.7 / 79.7, so the same there; 128^3 x57 58.9 / 61.4; FP64 48^3 x256 31.0 / 33.0, 64^3
+// x64 20.7 / 22.2.
 template <typename T> inline int plane_line_threads(int H, int nch, bool folded, int ntasks) {
   constexpr int v = 16 / static_cast<int>(sizeof(T));
   const int base = std::max(64, ((nch * H + 31) / 32) * 32);
   const int items = H * H / (H % v == 0 ? v : 1);
   const auto rounds = [&](int t) { return (items + t - 1) / t; };
-  const bool fits = sizeof(T) == 4 || H < 24 || ntasks <= 4 * kSMs;
+  const bool fits = H != 24 || (sizeof(T) == 4 && nch == 4) || ntasks <= 4 * kSMs;
   return folded && fits && rounds(base + 64) < rounds(base) && rounds(base + 64) <= 2 ? base + 64 : base;
 }
 
